@@ -60,21 +60,13 @@ int dense_plain_device(const double *dH, int n, int k, const double *dX0, int ma
                        int *iterations_done, double *fixed_point_residual, cudaStream_t stream)
 {
     const size_t elems = (size_t)n * (size_t)k;
-    DeviceBuffer<double> xa, xb, d, P;
+    DeviceBuffer<double> xa, xb, d;
     IPTGB_CHECK(xa.alloc(elems, stream));
     IPTGB_CHECK(xb.alloc(elems, stream));
     IPTGB_CHECK(d.alloc((size_t)n, stream));
     DenseFp64Operator op;
-    op.H = dH;
-    op.ldh = n;
-    op.n = n;
-    op.k = k;
-    op.S = dense64_split_for(n, k, device_sm_count());
-    op.stream = stream;
-    IPTGB_CHECK(P.alloc((size_t)op.S * elems, stream));
-    op.P = P.ptr;
     SolveScratch scratch;
-    int status = scratch.init(elems, stream);
+    int status = scratch.init(n, k, stream);
     if (status == IPT_CUDA_SUCCESS) {
         if (dX0 != nullptr) {
             status = cudaMemcpyAsync(xa.ptr, dX0, elems * sizeof(double),
@@ -86,7 +78,7 @@ int dense_plain_device(const double *dH, int n, int k, const double *dX0, int ma
         }
     }
     if (status == IPT_CUDA_SUCCESS) {
-        status = launch_extract_diagonal(dH, n, n, d.ptr, stream);
+        status = op.bind(dH, n, d.ptr, stream);
     }
     double *xfinal = nullptr;
     if (status == IPT_CUDA_SUCCESS) {
@@ -125,7 +117,7 @@ int csr_plain_device(const int *row_ptr, const int *col_ind, const double *vals,
     op.Y = Y.ptr;
     op.stream = stream;
     SolveScratch scratch;
-    int status = scratch.init(elems, stream);
+    int status = scratch.init(n, k, stream);
     if (status == IPT_CUDA_SUCCESS) {
         if (dX0 != nullptr) {
             status = cudaMemcpyAsync(xa.ptr, dX0, elems * sizeof(double),

@@ -18,6 +18,7 @@
 #include "fpconv.cuh"
 #include "ipt_plain.h"
 #include "lowp.h"
+#include "oz.cuh"
 #include "oz_product.h"
 #include "prep.h"
 #include "reduce.cuh"
@@ -31,8 +32,7 @@ namespace iptgb {
 // ---------------------------------------------------------------------------
 struct DenseApply final : Fp64Apply {
     const double *H = nullptr;
-    // optional split-operand product on the tensor cores (k_oz.cu), the
-    // default of the mixed solve
+    // split-operand product on the tensor cores (k_oz.cu), the default
     OzProduct *oz = nullptr;
     // optional double-FP32 copy of H: products in double-float arithmetic on
     // the FP32 pipe (k_df64.cu) instead of FP64 FMAs
@@ -105,32 +105,27 @@ struct CsrApply final : Fp64Apply {
 // ---------------------------------------------------------------------------
 struct Fp64Stage final : IptStage {
     std::unique_ptr<Fp64Operator> op;
-    DenseFp64Operator *dense = nullptr;
     CsrFp64Operator *csr = nullptr;
     const double *d = nullptr;
     int n = 0;
     int sms = 148;
     cudaStream_t s = nullptr;
-    DeviceBuffer<double> P, Y, Xb;
+    DeviceBuffer<double> Y, Xb;
 
     int run(int p, int maxiter, double tol, int check_every, double *X, int *iterations,
             double *fpres_out, long long *matvecs) override
     {
         const size_t elems = (size_t)n * (size_t)p;
-        if (dense != nullptr) {
-            dense->k = p;
-            dense->S = dense64_split_for(n, p, sms);
-            IPTGB_CHECK(P.alloc((size_t)dense->S * elems, s));
-            dense->P = P.ptr;
-        } else {
+        if (csr != nullptr) {
             csr->k = p;
             IPTGB_CHECK(Y.alloc(elems, s));
             csr->Y = Y.ptr;
         }
         IPTGB_CHECK(Xb.alloc(elems, s));
         SolveScratch scratch;
-        IPTGB_CHECK(scratch.init(elems, s));
+        IPTGB_CHECK(scratch.init(n, p, s));
         IPTGB_CHECK(launch_set_identity(X, n, p, s));
+        IPTGB_CHECK(op->start(X, p, d));
         double *x = X;
         double *y = Xb.ptr;
         double best = INFINITY;
@@ -189,12 +184,11 @@ IptStage *make_fp64_dense_stage(const double *dH, int n, const double *d, cudaSt
 {
     auto *st = new Fp64Stage();
     auto *op = new DenseFp64Operator();
-    op->H = dH;
-    op->ldh = n;
-    op->n = n;
-    op->stream = stream;
     st->op.reset(op);
-    st->dense = op;
+    if (op->bind(dH, n, nullptr, stream) != IPT_CUDA_SUCCESS) {
+        delete st;
+        return nullptr;
+    }
     st->d = d;
     st->n = n;
     st->sms = device_sm_count();
@@ -474,25 +468,22 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
                                                            : kLowpTF32;
     double hnorm = 0.0, maxabs_off = 0.0;
     unsigned long long descents = 0;
-    // The mixed-precision solve forms its FP64-accurate products on the
-    // tensor cores from digit slices of Delta (one split per solve, k_oz.cu);
-    // tuning knob IPT_GB300_ACCURATE_PRODUCT = df selects double-FP32
-    // arithmetic on the FP32 pipe instead, fp64 (or IPT_GB300_FP64_DFMA=1)
-    // FP64 FMAs.  The plain FP64 path keeps FP64 FMAs throughout.
+    // The FP64-accurate products run on the tensor cores from digit slices of
+    // Delta (k_oz.cu): six slices (48 bits) in the mixed solve, seven (56
+    // bits) in the plain FP64 solve.  Tuning knob IPT_GB300_ACCURATE_PRODUCT
+    // = df selects double-FP32 arithmetic on the FP32 pipe for the mixed solve
+    // instead, fp64 (or IPT_GB300_FP64_DFMA=1) FP64 FMAs.
     const char *ap = getenv("IPT_GB300_ACCURATE_PRODUCT");
     const bool want_fp64 = env_flag("IPT_GB300_FP64_DFMA", 0) ||
                            (ap != nullptr && strcmp(ap, "fp64") == 0);
     const bool want_df = ap != nullptr && strcmp(ap, "df") == 0;
-    const bool use_oz = lowp_mode && !want_fp64 && !want_df;
+    const bool use_oz = !want_fp64 && (!lowp_mode || !want_df);
     DeviceBuffer<float> Hsplit;
-    OzDelta ozd;
+    OzMatrix ozm;
     OzProduct ozp;
     const size_t mat = (size_t)n * n;
     if (lowp_mode && want_df) {
         IPTGB_CHECK(Hsplit.alloc(2 * mat, s));
-    }
-    if (use_oz) {
-        IPTGB_CHECK(ozd.init_storage(n, s));
     }
     std::unique_ptr<LowpDenseOperator> lowp;
     int st = IPT_CUDA_SUCCESS;
@@ -521,8 +512,10 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         su.diag = d.ptr;
         su.stats = stats.ptr;
         if (use_oz) {
-            su.oz = ozd.A.ptr;
-            su.oz_rowexp = ozd.rowexp.ptr;
+            IPTGB_CHECK(ozm.init_storage(n, s));
+            IPTGB_CHECK(ozm.alloc_words(kOzSlices, s));
+            su.oz_rowexp = ozm.rowexp.ptr;
+            su.oz_words = ozm.words.ptr;
         }
         lowp.reset(make_lowp_dense_operator(dH_in, n, kind, s, &st, &su));
         if (lowp == nullptr) {
@@ -588,10 +581,13 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         apply.Hl = Hsplit.ptr + mat;
     }
     if (use_oz) {
-        // the fused pass wrote the slices of the (unpermuted) matrix; any
-        // other path splits the matrix the solve iterates on
-        if (!fused) IPTGB_CHECK(ozd.split_from(dH, n, s));
-        IPTGB_CHECK(ozp.bind(&ozd, d.ptr, s));
+        // the fused pass wrote the digit words of the (unpermuted) matrix;
+        // any other path those of the matrix the solve iterates on
+        if (!fused) {
+            IPTGB_CHECK(ozm.scan_rows(dH, n, nullptr, s));
+            IPTGB_CHECK(ozm.build_words(lowp_mode ? kOzSlices : 7, s));
+        }
+        IPTGB_CHECK(ozp.bind(&ozm, d.ptr, lowp_mode ? kOzSlices : 7, s));
         apply.oz = &ozp;
     }
     if (lowp_mode && fused) {
@@ -627,6 +623,7 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         stage.reset(make_lowp_stage_on(lowp.get(), d.ptr, n, s));
     } else {
         stage.reset(make_fp64_dense_stage(dH, n, d.ptr, s));
+        if (stage == nullptr) return IPT_CUDA_CUDA_ERROR;
     }
     std::unique_ptr<LearnedCorrection> learned;
     DeviceBuffer<double> coupling;

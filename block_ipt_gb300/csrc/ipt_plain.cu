@@ -1,5 +1,6 @@
 // ipt_plain.cu - FP64 plain-IPT driver loop.
 #include <math.h>
+#include <stdint.h>
 
 #include "common.cuh"
 #include "ipt_plain.h"
@@ -18,20 +19,34 @@ int device_sm_count()
     return sms;
 }
 
+int DenseFp64Operator::bind(const double *H_, int n_, double *d, cudaStream_t s)
+{
+    H = H_;
+    n = n_;
+    stream = s;
+    IPTGB_CHECK(matrix.scan_rows(H, n, d, s));
+    return matrix.build_words(7, s);
+}
+
+int DenseFp64Operator::start(const double *X, int k_, const double *d)
+{
+    k = k_;
+    IPTGB_CHECK(product.bind(&matrix, d, 7, stream));
+    if (g.count < (size_t)n * k) IPTGB_CHECK(g.alloc((size_t)n * k, stream));
+    IPTGB_CHECK(launch_gap_reciprocals(d, n, k, g.ptr, stream));
+    return product.begin(X, k);
+}
+
 int DenseFp64Operator::step(const double *X, double *Xn, const double *d, int want_norms,
                             NormScratch *ns)
 {
-    {
-        KernelTimerScope timer(kProfFp64Product, stream);
-        IPTGB_CHECK(launch_dense64_partial(H, n, ldh, X, n, k, P, S, stream));
-    }
-    KernelTimerScope timer(kProfFp64Update, stream);
-    return launch_dense64_update(P, S, n, k, X, d, Xn, want_norms, ns, stream);
+    (void)d;
+    return product.step(X, g.ptr, Xn, want_norms, ns);
 }
 
 int DenseFp64Operator::diag_values(const double *X, double *values)
 {
-    return launch_dense64_diag_values(H, ldh, n, X, k, values, stream);
+    return launch_dense64_diag_values(H, n, n, X, k, values, stream);
 }
 
 int CsrFp64Operator::step(const double *X, double *Xn, const double *d, int want_norms,
@@ -60,6 +75,11 @@ int SolveScratch::init(size_t max_elems, cudaStream_t stream)
     ns.capacity = slots;
     IPTGB_CUDA(cudaMemsetAsync(ns.counter, 0, 16, stream));
     return IPT_CUDA_SUCCESS;
+}
+
+int SolveScratch::init(int n, int k, cudaStream_t stream)
+{
+    return init((size_t)blocks_for((size_t)n) * kThreads * (size_t)k, stream);
 }
 
 int SolveScratch::arm_history(int steps, double tol, cudaStream_t stream)
@@ -113,45 +133,131 @@ void SolveScratch::release(cudaStream_t stream)
     ns = NormScratch();
 }
 
+namespace {
+
+// Per host thread: two page-locked slots of two norms each that the update
+// kernels of alternate steps write directly (allocated on the thread's first
+// tolerance-stopped solve and kept for the life of the process).
+constexpr int kNormSlots = 2;
+
+double *pinned_norm_slots()
+{
+    static thread_local double *buf = nullptr;
+    if (buf == nullptr) {
+        void *p = nullptr;
+        if (cudaMallocHost(&p, 2 * kNormSlots * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        buf = static_cast<double *>(p);
+    }
+    return buf;
+}
+
+// A NaN no kernel produces marks a slot as not yet written.
+constexpr uint64_t kNormPending = 0x7FF45EED00000001ULL;
+
+void arm_slot(volatile uint64_t *slot)
+{
+    slot[0] = kNormPending;
+    slot[1] = kNormPending;
+}
+
+bool slot_written(const volatile uint64_t *slot)
+{
+    return slot[0] != kNormPending && slot[1] != kNormPending;
+}
+
+// Waits for a slot without a call into the driver per step; the stream is
+// queried now and then so that a failed launch ends the wait.
+int wait_slot(const volatile uint64_t *slot, cudaStream_t stream)
+{
+    for (unsigned int polls = 1; !slot_written(slot); ++polls) {
+        if ((polls & 0x3FFFu) != 0) continue;
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e == cudaSuccess && slot_written(slot)) break;
+        fprintf(stderr, "ipt_gb300: IPT step did not finish: %s\n", cudaGetErrorString(e));
+        return IPT_CUDA_CUDA_ERROR;
+    }
+    return IPT_CUDA_SUCCESS;
+}
+
+}  // namespace
+
 int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, double tol,
                   int use_tol, double *X_a, double *X_b, double **X_final,
                   int *iterations_done, double *fixed_point_residual, SolveScratch *scratch,
                   cudaStream_t stream)
 {
-    double *x = X_a;
-    double *y = X_b;
-    int done = 0;
-    double fpres = NAN;
     (void)n;
-    (void)k;
-    for (int iter = 0; iter < maxiter; ++iter) {
-        IPTGB_CHECK(op.step(x, y, d, use_tol, &scratch->ns));
-        done = iter + 1;
-        if (use_tol) {
-            IPTGB_CUDA(cudaMemcpyAsync(scratch->host_norms, scratch->ns.norms,
-                                       2 * sizeof(double), cudaMemcpyDeviceToHost, stream));
-            IPTGB_CUDA(cudaStreamSynchronize(stream));
-            const double delta_norm = scratch->host_norms[0];
-            const double current_norm = scratch->host_norms[1];
-            if (current_norm <= 0.0 || !isfinite(current_norm)) {
-                return IPT_CUDA_INVALID_ARGUMENT;
-            }
-            fpres = delta_norm / current_norm;
-            double *t = x;
-            x = y;
-            y = t;
-            if (fpres <= tol) {
-                break;
-            }
-        } else {
-            double *t = x;
-            x = y;
-            y = t;
+    double *X[2] = {X_a, X_b};  // step i reads X[i % 2] and writes the other
+    IPTGB_CHECK(op.start(X_a, k, d));
+    if (!use_tol) {
+        for (int iter = 0; iter < maxiter; ++iter) {
+            IPTGB_CHECK(op.step(X[iter & 1], X[(iter + 1) & 1], d, 0, &scratch->ns));
         }
+        *X_final = X[maxiter & 1];
+        *iterations_done = maxiter;
+        *fixed_point_residual = NAN;
+        return IPT_CUDA_SUCCESS;
     }
-    *X_final = x;
+    // Tolerance mode: the host judges every step, and the GPU would wait ~25 us
+    // for it (the norms' copy, the synchronisation and the next launches; a
+    // step at n = 1024, k = 8 takes less).  So the next step is launched
+    // before the norms of the running one are known, unless the residuals so
+    // far say that the running step meets the tolerance.  A step past the
+    // converged one writes only the block that step read.
+    double *slots = pinned_norm_slots();
+    if (slots == nullptr) return IPT_CUDA_ALLOCATION_FAILED;
+    double *const device_norms = scratch->ns.norms;
+    int launched = 0, status = IPT_CUDA_SUCCESS;
+    double r1 = NAN, r2 = NAN;  // the last two residuals
+    auto launch = [&]() -> int {
+        double *slot = slots + 2 * (launched % kNormSlots);
+        arm_slot(reinterpret_cast<volatile uint64_t *>(slot));
+        scratch->ns.norms = slot;
+        IPTGB_CHECK(op.step(X[launched & 1], X[(launched + 1) & 1], d, 1, &scratch->ns));
+        ++launched;
+        return IPT_CUDA_SUCCESS;
+    };
+    int done = 0;
+    while (done < maxiter) {
+        if (launched == done) status = launch();
+        const bool expect_stop = r1 * r1 <= 2.0 * tol * r2;
+        if (status == IPT_CUDA_SUCCESS && launched == done + 1 && launched < maxiter &&
+            !expect_stop) {
+            status = launch();
+        }
+        const double *slot = slots + 2 * (done % kNormSlots);
+        if (status == IPT_CUDA_SUCCESS) {
+            status = wait_slot(reinterpret_cast<const volatile uint64_t *>(slot), stream);
+        }
+        if (status != IPT_CUDA_SUCCESS) break;
+        const double delta_norm = slot[0];
+        const double current_norm = slot[1];
+        if (current_norm <= 0.0 || !isfinite(current_norm)) {
+            status = IPT_CUDA_INVALID_ARGUMENT;
+            break;
+        }
+        ++done;
+        r2 = r1;
+        r1 = delta_norm / current_norm;
+        if (r1 <= tol) break;
+    }
+    // no step may still be writing a slot (or X) once this call returns
+    if (status != IPT_CUDA_SUCCESS) {
+        cudaStreamSynchronize(stream);
+    } else if (launched > done) {
+        status = wait_slot(reinterpret_cast<const volatile uint64_t *>(
+                               slots + 2 * ((launched - 1) % kNormSlots)),
+                           stream);
+    }
+    scratch->ns.norms = device_norms;
+    IPTGB_CHECK(status);
+    *X_final = X[done & 1];
     *iterations_done = done;
-    *fixed_point_residual = fpres;
+    *fixed_point_residual = r1;
     return IPT_CUDA_SUCCESS;
 }
 

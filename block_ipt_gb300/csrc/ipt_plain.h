@@ -6,12 +6,15 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "oz_product.h"
 
 namespace iptgb {
 
 // One application of the IPT map X' = F(X) in FP64, plus (H X)_jj.
 struct Fp64Operator {
     virtual ~Fp64Operator() = default;
+    // Before the first step from an n x k block X with diagonal d.
+    virtual int start(const double *X, int k, const double *d) = 0;
     // Xn = F(X); with want_norms the step leaves ||Xn - X||_F, ||X||_F in ns->norms.
     virtual int step(const double *X, double *Xn, const double *d, int want_norms,
                      NormScratch *ns) = 0;
@@ -19,12 +22,25 @@ struct Fp64Operator {
     virtual int diag_values(const double *X, double *values) = 0;
 };
 
+// Dense H: Delta X by the 56-bit digit-slice product on the tensor cores
+// (k_oz.cu), whose consumer applies the map.  It replaces a split-K FP64 SIMT
+// product (GB300 runs FP64 FMAs at 1/64 of the FP32 rate; on a matrix of few
+// row blocks most SMs stood idle as well): a step takes 140 us instead of 3.7
+// ms at n = 8192, k = 32, 17 us instead of 105 us at n = 1024, k = 8 and 12 us
+// at n = 256, k = 4, so no size keeps the old one; 0.45 instead of 6.1 ms with
+// all n = 1501 columns.  Its error is the smaller one (after 12 steps at n =
+// k = 1501 8e-16 against 7e-14 in the 2-norm: the diagonal, which the FP64
+// product carried through y and the map took off again, is left out).
 struct DenseFp64Operator final : Fp64Operator {
+    OzMatrix matrix;
+    OzProduct product;
+    DeviceBuffer<double> g;  // n x k gap reciprocals
     const double *H = nullptr;
-    long long ldh = 0;
-    int n = 0, k = 0, S = 1;
-    double *P = nullptr;  // S * n * k partial slices
+    int n = 0, k = 0;
     cudaStream_t stream = nullptr;
+    // scans H (column-major n x n); d (optional) receives its diagonal
+    int bind(const double *H, int n, double *d, cudaStream_t s);
+    int start(const double *X, int k, const double *d) override;
     int step(const double *X, double *Xn, const double *d, int want_norms,
              NormScratch *ns) override;
     int diag_values(const double *X, double *values) override;
@@ -37,6 +53,7 @@ struct CsrFp64Operator final : Fp64Operator {
     int n = 0, k = 0;
     double *Y = nullptr;  // n * k
     cudaStream_t stream = nullptr;
+    int start(const double *, int, const double *) override { return IPT_CUDA_SUCCESS; }
     int step(const double *X, double *Xn, const double *d, int want_norms,
              NormScratch *ns) override;
     int diag_values(const double *X, double *values) override;
@@ -51,6 +68,8 @@ struct SolveScratch {
     double host_norms[2] = {0.0, 0.0};
     std::vector<double> host_hist;
     int init(size_t max_elems, cudaStream_t stream);
+    // for an n x k block, whose reductions may take whole blocks per column
+    int init(int n, int k, cudaStream_t stream);
     void release(cudaStream_t stream);
     // zeroed history for up to `steps` steps with the device-side stop at tol
     int arm_history(int steps, double tol, cudaStream_t stream);

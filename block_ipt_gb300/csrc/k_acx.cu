@@ -10,7 +10,7 @@
 // with cublasDgemm and reads a flag, k residuals and two cuBLAS norms back
 // per map evaluation.
 //
-// Here HX is the split-K FP64 product of the plain path (k_dense64.cu); F is
+// Here HX is the plain path's FP64-accurate tensor-core product (k_oz.cu); F is
 // one CTA per column that reads (HX)_cc, evaluates the column's residual
 // norm and the map in one pass, in place; the two Frobenius norms are one
 // deterministic grid reduction; an extrapolation step is one CTA per column
@@ -30,6 +30,7 @@
 #include "rayleigh.h"
 #include "ipt_plain.h"
 #include "kernels.cuh"
+#include "oz_product.h"
 #include "reduce.cuh"
 
 namespace iptgb {
@@ -234,21 +235,17 @@ __global__ void acx_identity_f32_kernel(float *__restrict__ X, int n, int k)
 namespace {
 
 struct AcxDense {
-    const double *H = nullptr;
-    int n = 0, k = 0, S = 1;
+    OzMatrix matrix;
+    OzProduct product;
+    int n = 0, k = 0;
     cudaStream_t s = nullptr;
     const double *d = nullptr;
-    double *P = nullptr, *resid = nullptr;
+    double *resid = nullptr;
     int *flag = nullptr;
     // Y = F(X)
     int apply(const double *X, double *Y)
     {
-        if (S > 1) {
-            IPTGB_CHECK(launch_dense64_partial(H, n, n, X, n, k, P, S, s));
-            IPTGB_CHECK(launch_sum_partials(P, S, (size_t)n * k, Y, s));
-        } else {
-            IPTGB_CHECK(launch_dense64_partial(H, n, n, X, n, k, Y, 1, s));
-        }
+        IPTGB_CHECK(product.apply(X, n, k, Y, n));
         return launch_pdl(acx_map_kernel, dim3(k), dim3(kAcxThreads), 0, s, Y, X, d, n, resid,
                           flag);
     }
@@ -308,18 +305,15 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
     int status = ACX_CUDA_SUCCESS;
     {
         AcxDense F;
-        F.H = H;
         F.n = n;
         F.k = k;
         F.s = s;
-        F.S = dense64_split_for(n, k, device_sm_count());
-        DeviceBuffer<double> X, F2, F3, P, small;
+        DeviceBuffer<double> X, F2, F3, small;
         DeviceBuffer<double2> part;
         DeviceBuffer<int> flags;
         // small: d (n) | resid (k) | norms (2)
         bool ok = X.alloc(elems, s) == IPT_CUDA_SUCCESS && F2.alloc(elems, s) == IPT_CUDA_SUCCESS &&
                   F3.alloc(elems, s) == IPT_CUDA_SUCCESS &&
-                  (F.S <= 1 || P.alloc(elems * (size_t)F.S, s) == IPT_CUDA_SUCCESS) &&
                   small.alloc((size_t)n + (size_t)k + 2, s) == IPT_CUDA_SUCCESS &&
                   part.alloc(kAcxNormBlocks, s) == IPT_CUDA_SUCCESS &&
                   flags.alloc(2, s) == IPT_CUDA_SUCCESS;
@@ -328,7 +322,6 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         int *flag = flags.ptr;
         unsigned int *counter = reinterpret_cast<unsigned int *>(flags.ptr + 1);
         F.d = d;
-        F.P = P.ptr;
         F.resid = resid;
         F.flag = flag;
         auto cuda_ok = [&](cudaError_t e) {
@@ -341,7 +334,9 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         };
         if (status == ACX_CUDA_SUCCESS) {
             cuda_ok(cudaMemsetAsync(flags.ptr, 0, 2 * sizeof(int), s));
-            lib_ok(launch_extract_diagonal(H, n, n, d, s));
+            lib_ok(F.matrix.scan_rows(H, n, d, s));
+            lib_ok(F.matrix.build_words(7, s));
+            lib_ok(F.product.bind(&F.matrix, d, 7, s));
             if (initial == nullptr) {
                 lib_ok(launch_set_identity(X.ptr, n, k, s));
             } else {

@@ -1,33 +1,47 @@
 // k_oz.cu - FP64-accurate block product Y = H X on the FP16 tensor cores.
 //
-// Replaces the reference's FP64 cublasDgemm of the mixed refinement
+// Replaces the reference's FP64 cublasDgemm of the plain IPT loop
+// (IPT_C_GPU/src/ipt_cuda.cu:1649,1888), of the mixed refinement
 // (IPT_C_GPU/src/mixed_precision/ipt_mixed_precision_cuda.cu:917,958) and of
 // the Rayleigh-Ritz products.  H = D + Delta: the diagonal part is applied
-// in FP64, Delta X by the split-operand scheme of oz.cuh:
+// in FP64, Delta X by the split-operand scheme of oz.cuh.
 //
-//  * Delta is split once per matrix into kOzSlices FP16 digit slices
-//    A_s (row-major, K-major for the MMA, [slice][row][ldp]) with one
-//    exponent per row; X is split per product into B_t ([slice][col][ldp]
-//    concatenated as 6 * cp rows, cp = columns padded to 16) with one
-//    exponent per column (oz_slice_x_kernel);
-//  * oz_product_kernel is persistent: one CTA per SM walks a contiguous range
-//    of (128-row tile, 128-element K period) items.  Warp 4 streams the A
-//    slices (each byte of A is read once per product, L2 evict_first) and
-//    the B chunk through TMA into shared memory; warp 5 issues tcgen05.mma:
-//    per A slice s and K step one MMA of N = (6 - s) cp (two above N = 256)
-//    that adds every pair (s, t), t <= 5 - s, into the TMEM accumulator of
-//    level s + t (the B slices are consecutive rows, the level accumulators
-//    consecutive columns).  One thread issues every MMA of the SM and each
-//    issue costs it about 50-65 cycles whatever N, so the kernel issues as
-//    few and as wide MMAs as the level structure allows (24 per 64-element K
-//    chunk; one per pair took 84).  Two accumulator sets when they fit in
-//    TMEM, so the MMAs of the next period run while the last one drains;
-//    warps 0-3 drain the six level
-//    accumulators after every period, combine them in double-float
-//    arithmetic and keep a running sum per (row, column) until the CTA
-//    leaves the tile, then write one FP64 partial per (tile, CTA);
-//  * oz_finish_kernel adds the partials of each tile in a fixed order,
-//    scales by 2^(e_i + f_c - 16) and adds d_i X_ic.
+// oz_product_kernel<S, CP, MODE> is persistent, one CTA per SM over a
+// contiguous range of (column group, 128-row tile, K period) items, in stages
+// of 32 K elements, with a warp role for each resource:
+//  * warp 18 streams the digit words of Delta (8 bytes per entry, written once
+//    per solve) by 32 KB bulk copies; without words (one-off products, very
+//    large n) the converters copy the entries of H themselves (cp.async);
+//  * warps 0-7, the converters, expand the words into S FP16 digits per entry
+//    (one byte permute and one subtraction per two digits; from entries of H
+//    ~25 integer instructions more) and store 16-byte runs into the stage's
+//    64-byte-swizzled K-major A slices.  The words of the next stage are read
+//    before the current one is stored;
+//  * warp 16 brings the S x CP digit rows of X by TMA;
+//  * warp 17 issues tcgen05.mma: per slice s and 16-element K step one MMA of
+//    N = (slices t with s + t < V) * CP that adds every pair (s, t) into the
+//    TMEM accumulator of level s + t (the B slices are consecutive rows, the
+//    level accumulators consecutive columns): few and wide MMAs, since each
+//    costs its issuing thread tens of cycles;
+//  * warps 8-15 drain the level accumulators after every period (two sets, so
+//    the next period's MMAs run meanwhile, when they fit in TMEM).  S = 7 adds
+//    the levels as 96-bit integers, exactly; S = 6 combines them in
+//    double-float arithmetic.  A CTA leaving a tile writes one FP64 partial.
+// The consumer of the partials (oz_finish_kernel or oz_update_kernel) adds
+// those of a tile in a fixed order, so the product is deterministic.
+//
+// What bounds it: shared-memory bandwidth.  A stage moves 32 KB of words in
+// and out, 56 KB (S = 7) of digits in and, through the MMAs, out again, and
+// the MMAs read the digit rows of X 34 times 2 KB: 265 KB, 2070 cycles at 128
+// bytes per cycle, against 1090 cycles of MMA and 32 KB of HBM traffic (79 us
+// per product of n = 8192 at the measured 6.8 TB/s).  Measured at n = 8192, 32
+// columns: 127 us per product (2240 cycles per stage; tensor pipe 50 %, HBM
+// 54 %); the split-K FP64 SIMT product it replaces in the plain path 3.6 ms
+// (95 % of the FP64 pipe).  Digit slices stored as FP16 (14 bytes per entry
+// with 7 slices) would need 139 us of HBM time; extracting the digits from H
+// in every product took 205 us (55 instructions per entry); A operands
+// in TMEM instead of shared memory 137 us (their tcgen05.st wait for the
+// MMAs, and only one accumulator set fits).
 //
 // Every mbarrier wait is bounded; a timeout sets the error flag, the CTA
 // drains its own copies and MMAs (bounded), frees TMEM and returns.
@@ -44,37 +58,63 @@
 #include "kernels.cuh"
 #include "oz.cuh"
 #include "oz_product.h"
+#include "reduce.cuh"
 #include "tcgen05.cuh"
 
 namespace iptgb {
 
 namespace oz {
 
-constexpr int kBM = 128;                      // UMMA M: rows per tile
-constexpr int kChunk = 64;                    // K elements per TMA chunk (128 B of FP16)
-constexpr uint32_t kABytes = kBM * 128;       // one slice of one chunk: 16 KB
-constexpr int kThreads = 192;                 // warps 0-3 epilogue, 4 producer, 5 MMA
-constexpr int kProducerWarp = 4;
-constexpr int kMmaWarp = 5;
-constexpr int kMaxASlots = 12;  // A ring depth (slices in flight), set by the shared memory left
-constexpr int kMaxBSlots = 2;   // B ring depth (chunks)
-constexpr int kChunksPerPeriod = kOzPeriod / kChunk;
+constexpr int kBM = 128;                       // UMMA M: rows per tile
+constexpr int kStageK = 32;                    // K elements per stage (64 B of FP16)
+constexpr uint32_t kABytes = kBM * 64;         // one slice of one stage: 8 KB
+constexpr int kConvWarps = 8;                  // warps 0-7: digits into the A ring
+constexpr int kDrainWarps = 8;                 // warps 8-15: accumulators to running sums
+constexpr int kProducerWarp = kConvWarps + kDrainWarps;
+constexpr int kMmaWarp = kProducerWarp + 1;
+constexpr int kWordsWarp = kProducerWarp + 2;
+constexpr int kThreads = 32 * (kConvWarps + kDrainWarps + 3);
+constexpr int kStages = 2;                     // A ring depth
+constexpr int kMaxBStages = 3;                 // B ring depth, where shared memory allows
+constexpr int kRawStages = 2;                  // ring of digit words / H entries
+constexpr uint32_t kRawBytes = kBM * kStageK * 8;
+constexpr int kMaxStagesPerItem = kOzPeriod / kStageK;
+// a matrix below this size stays in L2 between the products of a solve (126
+// MB usable); larger ones are streamed past it
+constexpr size_t kL2ResidentBytes = 96u << 20;
+
+// Where the digits come from: kWords - digit words written once per solve
+// (OzMatrix::words), 32 KB blocks by bulk copies; kRows - the entries of H
+// themselves, by each converter thread's own cp.async copies (one-off
+// products, and matrices whose digit words would take too much memory).
+enum Mode { kRows = 0, kWords = 1 };
 
 struct Params {
-    int n, C, cp;
-    int a_slots;   // A ring depth
-    int b_slots;   // B ring depth
-    int acc_bufs;  // TMEM accumulator sets (2: the epilogue drains one while the MMAs fill the other)
-    int nchunks, periods;
+    const double *H;
+    const uint4 *words;
+    const int *rowexp;
+    int n, groups, tiles, periods, nstages;  // nstages: K stages of a row
+    int spp;         // stages per period (item): at most kMaxStagesPerItem
     long long items;
     int maxslots;
+    int stream_h;    // H is read past L2 (evict first)
+    int b_loads;     // TMA boxes per B stage
     uint32_t b_bytes;
-    uint32_t idesc;  // M = 128, N = cp, FP16 x FP16 -> FP32
+};
+
+template <int S, int CP>
+struct Layout {
+    static constexpr int V = OzSplit<S>::kLevels;
+    static constexpr int kSets = 2 * V * CP <= 512 ? 2 : 1;  // accumulator sets in TMEM
+    static constexpr uint32_t kA = S * kABytes;    // A digits of a stage
+    static constexpr uint32_t kB = S * CP * 64;    // B digits of a stage
+    static constexpr uint32_t kFixed = 1024 + kStages * kA + kRawStages * kRawBytes;
+    static constexpr int kBStages = kFixed + kMaxBStages * kB + 512 <= 227 * 1024 ? kMaxBStages : 2;
+    static constexpr uint32_t kSmem = kFixed + kBStages * kB;
+    static_assert(kSmem + 512 <= 227 * 1024, "shared memory");
 };
 
 using tc::owner_of;
-
-using tc::mbar_arrive;
 
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
 {
@@ -83,22 +123,198 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e)
     e = (a - (s - bb)) + (b - bb);
 }
 
-template <int CP>
-__global__ void __launch_bounds__(kThreads, 1)
-oz_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ Params prm, double *__restrict__ P, int *err)
+// Instruction descriptor without N: M = 128, FP16 x FP16 -> FP32.
+constexpr uint32_t kIdesc = (1u << 4) | ((uint32_t)(kBM >> 4) << 24);
+
+// K-major operand, 64-byte swizzle: rows of 64 bytes, 8-row atoms of 512
+// bytes, descriptor version 1.
+__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr)
 {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(16u >> 4) << 16;
+    d |= (uint64_t)(512u >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
+// Asynchronous copies of H entries into a converter thread's own slots
+// (`bytes` 0 writes zeros).
+__device__ __forceinline__ void copy8(uint32_t dst, const double *src, int bytes, uint64_t pol)
+{
+    asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 8, %2, %3;" ::"r"(dst),
+                 "l"(src), "r"(bytes), "l"(pol)
+                 : "memory");
+}
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes,
+                                          uint32_t bar, uint64_t pol)
+{
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+        " [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar), "l"(pol)
+        : "memory");
+}
+
+__device__ __forceinline__ uint64_t l2_normal_policy()
+{
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+
+// Position in a CTA's sequence of stages: item it = (group * tiles + tile) *
+// periods + per, stage st of its period.
+struct Walk {
+    long long it;
+    int tile, per, st, count;  // count: stages of this period
+    __device__ __forceinline__ void start(long long first, const Params &p)
+    {
+        it = first;
+        per = (int)(first % p.periods);
+        tile = (int)((first / p.periods) % p.tiles);
+        st = 0;
+        count = min(p.spp, p.nstages - per * p.spp);
+    }
+    __device__ __forceinline__ void next(const Params &p)
+    {
+        if (++st < count) return;
+        st = 0;
+        ++it;
+        if (++per == p.periods) {
+            per = 0;
+            if (++tile == p.tiles) tile = 0;
+        }
+        count = min(p.spp, p.nstages - per * p.spp);
+    }
+};
+
+// Starts the copies of a thread's eight K entries l0..l0+7 of row `row` of H
+// (zeros outside the matrix) into its slots of the raw tile [32 K][128 rows].
+__device__ __forceinline__ void fetch8(const Params &p, const Walk &w, int r, int g, uint64_t pol,
+                                       uint32_t raw)
+{
+    const int row0 = w.tile * kBM;
+    const int row = row0 + r;
+    const int k0 = (w.per * p.spp + w.st) * kStageK;
+    const int l0 = k0 + 8 * g;
+    if (row0 + kBM <= p.n && k0 + kStageK <= p.n) {
+        const double *h = p.H + (size_t)l0 * p.n + row;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            copy8(raw + (uint32_t)(u * kBM * 8), h, 8, pol);
+            h += p.n;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int l = l0 + u;
+            const bool in = row < p.n && l < p.n;
+            copy8(raw + (uint32_t)(u * kBM * 8), in ? p.H + (size_t)l * p.n + row : p.H,
+                  in ? 8 : 0, pol);
+        }
+    }
+}
+
+__device__ __forceinline__ void tmem_ld_4cols(uint32_t taddr, uint32_t (&r)[4])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
+
+// Running sums of a thread's columns over the periods of a tile.
+template <int S, int NC>
+struct Sums;
+// 56-bit split: exact 96-bit integers (three words; a pair of 64-bit sums
+// would not leave the drain's loads enough registers).  Per period the levels
+// 0-3 and 4-7 are each combined by one wide multiply-add per level into 64
+// bits (below 2^48), with weights 2^24, 2^16, 2^8, 1.
+template <int NC>
+struct Sums<7, NC> {
+    uint32_t w[NC][3];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) w[j][0] = w[j][1] = w[j][2] = 0;
+    }
+    __device__ __forceinline__ void add(int j, const uint32_t (&l)[8])
+    {
+        constexpr int kWeight[4] = {1 << 24, 1 << 16, 1 << 8, 1};
+        long long part[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            part[h] = __float2int_rn(__uint_as_float(l[4 * h + 3]));
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const int v = __float2int_rn(__uint_as_float(l[4 * h + q]));
+                asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(part[h]) : "r"(v), "r"(kWeight[q]));
+            }
+        }
+        asm("{\n\t.reg .u32 a, b, c, d, e;\n\t"
+            "mov.b64 {a, b}, %3;\n\t"
+            "mov.b64 {c, d}, %4;\n\t"
+            "shr.s32 e, d, 31;\n\t"
+            "add.cc.u32 %0, %0, c;\n\t"
+            "addc.cc.u32 %1, %1, d;\n\t"
+            "addc.u32 %2, %2, e;\n\t"
+            "add.cc.u32 %1, %1, a;\n\t"
+            "addc.u32 %2, %2, b;\n\t}"
+            : "+r"(w[j][0]), "+r"(w[j][1]), "+r"(w[j][2])
+            : "l"(part[0]), "l"(part[1]));
+    }
+    __device__ __forceinline__ double value(int j) const
+    {
+        const long long hi = (long long)(((uint64_t)w[j][2] << 32) | w[j][1]);
+        return (double)hi * 4294967296.0 + (double)w[j][0];
+    }
+};
+// 48-bit split: double-float (H, L).
+template <int NC>
+struct Sums<6, NC> {
+    float H[NC], L[NC];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) H[j] = L[j] = 0.0f;
+    }
+    __device__ __forceinline__ void add(int j, const uint32_t (&l)[6])
+    {
+        float v[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[q] = __uint_as_float(l[q]);
+        float h, hh, e1, e2;
+        two_sum(v[0], v[1] * 0x1p-8f, h, e1);
+        two_sum(h, v[2] * 0x1p-16f, hh, e2);
+        const float ll = e1 + e2;
+        const float t = ll + (v[3] * 0x1p-24f + (v[4] * 0x1p-32f + v[5] * 0x1p-40f));
+        float s, e;
+        two_sum(H[j], hh, s, e);
+        H[j] = s;
+        L[j] += t + e;
+    }
+    __device__ __forceinline__ double value(int j) const { return (double)H[j] + (double)L[j]; }
+};
+
+template <int S, int CP, int MODE>
+__global__ void __launch_bounds__(kThreads, 1)
+oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ Params prm,
+                  double *__restrict__ P, int *err)
+{
+    using Lay = Layout<S, CP>;
+    constexpr int V = Lay::V;
+    constexpr int kSets = Lay::kSets;
+    constexpr int NC = CP / 2;                        // columns a drain warp sums
+    constexpr uint32_t kBBytes = Lay::kB;
+    constexpr int kBStages = Lay::kBStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int kBSlots = prm.b_slots;
-    const int kASlots = prm.a_slots;
-    uint8_t *a_ring = smem;
-    uint8_t *b_ring = smem + (size_t)kASlots * kABytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(b_ring + (size_t)kBSlots * prm.b_bytes);
-    uint32_t *tmem_slot =
-        reinterpret_cast<uint32_t *>(bars + 2 * kMaxASlots + 2 * kMaxBSlots + 5);
+    __shared__ uint64_t bars[2 * kStages + 2 * kBStages + 2 * kRawStages + 5];
+    __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
-    __shared__ int a_issued, b_issued;
+    __shared__ int b_issued, h_issued;
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -106,43 +322,49 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const long long it0 = (long long)blockIdx.x * prm.items / G;
     const long long it1 = ((long long)blockIdx.x + 1) * prm.items / G;
     const uint32_t bar0 = tc::smem_u32(bars);
-    auto a_full = [&](int q) { return bar0 + 8u * (uint32_t)q; };
-    auto a_empty = [&](int q) { return bar0 + 8u * (uint32_t)(kMaxASlots + q); };
-    auto b_full = [&](int q) { return bar0 + 8u * (uint32_t)(2 * kMaxASlots + q); };
-    auto b_empty = [&](int q) {
-        return bar0 + 8u * (uint32_t)(2 * kMaxASlots + kMaxBSlots + q);
-    };
-    // acc_full(b), acc_empty(b) for the accumulator sets b = 0, 1; mma_done
-    const uint32_t acc_base = bar0 + 8u * (uint32_t)(2 * kMaxASlots + 2 * kMaxBSlots);
-    auto acc_full = [&](int b) { return acc_base + 8u * (uint32_t)b; };
-    auto acc_empty = [&](int b) { return acc_base + 16u + 8u * (uint32_t)b; };
-    const uint32_t mma_done = acc_base + 32u;
-    const uint32_t a_base = tc::smem_u32(a_ring);
-    const uint32_t b_base = tc::smem_u32(b_ring);
+    auto bar = [&](int q) { return bar0 + 8u * (uint32_t)q; };
+    auto a_full = [&](int q) { return bar(q); };
+    auto a_empty = [&](int q) { return bar(kStages + q); };
+    auto b_full = [&](int q) { return bar(2 * kStages + q); };
+    auto b_empty = [&](int q) { return bar(2 * kStages + kBStages + q); };
+    constexpr int kRawBar = 2 * kStages + 2 * kBStages;
+    auto raw_full = [&](int q) { return bar(kRawBar + q); };
+    auto raw_empty = [&](int q) { return bar(kRawBar + kRawStages + q); };
+    constexpr int kAccBar = kRawBar + 2 * kRawStages;
+    auto acc_full = [&](int b) { return bar(kAccBar + b); };
+    auto acc_empty = [&](int b) { return bar(kAccBar + 2 + b); };
+    const uint32_t mma_done = bar(kAccBar + 4);
+    const uint32_t base = tc::smem_u32(smem);
+    const uint32_t b0 = base + kStages * Lay::kA;
+    const uint32_t raw0 = b0 + kBStages * kBBytes;
 
     if (threadIdx.x == 0) {
-        for (int q = 0; q < kASlots; ++q) {
-            tc::mbar_init(a_full(q), 1);
+        for (int q = 0; q < kStages; ++q) {
+            tc::mbar_init(a_full(q), kConvWarps);
             tc::mbar_init(a_empty(q), 1);
         }
-        for (int q = 0; q < kBSlots; ++q) {
+        for (int q = 0; q < kBStages; ++q) {
             tc::mbar_init(b_full(q), 1);
             tc::mbar_init(b_empty(q), 1);
         }
         for (int b = 0; b < 2; ++b) {
             tc::mbar_init(acc_full(b), 1);
-            tc::mbar_init(acc_empty(b), 4);  // one arrival per epilogue warp
+            tc::mbar_init(acc_empty(b), kDrainWarps);
+        }
+        for (int q = 0; q < kRawStages; ++q) {
+            tc::mbar_init(raw_full(q), 1);
+            tc::mbar_init(raw_empty(q), kConvWarps);
         }
         tc::mbar_init(mma_done, 1);
         abort_flag = 0;
-        a_issued = 0;
         b_issued = 0;
+        h_issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == kProducerWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         tc::smem_u32(tmem_slot)),
+                         tc::smem_u32(&tmem_slot)),
                      "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -150,228 +372,343 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = tmem_slot;
 
-    if (warp == kProducerWarp && lane == 0) {
-        // ---- TMA producer: per chunk the B chunk, then the six A slices ----
-        const uint64_t pol = tc::l2_stream_policy();
-        int ac = 0, bc = 0;
-        int aq = 0, bq = 0;            // ring slots of copy ac / bc
-        uint32_t apar = 0, bpar = 0;   // parities of their rounds
-        bool waited = false;
-        for (long long it = it0; it < it1 && !abort_flag; ++it) {
-            const int tile = (int)(it / prm.periods);
-            const int per = (int)(it % prm.periods);
-            const int c0 = per * kChunksPerPeriod;
-            const int c1 = min(prm.nchunks, c0 + kChunksPerPeriod);
-            for (int c = c0; c < c1 && !abort_flag; ++c) {
-                if (!waited) {
-                    // Delta's slices do not depend on the preceding kernel: the
-                    // first chunk's slices are requested before waiting for the
-                    // grid that wrote the X slices
-                    for (int s = 0; s < kOzSlices; ++s) {
-                        tc::mbar_expect_tx(a_full(s), kABytes);
-                        tc::tma_load_3d_hint(a_base + (uint32_t)s * kABytes, &tmA, c * kChunk,
-                                             tile * kBM, s, a_full(s), pol);
-                    }
-                    ac = kOzSlices;
-                    aq = kOzSlices % kASlots;
-                    apar = kOzSlices >= kASlots ? 1u : 0u;
-                    pdl_wait();
-                    waited = true;
-                    const uint32_t dst = b_base;
-                    tc::mbar_expect_tx(b_full(0), prm.b_bytes);
-                    tc::tma_load_2d(dst, &tmB, c * kChunk, 0, b_full(0));
-                    tc::tma_load_2d(dst + (uint32_t)(3 * CP * 128), &tmB, c * kChunk, 3 * CP,
-                                    b_full(0));
-                    bc = 1;
-                    bq = 1 % kBSlots;
-                    bpar = kBSlots == 1 ? 1u : 0u;
-                    continue;
-                }
-                {
-                    // slot bq of the B ring, round bc / kBSlots (kept incrementally:
-                    // this one thread issues every copy of the SM)
-                    if (bc >= kBSlots &&
-                        !tc::mbar_wait(b_empty(bq), bpar ^ 1u, err, 12, false)) {
-                        abort_flag = 1;
-                        break;
-                    }
-                    const uint32_t dst = b_base + (uint32_t)bq * prm.b_bytes;
-                    tc::mbar_expect_tx(b_full(bq), prm.b_bytes);
-                    tc::tma_load_2d(dst, &tmB, c * kChunk, 0, b_full(bq));
-                    tc::tma_load_2d(dst + (uint32_t)(3 * CP * 128), &tmB, c * kChunk, 3 * CP,
-                                    b_full(bq));
-                    ++bc;
-                    if (++bq == kBSlots) {
-                        bq = 0;
-                        bpar ^= 1u;
-                    }
-                }
-                for (int s = 0; s < kOzSlices; ++s) {
-                    if (ac >= kASlots &&
-                        !tc::mbar_wait(a_empty(aq), apar ^ 1u, err, 11, false)) {
-                        abort_flag = 1;
-                        break;
-                    }
-                    tc::mbar_expect_tx(a_full(aq), kABytes);
-                    tc::tma_load_3d_hint(a_base + (uint32_t)aq * kABytes, &tmA, c * kChunk,
-                                         tile * kBM, s, a_full(aq), pol);
-                    ++ac;
-                    if (++aq == kASlots) {
-                        aq = 0;
-                        apar ^= 1u;
-                    }
-                }
-            }
-        }
-        if (!waited) pdl_wait();
-        a_issued = ac;
-        b_issued = bc;
-    } else if (warp == kMmaWarp && lane == 0) {
-        // ---- tcgen05.mma issuer ----
-        // instruction descriptor without its N field (bits 17-22)
-        const uint32_t ibase = prm.idesc & ~(0x3Fu << 17);
-        int ac = 0, bc = 0;
-        int aq = 0, bq = 0;
-        uint32_t apar = 0, bpar = 0;
-        int k = 0;
-        const int nb = prm.acc_bufs;
-        for (long long it = it0; it < it1 && !abort_flag; ++it, ++k) {
-            // accumulator set k % nb: wait until the epilogue has drained its
-            // previous use (item k - nb)
-            const int ab = k % nb;
-            const int use = k / nb;
-            if (use > 0 &&
-                !tc::mbar_wait(acc_empty(ab), (uint32_t)((use - 1) & 1), err, 13, false)) {
-                abort_flag = 1;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t acc_tmem = tmem + (uint32_t)(ab * kOzSlices * CP);
-            const int per = (int)(it % prm.periods);
-            const int c0 = per * kChunksPerPeriod;
-            const int c1 = min(prm.nchunks, c0 + kChunksPerPeriod);
-            bool first = true;
-            for (int c = c0; c < c1 && !abort_flag; ++c) {
-                const int qb = bq;
-                if (!tc::mbar_wait(b_full(qb), bpar, err, 14, false)) {
+    if (warp == kProducerWarp) {
+        if (lane == 0) {
+            // ---- TMA producer: the digit rows of X, one stage at a time ----
+            pdl_wait();  // the grid that wrote them
+            int q = 0, issued = 0;
+            uint32_t par = 0;
+            Walk w;
+            w.start(it0, prm);
+            while (w.it < it1 && !abort_flag) {
+                if (issued >= kBStages && !tc::mbar_wait(b_empty(q), par ^ 1u, err, 12, false)) {
                     abort_flag = 1;
                     break;
                 }
-                const uint32_t bsm = b_base + (uint32_t)qb * prm.b_bytes;
-                for (int s = 0; s < kOzSlices; ++s) {
-                    const int qa = aq;
-                    if (!tc::mbar_wait(a_full(qa), apar, err, 15, false)) {
-                        abort_flag = 1;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = tc::sw128_desc(a_base + (uint32_t)qa * kABytes);
-                    // one MMA for every pair (s, t <= 5 - s): the B slices t
-                    // lie in consecutive rows, so an MMA of N = (6 - s) cp
-                    // rows written at column s cp puts pair (s, t) into the
-                    // accumulator of level s + t (two MMAs when N exceeds
-                    // 256).  The first K step of an item (s = 0, which covers
-                    // every level) initialises the accumulators.
-                    const int nt = kOzSlices - s;
-                    const int t1 = nt * CP > 256 ? nt / 2 : nt;
-                    const uint64_t bd0 = tc::sw128_desc(bsm);
-                    const uint64_t bd1 = tc::sw128_desc(bsm + (uint32_t)(t1 * CP) * 128u);
-                    const uint32_t id0 = ibase | ((uint32_t)(t1 * CP) >> 3 << 17);
-                    const uint32_t id1 = ibase | ((uint32_t)((nt - t1) * CP) >> 3 << 17);
-                    const uint32_t acc_first = (first && s == 0) ? 0u : 1u;
+                const uint32_t dst = b0 + (uint32_t)q * kBBytes;
+                const int x = (w.per * prm.spp + w.st) * kStageK;
+                const int y = (int)(w.it / ((long long)prm.tiles * prm.periods)) * S * CP;
+                tc::mbar_expect_tx(b_full(q), prm.b_bytes);
+                tc::tma_load_2d(dst, &tmB, x, y, b_full(q));
+                if (prm.b_loads == 2) {
+                    tc::tma_load_2d(dst + (uint32_t)(S / 2 * CP * 64), &tmB, x, y + S / 2 * CP,
+                                    b_full(q));
+                }
+                ++issued;
+                if (++q == kBStages) {
+                    q = 0;
+                    par ^= 1u;
+                }
+                w.next(prm);
+            }
+            b_issued = issued;
+        }
+    } else if (warp == kWordsWarp) {
+        if (MODE == kWords && lane == 0) {
+            // ---- producer of the digit words (which no preceding kernel of
+            // the iteration writes), as far ahead as the converters free the
+            // ring ----
+            const uint64_t pol = prm.stream_h ? tc::l2_stream_policy() : l2_normal_policy();
+            int q = 0, issued = 0;
+            uint32_t par = 0;
+            Walk w;
+            w.start(it0, prm);
+            while (w.it < it1 && !abort_flag) {
+                if (issued >= kRawStages &&
+                    !tc::mbar_wait(raw_empty(q), par ^ 1u, err, 10, false)) {
+                    abort_flag = 1;
+                    break;
+                }
+                const size_t block = (size_t)w.tile * prm.nstages + (w.per * prm.spp + w.st);
+                tc::mbar_expect_tx(raw_full(q), kRawBytes);
+                bulk_load(raw0 + (uint32_t)q * kRawBytes, prm.words + block * (kRawBytes / 16),
+                          kRawBytes, raw_full(q), pol);
+                ++issued;
+                if (++q == kRawStages) {
+                    q = 0;
+                    par ^= 1u;
+                }
+                w.next(prm);
+            }
+            h_issued = issued;
+        }
+    } else if (warp == kMmaWarp) {
+        // ---- tcgen05.mma issuer: the whole warp walks the stages, one
+        // elected lane issues (see umma_f16_elect) ----
+        int q = 0, bq = 0;
+        uint32_t par = 0, bpar = 0;
+        bool ok = true;
+        Walk w;
+        w.start(it0, prm);
+        for (int k = 0; ok && w.it < it1; ++k) {
+            // accumulator set k % kSets: wait until its previous use (item
+            // k - kSets) has been drained
+            const int ab = k % kSets;
+            const int use = k / kSets;
+            if (use > 0) {
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_empty(ab), (uint32_t)((use - 1) & 1),
+                                                           err, 13, false));
+                if (!ok) break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + (uint32_t)(ab * V * CP);
+            const long long item = w.it;
+            bool first = true;
+            while (w.it == item) {
+                ok = tc::mbar_wait(b_full(bq), bpar, err, 14, false) &&
+                     tc::mbar_wait(a_full(q), par, err, 15, false);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t ad0 = sw64_desc(base + (uint32_t)q * Lay::kA);
+                const uint64_t bd0 = sw64_desc(b0 + (uint32_t)bq * kBBytes);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint32_t accum = kk > 0 ? 1u : acc_first;
-                        tc::umma<kLowpF16>(acc_tmem + (uint32_t)(s * CP), ad + (uint64_t)(2 * kk),
-                                           bd0 + (uint64_t)(2 * kk), id0, accum);
-                        if (t1 < nt) {
-                            tc::umma<kLowpF16>(acc_tmem + (uint32_t)((s + t1) * CP),
-                                               ad + (uint64_t)(2 * kk), bd1 + (uint64_t)(2 * kk),
-                                               id1, accum);
+                for (int kk = 0; kk < kStageK / 16; ++kk) {
+                    // the first K step of an item initialises the
+                    // accumulators: slice 0 those of its S levels, and
+                    // (V > S) slice 1 the one of level S
+                    const uint32_t acc_on = first && kk == 0 ? 0u : 1u;
+#pragma unroll
+                    for (int s = 0; s < S; ++s) {
+                        constexpr uint32_t kColStep = (uint32_t)(CP * 64) >> 4;
+                        const int nt = S < V - s ? S : V - s;
+                        const uint64_t ad =
+                            ad0 + (uint64_t)(s * (int)(kABytes >> 4) + 2 * kk);
+                        const uint64_t bd = bd0 + (uint64_t)(2 * kk);
+                        const uint32_t dst = acc + (uint32_t)(s * CP);
+                        auto mma = [&](int t0, int count, uint32_t accum) {
+                            tc::umma_f16_elect(dst + (uint32_t)(t0 * CP), ad,
+                                               bd + (uint64_t)(t0 * kColStep),
+                                               kIdesc | ((uint32_t)(count * CP) >> 3 << 17),
+                                               accum);
+                        };
+                        if (V > S && s == 1) {
+                            // level S starts here: its pair (1, S - 1) apart
+                            if (acc_on == 0u) {
+                                mma(0, nt - 1, 1u);
+                                mma(nt - 1, 1, 0u);
+                            } else {
+                                mma(0, nt, 1u);
+                            }
+                        } else if (nt * CP > 256) {
+                            mma(0, nt / 2, s == 0 ? acc_on : 1u);
+                            mma(nt / 2, nt - nt / 2, s == 0 ? acc_on : 1u);
+                        } else {
+                            mma(0, nt, s == 0 ? acc_on : 1u);
                         }
                     }
-                    tc::umma_commit(a_empty(qa));
-                    ++ac;
-                    if (++aq == kASlots) {
-                        aq = 0;
-                        apar ^= 1u;
-                    }
                 }
-                tc::umma_commit(b_empty(qb));
-                ++bc;
-                if (++bq == kBSlots) {
+                tc::umma_commit_elect(a_empty(q));
+                tc::umma_commit_elect(b_empty(bq));
+                if (++q == kStages) {
+                    q = 0;
+                    par ^= 1u;
+                }
+                if (++bq == kBStages) {
                     bq = 0;
                     bpar ^= 1u;
                 }
                 first = false;
+                w.next(prm);
             }
-            if (abort_flag) break;
-            tc::umma_commit(acc_full(ab));
+            if (ok) tc::umma_commit_elect(acc_full(ab));
         }
-        tc::umma_commit(mma_done);
-    } else if (warp < 4) {
-        // ---- epilogue: drain the six level accumulators every period ----
-        float Hs[CP], Ls[CP];
+        if (!ok) abort_flag = 1;
+        tc::umma_commit_elect(mma_done);
+    } else if (warp < kConvWarps) {
+        // ---- converters: a thread converts two runs of 8 K entries (groups
+        // g0 and g0 + 1 of the stage's four) of row r, lanes = rows ----
+        const int r = (int)threadIdx.x & 127;
+        const int g0 = 2 * ((int)threadIdx.x >> 7);
+        const uint64_t pol = prm.stream_h ? tc::l2_stream_policy() : l2_normal_policy();
+        const uint32_t my_raw = (uint32_t)(8 * g0 * kBM + r) * 8u;  // kRows
+        Walk w, lw;  // conversion and copy positions
+        w.start(it0, prm);
+        lw = w;
+        auto fetch = [&](int q) {  // kRows: the copies of the next stage, one group
+            if (lw.it < it1) {
+                fetch8(prm, lw, r, g0, pol, raw0 + (uint32_t)q * kRawBytes + my_raw);
+                fetch8(prm, lw, r, g0 + 1, pol,
+                       raw0 + (uint32_t)q * kRawBytes + my_raw + 8u * kBM * 8u);
+                lw.next(prm);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (MODE == kRows) {
+            for (int q = 0; q < kRawStages; ++q) fetch(q);
+        }
+        int q = 0, rq = 0, done = 0;
+        uint32_t par = 0, rpar = 0;
+        int e_row = 0, e_tile = -1;
+        bool good = true;
+        // the packed digits of this thread's 16 K entries of the stage at w,
+        // which then moves on
+        auto load = [&](uint4 (&x)[8]) {
+            if (MODE == kWords) {
+                if (!__all_sync(0xffffffffu, tc::mbar_wait(raw_full(rq), rpar, err, 9, false))) {
+                    good = false;
+                    return;
+                }
+                const uint32_t src = raw0 + (uint32_t)rq * kRawBytes + (uint32_t)(r * 256);
 #pragma unroll
-        for (int j = 0; j < CP; ++j) {
-            Hs[j] = 0.0f;
-            Ls[j] = 0.0f;
+                for (int j = 0; j < 8; ++j) {
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(x[j].x), "=r"(x[j].y), "=r"(x[j].z), "=r"(x[j].w)
+                                 : "r"(src + (uint32_t)(((4 * g0 + j) ^ (r & 7)) << 4))
+                                 : "memory");
+                }
+                // the slot may be refilled: every lane's reads precede the
+                // arrival (a release)
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(raw_empty(rq));
+            } else {
+                if (w.tile != e_tile) {
+                    e_tile = w.tile;
+                    const int row = w.tile * kBM + r;
+                    e_row = row < prm.n ? __ldg(prm.rowexp + row) : kOzNonFinite;
+                }
+                const int k0 = (w.per * prm.spp + w.st) * kStageK;
+                const bool on_diag = k0 < w.tile * kBM + kBM && k0 + kStageK > w.tile * kBM;
+                asm volatile("cp.async.wait_group %0;" ::"n"(kRawStages - 1) : "memory");
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    double v[8];
+                    const uint32_t src =
+                        raw0 + (uint32_t)rq * kRawBytes + my_raw + (uint32_t)(c * 8 * kBM * 8);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        asm volatile("ld.shared.f64 %0, [%1];"
+                                     : "=d"(v[u])
+                                     : "r"(src + (uint32_t)(u * kBM * 8))
+                                     : "memory");
+                    }
+                    if (on_diag) {  // Delta leaves the diagonal out
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            if (k0 + 8 * (g0 + c) + u == w.tile * kBM + r) v[u] = 0.0;
+                        }
+                    }
+                    if (e_row >= kOzFastExp) {
+                        const int nb = oz_shift_base<S>(e_row);
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            x[4 * c + p] = oz_pack_pair<S>(oz_biased<S>(v[2 * p], nb),
+                                                           oz_biased<S>(v[2 * p + 1], nb));
+                        }
+                    } else {
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            x[4 * c + p] = oz_pack_pair<S>(oz_biased_any<S>(v[2 * p], e_row),
+                                                           oz_biased_any<S>(v[2 * p + 1], e_row));
+                        }
+                    }
+                }
+                fetch(rq);
+            }
+            if (++rq == kRawStages) {
+                rq = 0;
+                rpar ^= 1u;
+            }
+            w.next(prm);
+        };
+        // their FP16 digits into the next slot of the A ring, one 16-byte run
+        // of K per slice and K group
+        auto emit = [&](const uint4 (&x)[8]) {
+            if (done >= kStages &&
+                !__all_sync(0xffffffffu, tc::mbar_wait(a_empty(q), par ^ 1u, err, 11, false))) {
+                good = false;
+                return;
+            }
+            const uint32_t row = base + (uint32_t)q * Lay::kA + (uint32_t)(r * 64);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t dst = row + (uint32_t)(((g0 + c) ^ ((r >> 1) & 3)) << 4);
+#pragma unroll
+                for (int s = S - 1; s >= 0; --s) {
+                    uint32_t h[4];
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) h[p] = oz_slice_pair<S>(x[4 * c + p], s);
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst +
+                                                                                  s * kABytes),
+                                 "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
+                                 : "memory");
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(a_full(q));
+            ++done;
+            if (++q == kStages) {
+                q = 0;
+                par ^= 1u;
+            }
+        };
+        // the words of the next stage are read before those of the current
+        // one are stored
+        uint4 xa[8], xb[8];
+        if (w.it < it1) load(xa);
+        while (good) {
+            const bool more = w.it < it1;
+            if (more) load(xb);
+            if (good) emit(xa);
+            if (!more || !good) break;
+            const bool again = w.it < it1;
+            if (again) load(xa);
+            if (good) emit(xb);
+            if (!again) break;
         }
-        const int row_local = warp * 32 + lane;
-        const int nb = prm.acc_bufs;
+        if (!good) abort_flag = 1;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        // ---- drain: the level accumulators of every item into running sums,
+        // warp = 32 rows x NC columns, and a tile's sums to its partial ----
+        const int drow = (warp & 3) * 32 + lane;
+        const int dcol = ((warp - kConvWarps) >> 2) * NC;
+        Sums<S, NC> sums;
+        sums.clear();
         int k = 0;
         for (long long it = it0; it < it1; ++it, ++k) {
-            const int ab = k % nb;
-            const uint32_t lane_addr =
-                tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(ab * kOzSlices * CP);
-            const bool ok =
-                tc::mbar_wait(acc_full(ab), (uint32_t)((k / nb) & 1), err, 16, true);
+            const int ab = k % kSets;
             // warp-uniform decision: the TMEM loads below are warp-collective
-            if (__any_sync(0xffffffffu, !ok || abort_flag)) {
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(acc_full(ab), (uint32_t)((k / kSets) & 1),
+                                                       err, 16, false))) {
                 abort_flag = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t addr =
+                tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ab * V * CP + dcol);
 #pragma unroll
-            for (int g = 0; g < CP / 16; ++g) {
-                float v0[16], v1[16], v2[16];
-                tc::tmem_ld_16cols_x3(lane_addr + (uint32_t)(16 * g), CP, v0, v1, v2);
-                float hh[16], ll[16];
+            for (int j0 = 0; j0 < NC; j0 += 4) {
+                uint32_t v[V][4];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float h, e1, e2;
-                    two_sum(v0[j], v1[j] * 0x1p-8f, h, e1);
-                    two_sum(h, v2[j] * 0x1p-16f, hh[j], e2);
-                    ll[j] = e1 + e2;
+                for (int l = 0; l < V; ++l) tmem_ld_4cols(addr + (uint32_t)(l * CP + j0), v[l]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (j0 + 4 >= NC) {
+                    // the last columns are in registers: the MMAs of a later
+                    // item may overwrite the set
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(acc_empty(ab));
                 }
-                tc::tmem_ld_16cols_x3(lane_addr + (uint32_t)(3 * CP + 16 * g), CP, v0, v1, v2);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float l = ll[j] + (v0[j] * 0x1p-24f + (v1[j] * 0x1p-32f +
-                                                                 v2[j] * 0x1p-40f));
-                    float s, e;
-                    two_sum(Hs[16 * g + j], hh[j], s, e);
-                    Hs[16 * g + j] = s;
-                    Ls[16 * g + j] += l + e;
+                for (int j = 0; j < 4; ++j) {
+                    uint32_t lv[V];
+#pragma unroll
+                    for (int l = 0; l < V; ++l) lv[l] = v[l][j];
+                    sums.add(j0 + j, lv);
                 }
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty(ab));
-            const long long tile = it / prm.periods;
-            const bool last = (it + 1 == it1) || ((it + 1) / prm.periods != tile);
-            if (last) {
-                const long long slot = (long long)blockIdx.x -
-                                       owner_of(tile * prm.periods, prm.items, G);
-                double *dst = P + ((size_t)(tile * prm.maxslots + slot) * prm.C) * kBM + row_local;
+            const long long gt = it / prm.periods;
+            if (it + 1 == it1 || (it + 1) / prm.periods != gt) {
+                const long long slot =
+                    (long long)blockIdx.x - owner_of(gt * prm.periods, prm.items, G);
+                double *dst = P + ((size_t)(gt * prm.maxslots + slot) * CP + dcol) * kBM + drow;
 #pragma unroll
-                for (int j = 0; j < CP; ++j) {
-                    if (j < prm.C) dst[(size_t)j * kBM] = (double)Hs[j] + (double)Ls[j];
-                    Hs[j] = 0.0f;
-                    Ls[j] = 0.0f;
-                }
+                for (int j = 0; j < NC; ++j) dst[(size_t)j * kBM] = sums.value(j);
+                sums.clear();
             }
         }
     }
@@ -384,14 +721,13 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         tc::mbar_wait(mma_done, 0u, err, 17, true);
         if (abort_flag) {
             // drain the copies still in flight (bounded)
-            const int ai = a_issued, bi = b_issued;
-            for (int i = max(0, ai - prm.a_slots); i < ai; ++i) {
-                tc::mbar_wait(a_full(i % prm.a_slots), (uint32_t)((i / prm.a_slots) & 1), err, 18,
-                              true);
+            const int bi = b_issued, hi = h_issued;
+            for (int i = max(0, bi - kBStages); i < bi; ++i) {
+                tc::mbar_wait(b_full(i % kBStages), (uint32_t)((i / kBStages) & 1), err, 18, true);
             }
-            for (int i = max(0, bi - prm.b_slots); i < bi; ++i) {
-                tc::mbar_wait(b_full(i % prm.b_slots), (uint32_t)((i / prm.b_slots) & 1), err,
-                              19, true);
+            for (int i = max(0, hi - kRawStages); i < hi; ++i) {
+                tc::mbar_wait(raw_full(i % kRawStages), (uint32_t)((i / kRawStages) & 1), err, 19,
+                              true);
             }
         }
     }
@@ -402,8 +738,22 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
 }
 
+__device__ __forceinline__ unsigned long long abs_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
+}
+
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long m)
+{
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
+        m = o > m ? o : m;
+    }
+    return m;
+}
+
 // Column maxima of |X| as bit patterns (colmax zeroed by the caller): grid
-// (column, row chunk), atomicMax per CTA.
+// (column, row chunk), atomicMax per warp.
 __global__ void oz_colmax_kernel(const double *__restrict__ X, long long ldx, int n,
                                  unsigned long long *__restrict__ colmax)
 {
@@ -412,120 +762,330 @@ __global__ void oz_colmax_kernel(const double *__restrict__ X, long long ldx, in
     const double *xc = X + (size_t)c * ldx;
     unsigned long long m = 0;
     for (int j = blockIdx.y * blockDim.x + threadIdx.x; j < n; j += gridDim.y * blockDim.x) {
-        const unsigned long long a =
-            (unsigned long long)__double_as_longlong(xc[j]) & 0x7FFFFFFFFFFFFFFFULL;
+        const unsigned long long a = abs_bits(xc[j]);
         m = a > m ? a : m;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
-        m = o > m ? o : m;
-    }
+    m = warp_max(m);
     if ((threadIdx.x & 31) == 0 && m != 0) atomicMax(colmax + c, m);
     pdl_trigger();
 }
 
-// B slices of X (columns c < C; zero rows for C <= c < cp): row t * cp + c
-// of B holds digit t of column c along K, zero beyond n.  Grid (column, K
-// chunk); colexp[c] records the column's exponent.
+// B slices of X: column c = group * cp + j of the padded block holds digit t
+// along K in row (group * S + t) * cp + j of B, zero beyond n and for
+// c >= C.  Grid (padded column, K chunk); colexp[c] records the column's
+// exponent; colmax_next (may be null) is cleared for the pass that writes
+// the next block.
+template <int S>
 __global__ void oz_slice_x_kernel(const double *__restrict__ X, long long ldx, int n, int C,
                                   int cp, int ldp, const unsigned long long *__restrict__ colmax,
+                                  unsigned long long *__restrict__ colmax_next,
                                   __half *__restrict__ B, int *__restrict__ colexp)
 {
     pdl_wait();
     const int c = blockIdx.x;
     const int e = c < C ? oz_exponent(colmax[c]) : 0;
-    if (blockIdx.y == 0 && threadIdx.x == 0 && c < C) colexp[c] = e;
+    if (blockIdx.y == 0 && threadIdx.x == 0 && c < C) {
+        colexp[c] = e;
+        if (colmax_next != nullptr) colmax_next[c] = 0;
+    }
     const double *xc = X + (size_t)c * ldx;
-    __half2 *row = reinterpret_cast<__half2 *>(B + (size_t)c * ldp);
-    const size_t stride = (size_t)cp * (size_t)ldp / 2;
-    for (int j = 2 * (blockIdx.y * blockDim.x + threadIdx.x); j < ldp;
-         j += 2 * gridDim.y * blockDim.x) {
-        const double v0 = (c < C && j < n) ? xc[j] : 0.0;
-        const double v1 = (c < C && j + 1 < n) ? xc[j + 1] : 0.0;
-        oz_store_pair(v0, v1, e, row + j / 2, stride);
+    uint2 *row = reinterpret_cast<uint2 *>(B + ((size_t)(c / cp) * S * cp + c % cp) * ldp);
+    const size_t stride = (size_t)cp * (size_t)ldp / 4;
+    for (int j = 4 * (blockIdx.y * blockDim.x + threadIdx.x); j < ldp;
+         j += 4 * gridDim.y * blockDim.x) {
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = (c < C && j + u < n) ? xc[j + u] : 0.0;
+        const uint4 p0 = oz_pack_pair<S>(oz_biased_any<S>(v[0], e), oz_biased_any<S>(v[1], e));
+        const uint4 p1 = oz_pack_pair<S>(oz_biased_any<S>(v[2], e), oz_biased_any<S>(v[3], e));
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            row[(size_t)s * stride + j / 4] =
+                make_uint2(oz_slice_pair<S>(p0, s), oz_slice_pair<S>(p1, s));
+        }
     }
     pdl_trigger();
 }
 
-// Y[:, c] = 2^(e_i + f_c - 16) (sum of the tile's partials) + d_i X[:, c].
-__global__ void oz_finish_kernel(const double *__restrict__ P, const int *__restrict__ rowexp,
-                                 const int *__restrict__ colexp, const double *__restrict__ d,
-                                 const double *__restrict__ X, long long ldx, int n, int C,
-                                 int periods, long long items, long long G, int maxslots,
-                                 double *__restrict__ Y, long long ldy)
+// What the consumers of the partials need.
+struct Partials {
+    const double *P;
+    const int *rowexp;
+    const int *colexp;
+    int n, cp, tiles, periods, maxslots, out;  // out: OzSplit::kOut
+    long long items, G;
+    const int *err;  // set by a product whose bounded wait gave up: its results are NaN
+};
+
+// Number of partials of column c's group in a tile.
+__device__ __forceinline__ int slots_of(const Partials &p, int c, int tile)
 {
+    if (tile >= p.tiles) return 0;
+    const long long gt = (long long)(c / p.cp) * p.tiles + tile;
+    return (int)(owner_of(gt * p.periods + p.periods - 1, p.items, p.G) -
+                 owner_of(gt * p.periods, p.items, p.G)) +
+           1;
+}
+
+// v 2^e; one multiplication where 2^e is a normal number.
+__device__ __forceinline__ double scale2(double v, int e)
+{
+    if (e > -1022 && e < 1023) return v * __hiloint2double((e + 1023) << 20, 0);
+    return ldexp(v, e);
+}
+
+// (Delta X)_ic from its `slots` partials, in their fixed order (finite row
+// and column scales).
+__device__ __forceinline__ double delta_entry(const Partials &p, int i, int c, int slots, int ei,
+                                              int fc)
+{
+    const int tile = i / kBM;
+    const int grp = c / p.cp;
+    const size_t gt = (size_t)grp * p.tiles + tile;
+    const double *q = p.P + ((size_t)(gt * p.maxslots) * p.cp + (c - grp * p.cp)) * kBM +
+                      (i - tile * kBM);
+    const size_t stride = (size_t)p.cp * kBM;
+    double s = 0.0;
+#pragma unroll 4
+    for (int u = 0; u < slots; ++u) s += q[u * stride];
+    return scale2(s, ei + fc + p.out);
+}
+
+constexpr int kFinishRows = 256;  // rows of one column a finish block covers
+
+// Y[:, c] = (Delta X)[:, c] + d_i X[:, c]; NaN where the row of Delta or the
+// column of X is not finite, or with H given (row i of H: H[i + l n]) the
+// FP64 sum over that row, whose Inf / NaN follow the operands'.
+__global__ void __launch_bounds__(kFinishRows)
+oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ H,
+                 const double *__restrict__ d, const double *__restrict__ X, long long ldx,
+                 int row_blocks, double *__restrict__ Y, long long ldy)
+{
+    constexpr int kTiles = kFinishRows / kBM;
+    __shared__ int slots[kTiles];
+    const int c = blockIdx.x / row_blocks;
+    const int row0 = (blockIdx.x % row_blocks) * kFinishRows;
+    const int i = row0 + threadIdx.x;
+    if (threadIdx.x < kTiles) slots[threadIdx.x] = slots_of(p, c, row0 / kBM + threadIdx.x);
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)n * (size_t)C) return;
-    const int i = (int)(e % (size_t)n);
-    const int c = (int)(e / (size_t)n);
-    const long long tile = i / kBM;
-    const int r = i - (int)tile * kBM;
-    const long long first = owner_of(tile * periods, items, G);
-    const long long last = owner_of(tile * periods + periods - 1, items, G);
-    double s = 0.0;
-    for (long long q = 0; q <= last - first; ++q) {
-        s += P[((size_t)(tile * maxslots + q) * C + c) * kBM + r];
+    if (i >= p.n) return;
+    const int ei = p.rowexp[i], fc = p.colexp[c];
+    double y;
+    if (*p.err != 0) {
+        y = NAN;
+    } else if (ei == kOzNonFinite || fc == kOzNonFinite) {
+        y = NAN;
+        if (H != nullptr) {
+            y = 0.0;
+            for (int l = 0; l < p.n; ++l) {
+                const double h = H[(size_t)i + (size_t)l * p.n];
+                if (l != i) y = fma(h, X[(size_t)l + (size_t)c * ldx], y);
+            }
+        }
+    } else {
+        y = delta_entry(p, i, c, slots[threadIdx.x / kBM], ei, fc);
     }
-    const int ei = rowexp[i], fc = colexp[c];
-    double y = (ei == kOzNonFinite || fc == kOzNonFinite) ? NAN : ldexp(s, ei + fc - 16);
     if (d != nullptr) y = fma(d[i], X[(size_t)i + (size_t)c * ldx], y);
     Y[(size_t)i + (size_t)c * ldy] = y;
 }
 
-// Row maxima of |H_il| (l != i) of a column-major H, as bit patterns.
-__global__ void oz_rowmax_kernel(const double *__restrict__ H, int n,
-                                 unsigned long long *__restrict__ rowmax)
-{
-    const int i = blockIdx.y * 32 + threadIdx.x;
-    const int l0 = blockIdx.x * 32;
-    if (i >= n) return;
-    unsigned long long m = 0;
-    for (int l = l0 + threadIdx.y; l < min(n, l0 + 32); l += blockDim.y) {
-        if (l == i) continue;
-        const unsigned long long a =
-            (unsigned long long)__double_as_longlong(H[(size_t)i + (size_t)l * n]) &
-            0x7FFFFFFFFFFFFFFFULL;
-        m = a > m ? a : m;
-    }
-    if (m != 0) atomicMax(rowmax + i, m);
-}
+// The IPT map from the partials of Delta X:
+//   c_j = (Delta X)_jj,  X'_ij = ((Delta X)_ij - X_ij c_j) g_ij,  X'_jj = 1
+// (IPT_C_GPU/src/ipt_cuda.cu:1369-1443), the column maxima of X' and with
+// want_norms ||X' - X||_F, ||X||_F (ipt_cuda.cu:1457-1467,1663-1688).  A row
+// of H or column of X that is not finite takes the FP64 sums the map is
+// defined by, so Inf and NaN travel as there.
+//
+// A block of 8 warps takes 256 R rows of one column, R per thread; a ninth
+// warp forms c_j while the others load.  With R = 4 the shuffle sums of the
+// norms (10 FP64 instructions per warp, each holding its partition's FP64
+// pipe for 64 cycles) are shared by four rows; R = 1 while the blocks of
+// R = 4 would not fill the chip.
+// n = 8192, k = 32: 13 us per step together with the digit pass of X.
+constexpr int kUpdateThreads = 256;
 
-// A slices of a column-major H: tile of 32 rows x 64 columns, read along
-// rows (coalesced), digits staged in shared memory, written along K.
-__global__ void oz_slice_h_kernel(const double *__restrict__ H, int n, int ldp,
-                                  const unsigned long long *__restrict__ rowmax,
-                                  __half *__restrict__ A, int *__restrict__ rowexp)
+template <int R>
+__global__ void __launch_bounds__(kUpdateThreads + 32)
+oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ H,
+                 const double *__restrict__ d, const double *__restrict__ g,
+                 const double *__restrict__ X, double *__restrict__ Xn,
+                 unsigned long long *__restrict__ colmax_next, int row_blocks, int want_norms,
+                 double2 *partials, unsigned int *counter, double *norms)
 {
-    __shared__ short dg[kOzSlices][32][66];
-    const int i0 = blockIdx.y * 32;
-    const int l0 = blockIdx.x * 64;
-    const int tx = threadIdx.x;  // 0..31
-    const int i = i0 + tx;
-    const int e = i < n ? oz_exponent(rowmax[i]) : 0;
-    if (blockIdx.x == 0 && threadIdx.y == 0 && i < n) rowexp[i] = e;
-    for (int ly = threadIdx.y; ly < 64; ly += blockDim.y) {
-        const int l = l0 + ly;
-        const double v = (i < n && l < n && l != i) ? H[(size_t)i + (size_t)l * n] : 0.0;
-        int dd[kOzSlices];
-        oz_digits_fast(v, e, dd);
+    constexpr int kRows = kUpdateThreads * R;
+    constexpr int kTiles = kRows / kBM;
+    __shared__ int slots[kTiles + 1];
+    __shared__ double cj_sh;
+    const int c = blockIdx.x / row_blocks;
+    const int row0 = (blockIdx.x % row_blocks) * kRows;
+    const int n = p.n;
+    const int t = (int)threadIdx.x;
+    if (t <= kTiles) slots[t] = slots_of(p, c, t < kTiles ? row0 / kBM + t : c / kBM);
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const double *xc = X + (size_t)c * n;
+    const int fc = p.colexp[c];
+    // (H X)_rc - d_r X_rc by the plain FP64 sum
+    auto direct = [&](int r) {
+        double y = 0.0;
+        for (int l = 0; l < n; ++l) y = fma(H[(size_t)r + (size_t)l * n], xc[l], y);
+        return y - d[r] * xc[r];
+    };
+    auto delta = [&](int r, int er, int count) {
+        return (er == kOzNonFinite || fc == kOzNonFinite) ? direct(r)
+                                                          : delta_entry(p, r, c, count, er, fc);
+    };
+    double y[R], x[R], gi[R];
+    if (t < kUpdateThreads) {
 #pragma unroll
-        for (int s = 0; s < kOzSlices; ++s) dg[s][tx][ly] = (short)dd[s];
+        for (int q = 0; q < R; ++q) {
+            const int i = row0 + q * kUpdateThreads + t;
+            y[q] = x[q] = gi[q] = 0.0;
+            if (i < n) {
+                x[q] = xc[i];
+                gi[q] = g[(size_t)i + (size_t)c * n];
+                y[q] = delta(i, p.rowexp[i], slots[(q * kUpdateThreads + t) / kBM]);
+            }
+        }
+    } else if (t == kUpdateThreads) {
+        cj_sh = delta(c, p.rowexp[c], slots[kTiles]);
     }
     __syncthreads();
-    // write: thread (tx, ty) covers column pair 2*tx of rows ty, ty + 8, ...
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int row = i0 + r;
-        if (row >= n) continue;
-        const int l = l0 + 2 * tx;
-        if (l >= ldp) continue;
+    const double cj = cj_sh;
+    const bool failed = *p.err != 0;
+    double dsq = 0.0, xsq = 0.0;
+    unsigned long long m = 0;
+    if (t < kUpdateThreads) {
 #pragma unroll
-        for (int s = 0; s < kOzSlices; ++s) {
-            reinterpret_cast<__half2 *>(A + ((size_t)s * n + row) * ldp + l)[0] =
-                oz_digit_pair(dg[s][r][2 * tx], dg[s][r][2 * tx + 1]);
+        for (int q = 0; q < R; ++q) {
+            const int i = row0 + q * kUpdateThreads + t;
+            if (i < n) {
+                double out = i == c ? 1.0 : fma(-x[q], cj, y[q]) * gi[q];
+                if (failed) out = NAN;
+                Xn[(size_t)i + (size_t)c * n] = out;
+                const unsigned long long a = abs_bits(out);
+                m = a > m ? a : m;
+                if (want_norms) {
+                    const double diff = out - x[q];
+                    dsq = fma(diff, diff, dsq);
+                    xsq = fma(x[q], x[q], xsq);
+                }
+            }
         }
     }
+    m = warp_max(m);
+    if ((t & 31) == 0 && m != 0) atomicMax(colmax_next + c, m);
+    if (want_norms) grid_finish_norms2(block_sum2(dsq, xsq), partials, counter, norms);
+}
+
+__global__ void gap_reciprocals_kernel(const double *__restrict__ d, int n, int k,
+                                       double *__restrict__ g)
+{
+    const int j = blockIdx.y;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double gap = d[j] - d[i];
+    g[(size_t)i + (size_t)j * n] = (isfinite(gap) && gap != 0.0) ? 1.0 / gap : NAN;
+}
+
+// Row maxima of |H_il| (l != i) of a column-major H, as bit patterns, and its
+// diagonal: 256 rows x kScanCols columns per block, two neighbouring rows per
+// thread (16-byte loads when n is even and H aligned), eight columns in flight.
+constexpr int kScanThreads = 128;
+constexpr int kScanCols = 64;
+
+template <bool VEC>
+__global__ void __launch_bounds__(kScanThreads)
+oz_rowmax_kernel(const double *__restrict__ H, int n, unsigned long long *__restrict__ rowmax,
+                 double *__restrict__ diag)
+{
+    const int i = (blockIdx.y * kScanThreads + threadIdx.x) * 2;
+    if (i >= n) return;
+    const int l0 = blockIdx.x * kScanCols;
+    const int l1 = min(n, l0 + kScanCols);
+    unsigned long long m0 = 0, m1 = 0;
+    for (int l = l0; l < l1; l += 8) {
+        double v0[8], v1[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const double *h = H + (size_t)(l + u) * n + i;
+            v0[u] = v1[u] = 0.0;
+            if (l + u < l1) {
+                if (VEC) {
+                    const double2 w = __ldcs(reinterpret_cast<const double2 *>(h));
+                    v0[u] = w.x;
+                    v1[u] = w.y;
+                } else {
+                    v0[u] = __ldcs(h);
+                    if (i + 1 < n) v1[u] = __ldcs(h + 1);
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const unsigned long long a0 = abs_bits(v0[u]), a1 = abs_bits(v1[u]);
+            if (l + u == i) {
+                if (diag != nullptr) diag[i] = v0[u];
+            } else {
+                m0 = a0 > m0 ? a0 : m0;
+            }
+            if (l + u == i + 1) {
+                if (diag != nullptr && l + u < l1) diag[i + 1] = v1[u];
+            } else {
+                m1 = a1 > m1 ? a1 : m1;
+            }
+        }
+    }
+    if (m0 != 0) atomicMax(rowmax + i, m0);
+    if (m1 != 0 && i + 1 < n) atomicMax(rowmax + i + 1, m1);
+}
+
+__global__ void oz_rowexp_kernel(const unsigned long long *__restrict__ rowmax, int n,
+                                 int *__restrict__ rowexp)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) rowexp[i] = oz_exponent(rowmax[i]);
+}
+
+// Digit words of Delta from H: one block per (K stage, row tile).  Lanes run
+// along rows (coalesced reads of H); the 32 KB block is put together in
+// shared memory in its final order and written as it lies.
+constexpr int kWordThreads = 512;
+
+template <int S>
+__global__ void __launch_bounds__(kWordThreads)
+oz_words_kernel(const double *__restrict__ H, int n, int nst, const int *__restrict__ rowexp,
+                uint4 *__restrict__ words)
+{
+    __shared__ uint4 img[kRawBytes / 16];
+    const int t = (int)threadIdx.x;
+    const int r = t & 127;
+    const int g = t >> 7;
+    const int row = blockIdx.y * kBM + r;
+    const int l0 = blockIdx.x * kStageK + 8 * g;
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const int l = l0 + u;
+        v[u] = (row < n && l < n) ? __ldcs(H + (size_t)l * n + row) : 0.0;
+    }
+    const int e = row < n ? rowexp[row] : kOzNonFinite;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        if (l0 + u == row) v[u] = 0.0;
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        img[r * 16 + ((4 * g + p) ^ (r & 7))] =
+            oz_pack_pair<S>(oz_biased_any<S>(v[2 * p], e), oz_biased_any<S>(v[2 * p + 1], e));
+    }
+    __syncthreads();
+    uint4 *dst = words + ((size_t)blockIdx.y * nst + blockIdx.x) * (kRawBytes / 16);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dst[q * kWordThreads + t] = img[q * kWordThreads + t];
 }
 
 }  // namespace oz
@@ -533,49 +1093,120 @@ __global__ void oz_slice_h_kernel(const double *__restrict__ H, int n, int ldp,
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
-int OzDelta::init_storage(int n_, cudaStream_t s)
+int OzMatrix::init_storage(int n_, cudaStream_t s)
 {
     n = n_;
-    ldp = (n + 63) / 64 * 64;
-    IPTGB_CHECK(A.alloc((size_t)kOzSlices * n * ldp, s));
-    IPTGB_CHECK(rowexp.alloc((size_t)n, s));
-    return make_map_3d(&mapA, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, A.ptr, ldp, n, kOzSlices,
-                       oz::kBM);
+    nst = (n + oz::kStageK - 1) / oz::kStageK;
+    words_slices = 0;
+    return rowexp.alloc((size_t)n, s);
 }
 
-int OzDelta::split_from(const double *H, int n_, cudaStream_t s)
+int OzMatrix::alloc_words(int slices, cudaStream_t s)
+{
+    const size_t blocks = (size_t)((n + oz::kBM - 1) / oz::kBM) * nst;
+    IPTGB_CHECK(words.alloc(blocks * (oz::kRawBytes / 16), s));
+    words_slices = slices;
+    return IPT_CUDA_SUCCESS;
+}
+
+int OzMatrix::build_words(int slices, cudaStream_t s)
+{
+    const size_t tiles = (size_t)(n + oz::kBM - 1) / oz::kBM;
+    if (tiles * nst * oz::kRawBytes > kMaxWordBytes) return IPT_CUDA_SUCCESS;
+    if (alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
+        cudaGetLastError();  // not enough memory: the product reads H itself
+        words_slices = 0;
+        return IPT_CUDA_SUCCESS;
+    }
+    auto kernel = slices == 7 ? oz::oz_words_kernel<7> : oz::oz_words_kernel<6>;
+    kernel<<<dim3((unsigned)nst, (unsigned)tiles), oz::kWordThreads, 0, s>>>(H, n, nst, rowexp.ptr,
+                                                                            words.ptr);
+    IPTGB_LAUNCH();
+    return IPT_CUDA_SUCCESS;
+}
+
+int OzMatrix::scan_rows(const double *H_, int n_, double *diag, cudaStream_t s)
 {
     IPTGB_CHECK(init_storage(n_, s));
+    H = H_;
     DeviceBuffer<unsigned long long> rm;
     IPTGB_CHECK(rm.alloc((size_t)n, s));
     IPTGB_CUDA(cudaMemsetAsync(rm.ptr, 0, (size_t)n * sizeof(unsigned long long), s));
-    const dim3 g1((n + 31) / 32, (n + 31) / 32);
-    oz::oz_rowmax_kernel<<<g1, dim3(32, 8), 0, s>>>(H, n, rm.ptr);
+    const int rows = 2 * oz::kScanThreads;
+    const dim3 grid((n + oz::kScanCols - 1) / oz::kScanCols, (n + rows - 1) / rows);
+    const bool vec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0;
+    auto scan = vec ? oz::oz_rowmax_kernel<true> : oz::oz_rowmax_kernel<false>;
+    scan<<<grid, oz::kScanThreads, 0, s>>>(H, n, rm.ptr, diag);
     IPTGB_LAUNCH();
-    const dim3 g2(ldp / 64, (n + 31) / 32);
-    oz::oz_slice_h_kernel<<<g2, dim3(32, 8), 0, s>>>(H, n, ldp, rm.ptr, A.ptr, rowexp.ptr);
+    oz::oz_rowexp_kernel<<<blocks_for((size_t)n), kThreads, 0, s>>>(rm.ptr, n, rowexp.ptr);
     IPTGB_LAUNCH();
     return IPT_CUDA_SUCCESS;
 }
 
 namespace {
 
-template <int CP>
-int launch_product(const CUtensorMap &mapA, const CUtensorMap &mapB, const oz::Params &prm,
-                   int grid, size_t smem, double *P, int *err, cudaStream_t s)
+// Columns per group: up to 64 for the 48-bit split (its 6 level accumulators
+// then fill TMEM), 32 for the 56-bit split (8 levels, two accumulator sets).
+int group_cols(int slices, int C)
 {
-    auto kfn = oz::oz_product_kernel<CP>;
+    const int most = slices == 7 ? 32 : 64;
+    return std::min(most, (C + 15) / 16 * 16);
+}
+
+template <int S, int CP, int MODE>
+int launch_product(const CUtensorMap &mapB, const oz::Params &prm, int grid, double *P, int *err,
+                   cudaStream_t s)
+{
+    auto kfn = oz::oz_product_kernel<S, CP, MODE>;
+    constexpr size_t smem = oz::Layout<S, CP>::kSmem;
     IPTGB_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return launch_pdl(kfn, dim3(grid), dim3(oz::kThreads), smem, s, mapA, mapB, prm, P, err);
+    return launch_pdl(kfn, dim3(grid), dim3(oz::kThreads), smem, s, mapB, prm, P, err);
+}
+
+template <int MODE>
+int launch_product_for(int slices, int cp, const CUtensorMap &mapB, const oz::Params &prm, int grid,
+                       double *P, int *err, cudaStream_t s)
+{
+    if (slices == 7) {
+        return cp == 16 ? launch_product<7, 16, MODE>(mapB, prm, grid, P, err, s)
+                        : launch_product<7, 32, MODE>(mapB, prm, grid, P, err, s);
+    }
+    switch (cp) {
+    case 16: return launch_product<6, 16, MODE>(mapB, prm, grid, P, err, s);
+    case 32: return launch_product<6, 32, MODE>(mapB, prm, grid, P, err, s);
+    case 48: return launch_product<6, 48, MODE>(mapB, prm, grid, P, err, s);
+    default: return launch_product<6, 64, MODE>(mapB, prm, grid, P, err, s);
+    }
+}
+
+int make_tile_map(CUtensorMap *map, CUtensorMapDataType dt, int esize, const void *base,
+                  size_t inner, size_t outer, int box_inner, int box_outer, CUtensorMapSwizzle sw)
+{
+    EncodeTiledFn fn = encode_fn();
+    if (fn == nullptr) return IPT_CUDA_CUDA_ERROR;
+    cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
+    cuuint64_t strides[1] = {(cuuint64_t)inner * esize};
+    cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
+    cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        fprintf(stderr, "ipt_gb300: cuTensorMapEncodeTiled failed (%d)\n", (int)r);
+        return IPT_CUDA_CUDA_ERROR;
+    }
+    return IPT_CUDA_SUCCESS;
 }
 
 }  // namespace
 
-int OzProduct::bind(const OzDelta *delta, const double *diag, cudaStream_t stream)
+int OzProduct::bind(const OzMatrix *matrix, const double *diag, int digit_slices,
+                    cudaStream_t stream)
 {
-    dl = delta;
+    m = matrix;
     d = diag;
     s = stream;
+    slices = digit_slices;
     sms = device_sm_count();
     if (err.ptr == nullptr) {
         IPTGB_CHECK(err.alloc(1, s));
@@ -584,79 +1215,153 @@ int OzProduct::bind(const OzDelta *delta, const double *diag, cudaStream_t strea
     return IPT_CUDA_SUCCESS;
 }
 
-int OzProduct::apply_group(const double *X, long long ldx, int C, double *Y, long long ldy)
+int OzProduct::shape_for(int C)
 {
-    const int n = dl->n;
-    const int ldp = dl->ldp;
-    const int cp = (C + 15) / 16 * 16;
-    if (C <= 0 || cp > kOzMaxCols) return IPT_CUDA_INVALID_ARGUMENT;
-    if (cp != cp_cur) {
-        IPTGB_CHECK(B.alloc((size_t)kOzSlices * cp * ldp, s));
-        IPTGB_CHECK(colexp.alloc((size_t)cp, s));
-        IPTGB_CHECK(colmax.alloc((size_t)cp, s));
-        IPTGB_CHECK(make_map(&mapB, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B.ptr, ldp, kOzSlices * cp,
-                             3 * cp));
-        cp_cur = cp;
+    if (sh.C == C && sh.n == m->n) return IPT_CUDA_SUCCESS;
+    const int n = m->n;
+    OzShape q;
+    q.n = n;
+    q.C = C;
+    q.cp = group_cols(slices, C);
+    q.groups = (C + q.cp - 1) / q.cp;
+    q.tiles = (n + oz::kBM - 1) / oz::kBM;
+    q.ldp = (n + 63) / 64 * 64;
+    // Items of kOzPeriod K elements, or (56-bit split, whose sums do not depend
+    // on it) half or a quarter of that while it shortens the longest CTA: a
+    // matrix of a few tiles then spreads over more SMs
+    const int nst = (n + oz::kStageK - 1) / oz::kStageK;
+    long long best = LLONG_MAX;
+    for (int spp = oz::kMaxStagesPerItem; spp >= (slices == 7 ? 1 : oz::kMaxStagesPerItem);
+         spp /= 2) {
+        const int periods = (nst + spp - 1) / spp;
+        const long long items = (long long)q.groups * q.tiles * periods;
+        const long long longest = (items + sms - 1) / sms * spp;
+        if (longest >= best) continue;
+        best = longest;
+        q.spp = spp;
+        q.periods = periods;
+        q.items = items;
     }
-    oz::Params prm = {};
-    prm.n = n;
-    prm.C = C;
-    prm.cp = cp;
-    prm.nchunks = ldp / oz::kChunk;
-    prm.periods = (prm.nchunks + oz::kChunksPerPeriod - 1) / oz::kChunksPerPeriod;
-    const int tiles = (n + oz::kBM - 1) / oz::kBM;
-    prm.items = (long long)tiles * prm.periods;
-    const int grid = (int)std::min<long long>(sms, prm.items);
-    int maxslots = 1;
-    for (int t = 0; t < tiles; ++t) {
-        const long long f = tc::owner_of((long long)t * prm.periods, prm.items, grid);
-        const long long l = tc::owner_of((long long)t * prm.periods + prm.periods - 1, prm.items,
-                                         grid);
-        maxslots = std::max(maxslots, (int)(l - f + 1));
+    q.grid = (int)std::min<long long>(sms, q.items);
+    q.maxslots = 1;
+    for (long long t = 0; t < (long long)q.groups * q.tiles; ++t) {
+        const long long f = tc::owner_of(t * q.periods, q.items, q.grid);
+        const long long l = tc::owner_of(t * q.periods + q.periods - 1, q.items, q.grid);
+        q.maxslots = std::max(q.maxslots, (int)(l - f + 1));
     }
-    prm.maxslots = maxslots;
-    prm.b_bytes = (uint32_t)(kOzSlices * cp * 128);
-    prm.b_slots = oz::kMaxBSlots;
-    // as many A slices in flight as the shared memory holds (>= one chunk)
-    const size_t budget = 225u * 1024u - (size_t)prm.b_slots * prm.b_bytes;
-    prm.a_slots = (int)std::min<size_t>(oz::kMaxASlots, budget / oz::kABytes);
-    if (prm.a_slots < kOzSlices) return IPT_CUDA_INVALID_ARGUMENT;
-    prm.acc_bufs = 2 * kOzSlices * cp <= 512 ? 2 : 1;
-    prm.idesc = (1u << 4) | ((uint32_t)(cp >> 3) << 17) | ((uint32_t)(oz::kBM >> 4) << 24);
-    const size_t pneed = (size_t)tiles * maxslots * C * oz::kBM;
+    const size_t rows = (size_t)q.groups * slices * q.cp;
+    const size_t bneed = rows * q.ldp;
+    const size_t pneed = (size_t)q.groups * q.tiles * q.maxslots * q.cp * oz::kBM;
+    const size_t cneed = (size_t)q.groups * q.cp;
+    if (B.count < bneed) IPTGB_CHECK(B.alloc(bneed, s));
+    if (colexp.count < cneed) IPTGB_CHECK(colexp.alloc(cneed, s));
+    if (colmax.count < 2 * cneed) IPTGB_CHECK(colmax.alloc(2 * cneed, s));
     if (P.count < pneed) IPTGB_CHECK(P.alloc(pneed, s));
-    const size_t smem = 1024 + (size_t)prm.a_slots * oz::kABytes +
-                        (size_t)prm.b_slots * prm.b_bytes +
-                        (2 * oz::kMaxASlots + 2 * oz::kMaxBSlots + 5) * 8 + 16;
+    cur = 0;
+    // digits: box of 64 bytes of K x the rows of a group (half of them when
+    // they exceed the 256 rows a box may have)
+    const int box_rows = slices * q.cp <= 256 ? slices * q.cp : slices / 2 * q.cp;
+    IPTGB_CHECK(make_tile_map(&mapB, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, B.ptr, q.ldp, rows,
+                              oz::kStageK, box_rows, CU_TENSOR_MAP_SWIZZLE_64B));
+    sh = q;
+    return IPT_CUDA_SUCCESS;
+}
 
-    // X split: column maxima, then the digit slices (grids of about 4 CTAs per SM)
-    IPTGB_CUDA(cudaMemsetAsync(colmax.ptr, 0, (size_t)cp * sizeof(unsigned long long), s));
-    const int ychunks = std::max(1, std::min((n + 2047) / 2048, (4 * sms + cp - 1) / cp));
-    IPTGB_CHECK(launch_pdl(oz::oz_colmax_kernel, dim3(C, ychunks), dim3(256), 0, s, X, ldx, n,
-                           colmax.ptr));
-    IPTGB_CHECK(launch_pdl(oz::oz_slice_x_kernel, dim3(cp, ychunks), dim3(256), 0, s, X, ldx, n,
-                           C, cp, ldp, (const unsigned long long *)colmax.ptr, B.ptr,
+// B slices of X from the maxima of set `cur` (clearing the other set), then
+// the partials of Delta X.
+int OzProduct::slice_and_multiply(const double *X, long long ldx, int clear_other)
+{
+    const OzShape &q = sh;
+    const size_t set = (size_t)q.groups * q.cp;
+    const int pc = q.groups * q.cp;
+    const int ychunks = std::max(1, std::min((q.ldp + 1023) / 1024, (8 * sms + pc - 1) / pc));
+    auto slice = slices == 7 ? oz::oz_slice_x_kernel<7> : oz::oz_slice_x_kernel<6>;
+    IPTGB_CHECK(launch_pdl(slice, dim3(pc, ychunks), dim3(256), 0, s, X, ldx, q.n, q.C, q.cp,
+                           q.ldp, (const unsigned long long *)(colmax.ptr + cur * set),
+                           clear_other ? colmax.ptr + (1 - cur) * set : nullptr, B.ptr,
                            colexp.ptr));
-    int st;
-    switch (cp) {
-    case 16: st = launch_product<16>(dl->mapA, mapB, prm, grid, smem, P.ptr, err.ptr, s); break;
-    case 32: st = launch_product<32>(dl->mapA, mapB, prm, grid, smem, P.ptr, err.ptr, s); break;
-    case 48: st = launch_product<48>(dl->mapA, mapB, prm, grid, smem, P.ptr, err.ptr, s); break;
-    default: st = launch_product<64>(dl->mapA, mapB, prm, grid, smem, P.ptr, err.ptr, s); break;
-    }
-    IPTGB_CHECK(st);
-    return launch_pdl(oz::oz_finish_kernel, dim3(blocks_for((size_t)n * C)), dim3(kThreads), 0, s,
-                      (const double *)P.ptr, (const int *)dl->rowexp.ptr,
-                      (const int *)colexp.ptr, d, X, ldx, n, C, prm.periods, prm.items,
-                      (long long)grid, maxslots, Y, ldy);
+    oz::Params prm = {};
+    prm.H = m->H;
+    prm.words = m->words.ptr;
+    prm.rowexp = m->rowexp.ptr;
+    prm.n = q.n;
+    prm.groups = q.groups;
+    prm.tiles = q.tiles;
+    prm.periods = q.periods;
+    prm.spp = q.spp;
+    prm.nstages = m->nst;
+    prm.items = q.items;
+    prm.maxslots = q.maxslots;
+    prm.stream_h = (size_t)q.n * q.n * sizeof(double) > oz::kL2ResidentBytes;
+    prm.b_loads = slices * q.cp <= 256 ? 1 : 2;
+    prm.b_bytes = (uint32_t)(slices * q.cp * 64);
+    auto launch = m->words_slices == slices ? launch_product_for<oz::kWords>
+                                            : launch_product_for<oz::kRows>;
+    return launch(slices, q.cp, mapB, prm, q.grid, P.ptr, err.ptr, s);
+}
+
+oz::Partials OzProduct::partials() const
+{
+    oz::Partials p;
+    p.P = P.ptr;
+    p.rowexp = m->rowexp.ptr;
+    p.colexp = colexp.ptr;
+    p.n = sh.n;
+    p.cp = sh.cp;
+    p.tiles = sh.tiles;
+    p.periods = sh.periods;
+    p.maxslots = sh.maxslots;
+    p.out = slices == 7 ? OzSplit<7>::kOut : OzSplit<6>::kOut;
+    p.items = sh.items;
+    p.G = sh.grid;
+    p.err = err.ptr;
+    return p;
+}
+
+int OzProduct::scan_columns(const double *X, long long ldx)
+{
+    const size_t set = (size_t)sh.groups * sh.cp;
+    IPTGB_CUDA(cudaMemsetAsync(colmax.ptr + cur * set, 0, set * sizeof(unsigned long long), s));
+    const int ychunks = std::max(1, std::min((sh.n + 2047) / 2048, (4 * sms + sh.C - 1) / sh.C));
+    return launch_pdl(oz::oz_colmax_kernel, dim3(sh.C, ychunks), dim3(256), 0, s, X, ldx, sh.n,
+                      colmax.ptr + cur * set);
 }
 
 int OzProduct::apply(const double *X, long long ldx, int C, double *Y, long long ldy)
 {
-    for (int c0 = 0; c0 < C; c0 += kOzMaxCols) {
-        const int cc = std::min(kOzMaxCols, C - c0);
-        IPTGB_CHECK(apply_group(X + (size_t)c0 * ldx, ldx, cc, Y + (size_t)c0 * ldy, ldy));
+    if (C <= 0) return IPT_CUDA_SUCCESS;
+    IPTGB_CHECK(shape_for(C));
+    IPTGB_CHECK(scan_columns(X, ldx));
+    IPTGB_CHECK(slice_and_multiply(X, ldx, 0));
+    const int row_blocks = (sh.n + oz::kFinishRows - 1) / oz::kFinishRows;
+    return launch_pdl(oz::oz_finish_kernel, dim3((unsigned)((long long)row_blocks * C)),
+                      dim3(oz::kFinishRows), 0, s, partials(),
+                      slices == 7 ? m->H : (const double *)nullptr, d, X, ldx, row_blocks, Y, ldy);
+}
+
+int OzProduct::begin(const double *X, int C)
+{
+    IPTGB_CHECK(shape_for(C));
+    return scan_columns(X, sh.n);
+}
+
+int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns)
+{
+    const int r1 = (sh.n + oz::kUpdateThreads - 1) / oz::kUpdateThreads;
+    const bool wide = (long long)((r1 + 3) / 4) * sh.C >= sms;
+    const int row_blocks = wide ? (r1 + 3) / 4 : r1;
+    const long long grid = (long long)row_blocks * sh.C;
+    if (want_norms && grid > ns->capacity) return IPT_CUDA_INVALID_ARGUMENT;
+    const size_t set = (size_t)sh.groups * sh.cp;
+    {
+        KernelTimerScope timer(kProfFp64Product, s);
+        IPTGB_CHECK(slice_and_multiply(X, sh.n, 1));
     }
+    KernelTimerScope timer(kProfFp64Update, s);
+    IPTGB_CHECK(launch_pdl(wide ? oz::oz_update_kernel<4> : oz::oz_update_kernel<1>,
+                           dim3((unsigned)grid), dim3(oz::kUpdateThreads + 32), 0, s, partials(), m->H, d, g, X, Xn, colmax.ptr + (1 - cur) * set, row_blocks,
+                           want_norms, ns->partials, ns->counter, ns->norms));
+    cur = 1 - cur;
     return IPT_CUDA_SUCCESS;
 }
 
@@ -664,6 +1369,14 @@ int OzProduct::read_error(int *host_err)
 {
     IPTGB_CUDA(cudaMemcpyAsync(host_err, err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
     IPTGB_CUDA(cudaStreamSynchronize(s));
+    return IPT_CUDA_SUCCESS;
+}
+
+int launch_gap_reciprocals(const double *d, int n, int k, double *g, cudaStream_t s)
+{
+    oz::gap_reciprocals_kernel<<<dim3((n + kThreads - 1) / kThreads, k), kThreads, 0, s>>>(d, n, k,
+                                                                                          g);
+    IPTGB_LAUNCH();
     return IPT_CUDA_SUCCESS;
 }
 
@@ -683,13 +1396,12 @@ IPT_API int ipt_block_accurate_product(const double *d_H, int n, const double *d
         return IPT_CUDA_INVALID_ARGUMENT;
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    OzDelta delta;
-    IPTGB_CHECK(delta.split_from(d_H, n, s));
     DeviceBuffer<double> d;
     IPTGB_CHECK(d.alloc((size_t)n, s));
-    IPTGB_CHECK(launch_extract_diagonal(d_H, n, n, d.ptr, s));
+    OzMatrix matrix;
+    IPTGB_CHECK(matrix.scan_rows(d_H, n, d.ptr, s));
     OzProduct prod;
-    IPTGB_CHECK(prod.bind(&delta, d.ptr, s));
+    IPTGB_CHECK(prod.bind(&matrix, d.ptr, kOzSlices, s));
     IPTGB_CHECK(prod.apply(d_X, n, c, d_Y, n));
     int herr = 0;
     IPTGB_CHECK(prod.read_error(&herr));

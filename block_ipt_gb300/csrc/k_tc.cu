@@ -1037,7 +1037,7 @@ __global__ void __launch_bounds__(256)
                        double *__restrict__ copy, LP *__restrict__ delta, float *__restrict__ hi,
                        float *__restrict__ lo, float *__restrict__ inv_row,
                        double *__restrict__ diag, DenseStats *__restrict__ stats, int vec,
-                       __half *__restrict__ oz, int *__restrict__ oz_rowexp, int c0)
+                       int *__restrict__ oz_rowexp, uint4 *__restrict__ oz_words, int c0)
 {
     __shared__ unsigned long long wmax[8];
     __shared__ float wS[8], wC[8];
@@ -1090,8 +1090,9 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     const int s2 = s2_sh;
     const double scale = ldexp(1.0, s2);
-    // exponent of row c's digit slices (symmetric H: column c is row c)
+    // exponent and digit words of row c (symmetric H: column c is row c)
     const int oz_e = oz_exponent(wmax[0]);
+    const int oz_nst = (n + 31) / 32;
     // the block's pass-0 writes of the copy are visible after the barrier;
     // pass 1 reads with ld.global.cg (coherent at L2), never through the
     // read-only path, since the copy is written by this kernel
@@ -1114,10 +1115,10 @@ __global__ void __launch_bounds__(256)
         if (!(l < n && l != c)) v0 = 0.0f;
         if (!(l + 1 < n && l + 1 != c)) v1 = 0.0f;
         *reinterpret_cast<LpPair<LP> *>(orow + l) = LpPair<LP>{to_lp<LP>(v0), to_lp<LP>(v1)};
-        if (oz != nullptr) {
-            oz_store_pair((l < n && l != c) ? h0 : 0.0, (l + 1 < n && l + 1 != c) ? h1 : 0.0,
-                          oz_e, reinterpret_cast<__half2 *>(oz + (size_t)c * ldp + l),
-                          (size_t)n * (size_t)ldp / 2);
+        if (oz_words != nullptr && l < 32 * oz_nst) {
+            oz_words[oz_word_index(c, l, oz_nst)] = oz_pack_pair<kOzSlices>(
+                oz_biased_any<kOzSlices>((l < n && l != c) ? h0 : 0.0, oz_e),
+                oz_biased_any<kOzSlices>((l + 1 < n && l + 1 != c) ? h1 : 0.0, oz_e));
         }
         df_abs_add(S, C, a0, b0);  // entries beyond n are zero
         df_abs_add(S, C, a1, b1);
@@ -1940,14 +1941,13 @@ struct LowpDense final : LowpDenseOperator {
                 kfn<<<n, 256, 0, s>>>(su.fused_src, n, ldp,
                                          LowpTypes<LP>::kind == kLowpF16 ? 1 : 0, su.fused_copy,
                                          delta.ptr, split_hi, split_lo, inv_rows.ptr, su.diag,
-                                         su.stats, vec, su.oz, su.oz_rowexp, 0);
+                                         su.stats, vec, su.oz_rowexp, su.oz_words, 0);
                 IPTGB_LAUNCH();
             }
             scale = 1.0;  // per-row scales in inv_rows
             per_row_scales = true;
             su.fused_done = true;
             su.split_done = split_hi != nullptr;
-            su.oz_done = su.oz != nullptr && su.oz_rowexp != nullptr;
             IPTGB_CHECK(make_map(&mapA, LowpTypes<LP>::dt, esize, delta.ptr, ldp, n, tc::kBM));
             IPTGB_CHECK(err.alloc(1, s));
             IPTGB_CUDA(cudaMemsetAsync(err.ptr, 0, sizeof(int), s));
@@ -2064,7 +2064,7 @@ struct LowpDense final : LowpDenseOperator {
             count_launch();
             fused_setup_kernel<LP><<<c1 - c0, 256, 0, s2>>>(
                 su.fused_copy, n, ldp, LowpTypes<LP>::kind == kLowpF16 ? 1 : 0, nullptr, delta.ptr,
-                split_hi, split_lo, inv_rows.ptr, su.diag, su.stats, vec, su.oz, su.oz_rowexp, c0);
+                split_hi, split_lo, inv_rows.ptr, su.diag, su.stats, vec, su.oz_rowexp, su.oz_words, c0);
             if (cudaGetLastError() != cudaSuccess) {
                 fail(IPT_CUDA_CUDA_ERROR);
                 break;

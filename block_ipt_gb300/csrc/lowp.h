@@ -89,12 +89,10 @@ struct LowpDenseSetup {
     double *diag = nullptr;         // n entries
     DenseStats *stats = nullptr;    // device, zeroed by the caller
     bool fused_done = false;        // out
-    // fused setup only: the digit slices of Delta for the FP64-accurate
-    // tensor-core product ([kOzSlices][n][ldp] FP16, ldp = n rounded up to
-    // 64) and their row exponents (oz.cuh)
-    __half *oz = nullptr;
+    // fused setup only: the exponents of Delta's rows and its digit words for
+    // the FP64-accurate tensor-core product (oz.cuh)
     int *oz_rowexp = nullptr;
-    bool oz_done = false;           // out
+    uint4 *oz_words = nullptr;
 };
 constexpr int kLowpColsumChunk = 2048;
 LowpDenseOperator *make_lowp_dense_operator(const double *dH, int n, int kind, cudaStream_t s,

@@ -1,4 +1,4 @@
-// oz.cuh - operand splitting of the FP64-accurate tensor-core product
+// oz.cuh - operand splitting of the FP64-accurate tensor-core products
 // (internal; host and device).
 //
 // The product Y = Delta X with FP64 operands runs on the FP16 tensor cores
@@ -10,20 +10,29 @@
 // Reproducible Versions", ISC 2020):
 //
 //  * every row i of Delta is scaled by 2^-e_i, e_i the smallest exponent
-//    with max_j |Delta_ij| < 2^e_i, and rounded to the 48-bit integer
-//    Q_ij = round(Delta_ij 2^(48 - e_i)); every column c of X likewise with
+//    with max_j |Delta_ij| < 2^e_i, and rounded to the fixed-point integer
+//    Q_ij = round(Delta_ij 2^(F - e_i)); every column c of X likewise with
 //    its own exponent f_c;
-//  * Q is written in kOzSlices balanced base-256 digits,
-//    Q = sum_{s=0..5} A_s 256^(5-s), A_0 in [-256, 256], A_s in [-128, 127]
-//    for s > 0: small integers that FP16 holds exactly;
-//  * Delta X = 2^(e_i + f_c - 16) sum_l 2^(-8 l) L_l with the level sums
-//    L_l = sum_{s+t=l} A_s B_t over the levels l = 0..kOzSlices-1 (the
-//    products of lower weight are dropped: each is below 2^-47 of the
-//    fixed-point scale).  Every product of two digits is an integer below
-//    2^16 in magnitude and every level sum over kOzPeriod consecutive K
-//    elements stays below 2^24, so the tensor cores' FP32 accumulation adds
-//    integers exactly; the accumulators are drained every kOzPeriod K
-//    elements and combined in double-float arithmetic.
+//  * Q is written in S balanced base-256 digits, Q = sum_s A_s 256^(S-1-s),
+//    A_s in [-128, 127] for s > 0: small integers that FP16 holds exactly;
+//  * the level sums L_l = sum_{s+t=l} A_s B_t are kept for l < V, the
+//    products of lower weight are dropped.  Every level sum over kOzPeriod
+//    consecutive K elements stays within 2^24, so the tensor cores' FP32
+//    accumulation adds integers exactly; the accumulators are drained every
+//    kOzPeriod K elements.
+//
+// Two instances (OzSplit<S>):
+//  * S = 6, F = 48, V = 6 (the mixed solve's defect and certification
+//    products): A_0 in [-256, 256]; the dropped products are each below
+//    2^-47 of the fixed-point scale; drains are combined in double-float
+//    arithmetic.
+//  * S = 7, F = 56, V = 8, rounded toward zero (the plain FP64 path): 56 bits
+//    hold every bit of a double within three binades of the row's largest
+//    entry; the errors are the truncation of the operands below 2^-56 of
+//    their row's (column's) scale and the dropped products, each below 2^-64
+//    of the product of the scales.  Levels 0 to 5 stay within 2^24 and add
+//    exactly; a level sum 6 or 7 beyond it may round by one unit, 2^-64 of
+//    the scale.  Drains are added in 64-bit integers, exactly.
 //
 // The rounding to Q and the digit extraction use integer operations only
 // (GB300 runs FP64 arithmetic at 1/64 of the FP32 rate).
@@ -33,9 +42,25 @@
 
 namespace iptgb {
 
-constexpr int kOzSlices = 6;      // digits per operand (48 bits)
+constexpr int kOzSlices = 6;      // digits per operand of the 48-bit split
 constexpr int kOzPeriod = 128;    // K elements between accumulator drains
-constexpr int kOzMaxCols = 64;    // columns per product launch
+
+// S slices: F fixed-point bits, V digit-product levels kept, the bias that
+// makes the low S - 1 digits unsigned bytes and puts the top digit, as the
+// FP16 bit pattern of 1536 + digit, into the 16 bits above them, and the
+// product's scale: Y = 2^(e_i + f_c + kOut) * (sum of the drains).
+template <int S>
+struct OzSplit;
+template <>
+struct OzSplit<6> {
+    static constexpr int kBits = 48, kLevels = 6, kOut = -16;
+    static constexpr uint64_t kBias = 0x0066008080808080ULL;
+};
+template <>
+struct OzSplit<7> {
+    static constexpr int kBits = 56, kLevels = 8, kOut = -72;
+    static constexpr uint64_t kBias = 0x6600808080808080ULL;
+};
 // Row / column exponent of a row that holds Inf or NaN: the product of that
 // row (column) is NaN.
 constexpr int kOzNonFinite = 0x7fffffff;
@@ -62,9 +87,10 @@ OZ_HD int oz_exponent(uint64_t absbits)
     return E - 1022;  // 1.f * 2^(E - 1023) < 2^(E - 1022)
 }
 
-// The 48-bit fixed-point value round(v 2^(48 - e)) (round half away from
+// The F-bit fixed-point value round(v 2^(F - e)) (round half away from
 // zero) of a finite v with |v| < 2^e; 0 for non-finite v.
-OZ_HD int64_t oz_fixed(double v, int e)
+template <int F>
+OZ_HD int64_t oz_fixed_bits(double v, int e)
 {
     uint64_t b;
 #if defined(__CUDA_ARCH__)
@@ -85,16 +111,21 @@ OZ_HD int64_t oz_fixed(double v, int e)
         M = (b & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL;
         x = E - 1075;
     }
-    const int sh = e - 48 - x;  // Q = M * 2^-sh
+    const int sh = e - F - x;  // Q = M * 2^-sh
     uint64_t q;
     if (sh >= 60) {
         q = 0;
     } else if (sh > 0) {
         q = (M >> sh) + ((M >> (sh - 1)) & 1ULL);
     } else {
-        q = M << (-sh);  // only for a row whose largest entry is subnormal
+        q = M << (-sh);  // exact: the row's largest entry is close to v
     }
     return neg ? -(int64_t)q : (int64_t)q;
+}
+
+OZ_HD int64_t oz_fixed(double v, int e)
+{
+    return oz_fixed_bits<OzSplit<6>::kBits>(v, e);
 }
 
 // Balanced base-256 digits of a fixed-point value: q = sum_s d[s] 256^(5-s).
@@ -109,11 +140,26 @@ OZ_HD void oz_digits_of(int64_t q, int (&d)[kOzSlices])
     d[0] = (int)q;
 }
 
-// The same digits as oz_digits_of(oz_fixed(v, e)) in 32-bit integer
-// arithmetic except one 64-bit shift: with q = H 2^24 + L (0 <= L < 2^24) the
-// three low digits depend only on L (carry c in {0, 1} out of them) and the
-// three high ones on H + c.
-OZ_HD void oz_digits_fast(double v, int e, int (&d)[kOzSlices])
+// Rows (columns) whose scale is below 2^kOzFastExp take the general form of
+// the split; subnormal entries of all others round to zero.
+constexpr int kOzFastExp = -900;
+
+// The offset nb that oz_biased subtracts an entry's exponent field from, for
+// a row of exponent e >= kOzFastExp (a non-finite row gets zero digits).
+template <int S>
+OZ_HD int oz_shift_base(int e)
+{
+    return e == kOzNonFinite ? 4096 : e + (S == 6 ? 1029 : 1022);
+}
+
+// Q + bias for an entry v of a row with shift base nb.  Adding 128 to every
+// digit below the top one turns the balanced digits into the bytes of the
+// sum (no carries to propagate): byte j holds digit S-1-j plus 128, the 16
+// bits above the S - 1 bytes hold 0x6600 + A_0.  With M the 53-bit
+// significand, one 64-bit shift of 8 M gives floor(|Q|) (S = 7), or
+// t = floor(2 |Q|) and the rounded |Q| = (t + 1) >> 1 (S = 6).
+template <int S>
+OZ_HD uint64_t oz_biased(double v, int nb)
 {
     uint64_t b;
 #if defined(__CUDA_ARCH__)
@@ -122,41 +168,42 @@ OZ_HD void oz_digits_fast(double v, int e, int (&d)[kOzSlices])
     __builtin_memcpy(&b, &v, sizeof(b));
 #endif
     const uint32_t hi = (uint32_t)(b >> 32);
-    const int E = (int)((hi >> 20) & 0x7FF);
-    const int sh = E == 0 ? e - 48 + 1074 : e - 48 - (E - 1075);
-    if (E == 2047 || e == kOzNonFinite || sh <= 0 || (b << 1) == 0) {
-        oz_digits_of(oz_fixed(v, e), d);  // zero, non-finite, or a subnormal-scale row
-        return;
+    const uint32_t sh = (uint32_t)(nb - (int)((hi >> 20) & 0x7FFu));
+    const uint32_t n8 = sh < 63u ? sh : 63u;
+    const uint64_t m8 = ((b << 3) & 0x007FFFFFFFFFFFFFULL) | 0x0080000000000000ULL;
+    uint64_t q = m8 >> n8;
+    if (S == 6) q = (q + 1) >> 1;
+    // two's complement by the sign, and the bias: its low word takes the
+    // + 1 without a carry
+    const uint32_t sg = (uint32_t)((int32_t)hi >> 31);
+    const uint64_t x = ((uint64_t)((uint32_t)(q >> 32) ^ sg) << 32) | ((uint32_t)q ^ sg);
+    const uint32_t low = (uint32_t)OzSplit<S>::kBias + (hi >> 31);
+    return x + ((OzSplit<S>::kBias & 0xFFFFFFFF00000000ULL) | low);
+}
+
+// The same for any row exponent.
+template <int S>
+OZ_HD uint64_t oz_biased_any(double v, int e)
+{
+    if (e != kOzNonFinite && e < kOzFastExp) {
+        return (uint64_t)oz_fixed_bits<OzSplit<S>::kBits>(v, e) + OzSplit<S>::kBias;
     }
-    uint32_t L;
-    int32_t H;
-    if (sh >= 60) {
-        L = 0;
-        H = 0;
-    } else {
-        const uint64_t M = E == 0 ? (b & 0x000FFFFFFFFFFFFFULL)
-                                  : ((b & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL);
-        const uint64_t q = (M + (1ULL << (sh - 1))) >> sh;  // < 2^48 + 1
-        const bool neg = (hi >> 31) != 0;
-        const uint64_t qs = neg ? (uint64_t)0 - q : q;
-        L = (uint32_t)qs & 0xFFFFFFu;
-        H = (int32_t)((int64_t)qs >> 24);
-    }
-    int32_t t = (int32_t)L;
+    return oz_biased<S>(v, oz_shift_base<S>(e));
+}
+
+// The S digits packed in a biased value.
+template <int S>
+OZ_HD void oz_unpack(uint64_t w, int (&d)[S])
+{
 #pragma unroll
-    for (int s = kOzSlices - 1; s >= 3; --s) {
-        const int32_t r = ((t + 128) & 255) - 128;
-        d[s] = r;
-        t = (t - r) >> 8;
-    }
-    int32_t u = H + t;
-#pragma unroll
-    for (int s = 2; s >= 1; --s) {
-        const int32_t r = ((u + 128) & 255) - 128;
-        d[s] = r;
-        u = (u - r) >> 8;
-    }
-    d[0] = u;
+    for (int s = 1; s < S; ++s) d[s] = (int)((w >> (8 * (S - 1 - s))) & 255u) - 128;
+    d[0] = (int)((w >> (8 * (S - 1))) & 0xFFFFu) - 0x6600;
+}
+
+// The digits of oz_digits_of(oz_fixed(v, e)) as the kernels form them.
+OZ_HD void oz_digits_fast(double v, int e, int (&d)[kOzSlices])
+{
+    oz_unpack<kOzSlices>(oz_biased_any<kOzSlices>(v, e), d);
 }
 
 }  // namespace iptgb
@@ -166,26 +213,55 @@ OZ_HD void oz_digits_fast(double v, int e, int (&d)[kOzSlices])
 
 namespace iptgb {
 
-// FP16 values of two digits (|d| <= 256): 1536 + d has FP16 bit pattern
-// 0x6600 + d (unit spacing in [1024, 2048)), and subtracting 1536 is exact.
-__device__ __forceinline__ __half2 oz_digit_pair(int d0, int d1)
+// The digits of two neighbouring entries, from their biased values, as four
+// words: x = digits S-1 and S-2 of both (bytes: entry 0, entry 1, entry 0,
+// entry 1), y = digits S-3 and S-4, z = the one or two digits left, w = the
+// top digits' FP16 patterns.
+template <int S>
+__device__ __forceinline__ uint4 oz_pack_pair(uint64_t w0, uint64_t w1)
 {
-    const uint32_t bits = (uint32_t)(0x6600 + d0) | ((uint32_t)(0x6600 + d1) << 16);
-    return __hsub2(*reinterpret_cast<const __half2 *>(&bits), __float2half2_rn(1536.0f));
+    const uint32_t l0 = (uint32_t)w0, l1 = (uint32_t)w1;
+    const uint32_t u0 = (uint32_t)(w0 >> 32), u1 = (uint32_t)(w1 >> 32);
+    return make_uint4(__byte_perm(l0, l1, 0x5140), __byte_perm(l0, l1, 0x7362),
+                      __byte_perm(u0, u1, 0x5140),
+                      __byte_perm(u0, u1, S == 7 ? 0x7632 : 0x6521));
 }
 
-// Write the kOzSlices digit slices of two neighbouring entries (v0, v1) of a
-// row with exponent e: slice s goes to dst[s * slice_stride] (a __half2).
-__device__ __forceinline__ void oz_store_pair(double v0, double v1, int e, __half2 *dst,
-                                              size_t slice_stride)
+// FP16 digit pairs (first entry in the low half) from two bytes of a packed
+// word (sel 0x4140: the low two, 0x4342: the high two): a byte u under 0x64 is
+// the FP16 value 1024 + u, and subtracting 1152 leaves the digit u - 128,
+// exactly; 1536 for the top digit's word.
+__device__ __forceinline__ uint32_t oz_half_pair(uint32_t word, uint32_t sel)
 {
-    int a[kOzSlices], b[kOzSlices];
-    oz_digits_fast(v0, e, a);
-    oz_digits_fast(v1, e, b);
-#pragma unroll
-    for (int s = 0; s < kOzSlices; ++s) {
-        dst[(size_t)s * slice_stride] = oz_digit_pair(a[s], b[s]);
-    }
+    const uint32_t b = __byte_perm(word, 0x64646464u, sel);
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&b), __float2half2_rn(1152.0f));
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+__device__ __forceinline__ uint32_t oz_top_pair(uint32_t word)
+{
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&word), __float2half2_rn(1536.0f));
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+
+// Digit pair of slice s from a packed pair.
+template <int S>
+__device__ __forceinline__ uint32_t oz_slice_pair(const uint4 &p, int s)
+{
+    if (s == 0) return oz_top_pair(p.w);
+    const int j = S - 1 - s;  // byte of the biased value
+    return oz_half_pair(j < 2 ? p.x : j < 4 ? p.y : p.z, (j & 1) != 0 ? 0x4342u : 0x4140u);
+}
+
+// Digit words of Delta: per 128-row tile and 32-element K stage one 32 KB
+// block [row][16 pairs], the 16-byte pair j of row r at position j ^ (r % 8)
+// (the product kernel's 16-byte shared-memory reads, lanes = rows, then meet
+// every bank).  Index of the pair that holds K entry l (and l ^ 1) of `row`,
+// with nst stages per row.
+__host__ __device__ __forceinline__ size_t oz_word_index(int row, int l, int nst)
+{
+    const int r = row & 127;
+    return (((size_t)(row >> 7) * nst + (l >> 5)) * 128 + r) * 16 + (((l & 31) >> 1) ^ (r & 7));
 }
 
 }  // namespace iptgb

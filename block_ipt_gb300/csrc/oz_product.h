@@ -7,45 +7,91 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "kernels.cuh"
 
 namespace iptgb {
 
-// The digit slices of Delta = H - diag(H): kOzSlices FP16 matrices
-// [slice][row][ldp] (ldp = n rounded up to 64, zero beyond n and on the
-// diagonal) and one exponent per row, with the TMA map the product streams.
-struct OzDelta {
+// The matrix of a product: an FP64 column-major n x n H in device memory
+// (which must outlive the object's uses) and one exponent per row of
+// Delta = H - diag(H).  With digit words the product streams those (8 bytes
+// per entry, as H itself, but without the ~25 integer instructions per entry
+// that the extraction of the digits takes in every product); without them it
+// reads H and extracts the digits on the way.
+struct OzMatrix {
+    const double *H = nullptr;
     int n = 0;
-    int ldp = 0;
-    DeviceBuffer<__half> A;
+    int nst = 0;           // 32-element K stages of a row
+    int words_slices = 0;  // digits per entry in `words` (0: none)
     DeviceBuffer<int> rowexp;
-    CUtensorMap mapA;
-    // storage and tensor map only (the fused setup pass writes the slices)
+    DeviceBuffer<uint4> words;  // oz_word_index
     int init_storage(int n, cudaStream_t s);
-    // slices of a column-major n x n H (any H; the diagonal is left out)
-    int split_from(const double *H, int n, cudaStream_t s);
+    // storage of the words only (the mixed solve's fused setup writes them)
+    int alloc_words(int slices, cudaStream_t s);
+    // row exponents of H from one pass over it; diag (optional, n) receives
+    // its diagonal
+    int scan_rows(const double *H, int n, double *diag, cudaStream_t s);
+    // digit words from a second pass (for matrices multiplied more than once
+    // or twice); without an error none where they exceed kMaxWordBytes or the
+    // device's memory
+    int build_words(int slices, cudaStream_t s);
 };
 
-// Y = (diag(d) + Delta) X for an n x C block X (column-major, ld ldx), in
-// groups of at most kOzMaxCols columns; d may be null (Y = Delta X).
+// n up to 46340; the words go back to the stream-ordered pool after a solve.
+constexpr size_t kMaxWordBytes = (size_t)16 << 30;
+
+// Launch shape of a product with C columns: `groups` column groups of cp
+// columns; the work items (group, 128-row tile, period of K elements) are
+// split evenly over `grid` persistent CTAs.
+struct OzShape {
+    int n = 0, C = 0, cp = 0, groups = 0, tiles = 0, periods = 0, ldp = 0, grid = 0;
+    int spp = 0;       // 32-element K stages per item
+    int maxslots = 0;  // partials a (group, tile) can have
+    long long items = 0;
+};
+
+// Y = (diag(d) + Delta) X for an n x C block X (column-major, ld ldx); d may
+// be null (Y = Delta X).  slices = 6: the 48-bit split; 7: the 56-bit split
+// of the plain FP64 path (oz.cuh).
+namespace oz {
+struct Partials;
+}
 struct OzProduct {
-    const OzDelta *dl = nullptr;
+    const OzMatrix *m = nullptr;
     const double *d = nullptr;
     cudaStream_t s = nullptr;
     int sms = 148;
-    int cp_cur = 0;
+    int slices = 6;
+    OzShape sh;
     DeviceBuffer<__half> B;
     DeviceBuffer<int> colexp;
-    DeviceBuffer<unsigned long long> colmax;
+    DeviceBuffer<unsigned long long> colmax;  // two sets of C column maxima
+    int cur = 0;                              // the set the next product reads
     DeviceBuffer<double> P;
     DeviceBuffer<int> err;
     CUtensorMap mapB;
-    int bind(const OzDelta *delta, const double *diag, cudaStream_t stream);
+    int bind(const OzMatrix *matrix, const double *diag, int digit_slices, cudaStream_t stream);
     int apply(const double *X, long long ldx, int C, double *Y, long long ldy);
+
+    // The plain IPT loop keeps the column maxima of its iterate up to date
+    // itself: begin() scans the first block, step() forms Delta X from the
+    // maxima of set `cur` and then Xn = F(X) (IPT map with g = 1 / (d_j - d_i),
+    // n x C), the maxima of Xn in the other set, and with ns (want_norms)
+    // ||Xn - X||_F and ||X||_F in ns->norms.
+    int begin(const double *X, int C);
+    int step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns);
+
     // the kernel's error flag (non-zero: a bounded wait gave up)
     int read_error(int *host_err);
 
   private:
-    int apply_group(const double *X, long long ldx, int C, double *Y, long long ldy);
+    int shape_for(int C);
+    int scan_columns(const double *X, long long ldx);
+    int slice_and_multiply(const double *X, long long ldx, int clear_other);
+    oz::Partials partials() const;
 };
+
+// g_ij = 1 / (d_j - d_i) for the n x k block (NaN for a zero or non-finite
+// gap, as the reference's build_g_kernel with min_gap_allowed = 0).
+int launch_gap_reciprocals(const double *d, int n, int k, double *g, cudaStream_t s);
 
 }  // namespace iptgb
