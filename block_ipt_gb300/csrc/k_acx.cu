@@ -10,13 +10,12 @@
 // with cublasDgemm and reads a flag, k residuals and two cuBLAS norms back
 // per map evaluation.
 //
-// Here HX is the plain path's FP64-accurate tensor-core product (k_oz.cu); F is
-// one CTA per column that reads (HX)_cc, evaluates the column's residual
-// norm and the map in one pass, in place; the two Frobenius norms are one
-// deterministic grid reduction; an extrapolation step is one CTA per column
-// (the two inner products, then the update).  The host reads k + 3 values
-// per step.  The map's denominator test only depends on the diagonal, so the
-// first evaluation decides it for the whole run.
+// Here F is the plain path's step (k_oz.cu: the FP64-accurate product on the
+// tensor cores, whose consumer applies the map and forms the column residuals
+// and the two Frobenius norms in the same pass); an extrapolation step is two
+// launches over (row blocks, columns), the inner products and the update.  The
+// host reads k + 3 values per step.  The map's denominator test only depends
+// on the diagonal: it is made once, with the gap reciprocals.
 #include <cublas_v2.h>
 #include <float.h>
 #include <math.h>
@@ -38,48 +37,116 @@ namespace iptgb {
 constexpr int kAcxThreads = 256;
 constexpr int kAcxNormBlocks = 256;
 
-// Y = F(X) in place on Y = H X, one CTA per column c:
-//   m = Y[c,c], u = m - d[c] X[c,c], r_c = ||Y[:,c] - X[:,c] m||,
-//   Y[c,c] = 1, Y[i,c] = (Y[i,c] - d[i] X[i,c] - X[i,c] u) / (d[c] - d[i])
-// and a flag where |d[c] - d[i]| <= DBL_EPSILON (acx_cuda.cu:109-172).
-__global__ void __launch_bounds__(kAcxThreads)
-acx_map_kernel(double *__restrict__ Y, const double *__restrict__ X, const double *__restrict__ d,
-               int n, double *__restrict__ resid, int *__restrict__ flag)
+// g_ic = 1 / (d_c - d_i) of the ACX map, 0 and the flag where |d_c - d_i| <=
+// DBL_EPSILON (acx_cuda.cu:109-172).
+__global__ void acx_gaps_kernel(const double *__restrict__ d, int n, double *__restrict__ g,
+                                int *__restrict__ flag)
+{
+    const int c = blockIdx.y;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double den = d[c] - d[i];
+    const bool zero = fabs(den) <= DBL_EPSILON;
+    g[(size_t)i + (size_t)c * n] = zero ? 0.0 : 1.0 / den;
+    if (zero && i != c) atomicOr(flag, 1);
+}
+
+// resid[c] = ||(H X)_c - X_c (H X)_cc|| from the update's parts, in order.
+__global__ void acx_resid_kernel(const double *__restrict__ part, int row_blocks, int k,
+                                 double *__restrict__ resid)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
-    const int c = blockIdx.x;
-    double *y = Y + (size_t)c * n;
-    const double *x = X + (size_t)c * n;
-    __shared__ double mu[2];
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= k) return;
+    double s = 0.0;
+    for (int b = 0; b < row_blocks; ++b) s += part[(size_t)c * row_blocks + b];
+    resid[c] = sqrt(s);
+}
+
+// One FP64 extrapolation step (acx_cuda.cu:190-296) over (1024-row blocks,
+// columns): the inner products of each block, then - the blocks of a column
+// added in order - the update and the column maxima of the new X for the next
+// product.  F3 is null for an order-2 step.  (One CTA per column for both
+// took 36 us at n = 4096, k = 16: 16 SMs busy.)
+constexpr int kAcxRows = 4 * kAcxThreads;
+
+__global__ void __launch_bounds__(kAcxThreads)
+acx_products_kernel(const double *__restrict__ X, const double *__restrict__ F1,
+                    const double *__restrict__ F2, const double *__restrict__ F3, int n,
+                    double2 *__restrict__ part, unsigned long long *__restrict__ colmax)
+{
+    pdl_wait();  // programmatic dependent launch: predecessor done
+    pdl_trigger();
+    const size_t base = (size_t)blockIdx.y * n;
+    double num = 0.0, den = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = blockIdx.x * kAcxRows + q * kAcxThreads + threadIdx.x;
+        if (i >= n) break;
+        const double x = X[base + i], f1 = F1[base + i], f2 = F2[base + i];
+        const double d2 = fma(-2.0, f1, f2) + x;
+        if (F3 == nullptr) {
+            num = fma(d2, f1 - x, num);
+            den = fma(d2, d2, den);
+        } else {
+            const double d3 = fma(3.0, f1, fma(-3.0, f2, F3[base + i])) - x;
+            num = fma(d3, d2, num);
+            den = fma(d3, d3, den);
+        }
+    }
+    const double2 s = block_sum2(num, den);
     if (threadIdx.x == 0) {
-        const double m = y[c];
-        mu[0] = m;
-        mu[1] = fma(-d[c], x[c], m);
+        part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
+        if (blockIdx.x == 0) colmax[blockIdx.y] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(kAcxThreads)
+acx_update_kernel(double *__restrict__ X, const double *__restrict__ F1,
+                  const double *__restrict__ F2, const double *__restrict__ F3, int n,
+                  const double2 *__restrict__ part, unsigned long long *__restrict__ colmax)
+{
+    pdl_wait();  // programmatic dependent launch: predecessor done
+    pdl_trigger();
+    __shared__ double sig;
+    if (threadIdx.x == 0) {
+        double num = 0.0, den = 0.0;
+        for (int b = 0; b < (int)gridDim.x; ++b) {
+            const double2 p = part[(size_t)blockIdx.y * gridDim.x + b];
+            num += p.x;
+            den += p.y;
+        }
+        sig = den > 0.0 ? fabs(num / den) : 0.0;
     }
     __syncthreads();
-    const double m = mu[0], u = mu[1], dc = d[c];
-    double rr = 0.0;
-    bool bad = false;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double yi = y[i], xi = x[i];
-        const double r = fma(-xi, m, yi);
-        rr = fma(r, r, rr);
-        double v = 1.0;
-        if (i != c) {
-            const double den = dc - d[i];
-            if (fabs(den) <= DBL_EPSILON) {
-                bad = true;
-                v = 0.0;
-            } else {
-                v = fma(-xi, u, fma(-d[i], xi, yi)) / den;
-            }
+    const double g = sig, g2 = g * g, g3 = g2 * g;
+    const size_t base = (size_t)blockIdx.y * n;
+    unsigned long long m = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = blockIdx.x * kAcxRows + q * kAcxThreads + threadIdx.x;
+        if (i >= n) break;
+        const double x = X[base + i], f1 = F1[base + i], f2 = F2[base + i];
+        const double d1 = f1 - x;
+        const double d2 = fma(-2.0, f1, f2) + x;
+        double v;
+        if (F3 == nullptr) {
+            v = x + fma(2.0 * g, d1, g2 * d2);
+        } else {
+            const double d3 = fma(3.0, f1, fma(-3.0, f2, F3[base + i])) - x;
+            v = x + fma(3.0 * g, d1, fma(3.0 * g2, d2, g3 * d3));
         }
-        y[i] = v;
+        X[base + i] = v;
+        const unsigned long long a =
+            (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
+        m = a > m ? a : m;
     }
-    const double2 s = block_sum2(rr, 0.0);
-    if (threadIdx.x == 0) resid[c] = sqrt(s.x);
-    if (bad) atomicOr(flag, 1);
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
+        m = o > m ? o : m;
+    }
+    if ((threadIdx.x & 31) == 0 && m != 0) atomicMax(colmax + blockIdx.y, m);
 }
 
 // out = (||A - B||_F, ||B||_F), deterministic (sums in FP64 for either type).
@@ -102,9 +169,8 @@ acx_norms_kernel(const T *__restrict__ A, const T *__restrict__ B, size_t count,
     grid_finish_norms2(block_sum2(dd, bb), partials, counter, out);
 }
 
-// One extrapolation step, one CTA per column (acx_cuda.cu:190-296, and the
-// FP32 pair of acx_mixed_precision_cuda.cu:198-319); F3 is null for an
-// order-2 step.  The inner products accumulate in T, the step length is
+// One extrapolation step of the FP32 stage, one CTA per column
+// (acx_mixed_precision_cuda.cu:198-319); F3 is null for an order-2 step.  The inner products accumulate in T, the step length is
 // formed in FP64 from their block sums.
 template <typename T>
 __global__ void __launch_bounds__(kAcxThreads)
@@ -237,17 +303,20 @@ namespace {
 struct AcxDense {
     OzMatrix matrix;
     OzProduct product;
-    int n = 0, k = 0;
+    DeviceBuffer<double> g;      // gap reciprocals, n x k
+    DeviceBuffer<double> rpart;  // residual parts of the last norms step
+    NormScratch ns;
+    int n = 0, k = 0, row_blocks = 0;
     cudaStream_t s = nullptr;
-    const double *d = nullptr;
     double *resid = nullptr;
-    int *flag = nullptr;
-    // Y = F(X)
-    int apply(const double *X, double *Y)
+    // Y = F(X); with norms also ||Y - X||_F, ||X||_F and the column residuals
+    // of X.  The column maxima of X are those of the last Y (or begin()).
+    int apply(const double *X, double *Y, bool norms)
     {
-        IPTGB_CHECK(product.apply(X, n, k, Y, n));
-        return launch_pdl(acx_map_kernel, dim3(k), dim3(kAcxThreads), 0, s, Y, X, d, n, resid,
-                          flag);
+        IPTGB_CHECK(product.step(X, g.ptr, Y, norms, &ns, norms ? rpart.ptr : nullptr));
+        if (!norms) return IPT_CUDA_SUCCESS;
+        return launch_pdl(acx_resid_kernel, dim3(blocks_for((size_t)k)), dim3(kThreads), 0, s,
+                          (const double *)rpart.ptr, row_blocks, k, resid);
     }
 };
 
@@ -309,21 +378,28 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         F.k = k;
         F.s = s;
         DeviceBuffer<double> X, F2, F3, small;
-        DeviceBuffer<double2> part;
+        bool wide = false;
+        F.row_blocks = OzProduct::update_row_blocks(n, k, device_sm_count(), &wide);
+        const int ext_blocks = (n + kAcxRows - 1) / kAcxRows;
+        DeviceBuffer<double2> part, ext;
         DeviceBuffer<int> flags;
         // small: d (n) | resid (k) | norms (2)
         bool ok = X.alloc(elems, s) == IPT_CUDA_SUCCESS && F2.alloc(elems, s) == IPT_CUDA_SUCCESS &&
                   F3.alloc(elems, s) == IPT_CUDA_SUCCESS &&
                   small.alloc((size_t)n + (size_t)k + 2, s) == IPT_CUDA_SUCCESS &&
-                  part.alloc(kAcxNormBlocks, s) == IPT_CUDA_SUCCESS &&
+                  part.alloc((size_t)F.row_blocks * k, s) == IPT_CUDA_SUCCESS &&
+                  ext.alloc((size_t)ext_blocks * k, s) == IPT_CUDA_SUCCESS &&
+                  F.rpart.alloc((size_t)F.row_blocks * k, s) == IPT_CUDA_SUCCESS &&
+                  F.g.alloc(elems, s) == IPT_CUDA_SUCCESS &&
                   flags.alloc(2, s) == IPT_CUDA_SUCCESS;
         if (!ok) status = ACX_CUDA_ALLOCATION_FAILED;
         double *d = small.ptr, *resid = small.ptr + n, *norms = small.ptr + n + k;
         int *flag = flags.ptr;
-        unsigned int *counter = reinterpret_cast<unsigned int *>(flags.ptr + 1);
-        F.d = d;
         F.resid = resid;
-        F.flag = flag;
+        F.ns.partials = part.ptr;
+        F.ns.capacity = F.row_blocks * k;
+        F.ns.counter = reinterpret_cast<unsigned int *>(flags.ptr + 1);
+        F.ns.norms = norms;
         auto cuda_ok = [&](cudaError_t e) {
             if (e != cudaSuccess && status == ACX_CUDA_SUCCESS) status = ACX_CUDA_CUDA_ERROR;
             return status == ACX_CUDA_SUCCESS;
@@ -334,14 +410,21 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         };
         if (status == ACX_CUDA_SUCCESS) {
             cuda_ok(cudaMemsetAsync(flags.ptr, 0, 2 * sizeof(int), s));
-            lib_ok(F.matrix.scan_rows(H, n, d, s));
-            lib_ok(F.matrix.build_words(7, s));
-            lib_ok(F.product.bind(&F.matrix, d, 7, s));
+            if (lib_ok(F.matrix.scan_rows(H, n, d, s)) && lib_ok(F.matrix.build_words(7, s))) {
+                lib_ok(F.product.bind(&F.matrix, d, 7, s));
+            }
             if (initial == nullptr) {
                 lib_ok(launch_set_identity(X.ptr, n, k, s));
             } else {
                 cuda_ok(cudaMemcpyAsync(X.ptr, initial, elems * sizeof(double),
                                         cudaMemcpyDeviceToDevice, s));
+            }
+            if (status == ACX_CUDA_SUCCESS) {
+                acx_gaps_kernel<<<dim3(blocks_for((size_t)n), k), kThreads, 0, s>>>(d, n, F.g.ptr,
+                                                                                    flag);
+                cuda_ok(cudaGetLastError());
+                count_launch();
+                lib_ok(F.product.begin(X.ptr, k));
             }
         }
         std::vector<double> host((size_t)k + 2);
@@ -351,13 +434,8 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         for (int iter = 1; iter <= maxiter && status == ACX_CUDA_SUCCESS; ++iter) {
             const int order = (iter % 2 == 1) ? 2 : 3;
             result->iterations = iter;
-            if (!lib_ok(F.apply(X.ptr, f1))) break;
+            if (!lib_ok(F.apply(X.ptr, f1, true))) break;
             result->f_calls += 1;
-            if (!lib_ok(launch_pdl(acx_norms_kernel<double>, dim3(kAcxNormBlocks),
-                                   dim3(kAcxThreads), 0, s, (const double *)f1,
-                                   (const double *)X.ptr, elems, part.ptr, counter, norms))) {
-                break;
-            }
             if (!cuda_ok(cudaMemcpyAsync(host.data(), resid, ((size_t)k + 2) * sizeof(double),
                                          cudaMemcpyDeviceToHost, s)) ||
                 !cuda_ok(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, s)) ||
@@ -382,15 +460,20 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                 final_is_x = false;
                 break;
             }
-            if (!lib_ok(F.apply(f1, F2.ptr))) break;
+            if (!lib_ok(F.apply(f1, F2.ptr, false))) break;
             result->f_calls += 1;
             if (order == 3) {
-                if (!lib_ok(F.apply(F2.ptr, F3.ptr))) break;
+                if (!lib_ok(F.apply(F2.ptr, F3.ptr, false))) break;
                 result->f_calls += 1;
             }
-            lib_ok(launch_pdl(acx_extrapolate_kernel<double>, dim3(k), dim3(kAcxThreads), 0, s,
-                              X.ptr, (const double *)f1, (const double *)F2.ptr,
-                              order == 3 ? (const double *)F3.ptr : (const double *)nullptr, n));
+            const double *f3 = order == 3 ? F3.ptr : nullptr;
+            unsigned long long *maxima = F.product.column_maxima();
+            lib_ok(launch_pdl(acx_products_kernel, dim3(ext_blocks, k), dim3(kAcxThreads), 0, s,
+                              (const double *)X.ptr, (const double *)f1, (const double *)F2.ptr,
+                              f3, n, ext.ptr, maxima));
+            lib_ok(launch_pdl(acx_update_kernel, dim3(ext_blocks, k), dim3(kAcxThreads), 0, s,
+                              X.ptr, (const double *)f1, (const double *)F2.ptr, f3, n,
+                              (const double2 *)ext.ptr, maxima));
         }
         result->iteration_time_sec = seconds_since(t_iter);
         const auto t_fin = std::chrono::steady_clock::now();

@@ -225,6 +225,18 @@ __device__ __forceinline__ void tmem_ld_4cols(uint32_t taddr, uint32_t (&r)[4])
                  : "r"(taddr));
 }
 
+// Waits for the TMEM loads issued so far; naming the registers they fill keeps
+// every use of them behind the wait.
+template <int V>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[V][4])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int l = 0; l < V; ++l) {
+        asm volatile("" : "+r"(r[l][0]), "+r"(r[l][1]), "+r"(r[l][2]), "+r"(r[l][3])::"memory");
+    }
+}
+
 // Running sums of a thread's columns over the periods of a tile.
 template <int S, int NC>
 struct Sums;
@@ -685,7 +697,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
                 uint32_t v[V][4];
 #pragma unroll
                 for (int l = 0; l < V; ++l) tmem_ld_4cols(addr + (uint32_t)(l * CP + j0), v[l]);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                tmem_ld_wait<V>(v);
                 if (j0 + 4 >= NC) {
                     // the last columns are in registers: the MMAs of a later
                     // item may overwrite the set
@@ -894,8 +906,9 @@ oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
 // The IPT map from the partials of Delta X:
 //   c_j = (Delta X)_jj,  X'_ij = ((Delta X)_ij - X_ij c_j) g_ij,  X'_jj = 1
 // (IPT_C_GPU/src/ipt_cuda.cu:1369-1443), the column maxima of X' and with
-// want_norms ||X' - X||_F, ||X||_F (ipt_cuda.cu:1457-1467,1663-1688).  A row
-// of H or column of X that is not finite takes the FP64 sums the map is
+// want_norms ||X' - X||_F, ||X||_F (ipt_cuda.cu:1457-1467,1663-1688); with
+// resid_part also the block's part of ||(H X)_c - X_c (H X)_cc||^2 (ACX).  A
+// row of H or column of X that is not finite takes the FP64 sums the map is
 // defined by, so Inf and NaN travel as there.
 //
 // A block of 8 warps takes 256 R rows of one column, R per thread; a ninth
@@ -912,7 +925,8 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
                  const double *__restrict__ d, const double *__restrict__ g,
                  const double *__restrict__ X, double *__restrict__ Xn,
                  unsigned long long *__restrict__ colmax_next, int row_blocks, int want_norms,
-                 double2 *partials, unsigned int *counter, double *norms)
+                 double2 *partials, unsigned int *counter, double *norms,
+                 double *__restrict__ resid_part)
 {
     constexpr int kRows = kUpdateThreads * R;
     constexpr int kTiles = kRows / kBM;
@@ -956,13 +970,18 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     __syncthreads();
     const double cj = cj_sh;
     const bool failed = *p.err != 0;
-    double dsq = 0.0, xsq = 0.0;
+    double dsq = 0.0, xsq = 0.0, rsq = 0.0;
     unsigned long long m = 0;
+    const double hcc = resid_part != nullptr ? fma(d[c], xc[c], cj) : 0.0;  // (H X)_cc
     if (t < kUpdateThreads) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int i = row0 + q * kUpdateThreads + t;
             if (i < n) {
+                if (resid_part != nullptr) {
+                    const double r = fma(x[q], d[i] - hcc, y[q]);
+                    rsq = fma(r, r, rsq);
+                }
                 double out = i == c ? 1.0 : fma(-x[q], cj, y[q]) * gi[q];
                 if (failed) out = NAN;
                 Xn[(size_t)i + (size_t)c * n] = out;
@@ -978,6 +997,10 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     }
     m = warp_max(m);
     if ((t & 31) == 0 && m != 0) atomicMax(colmax_next + c, m);
+    if (resid_part != nullptr) {
+        const double2 r = block_sum2(rsq, 0.0);
+        if (t == 0) resid_part[blockIdx.x] = r.x;
+    }
     if (want_norms) grid_finish_norms2(block_sum2(dsq, xsq), partials, counter, norms);
 }
 
@@ -1345,11 +1368,18 @@ int OzProduct::begin(const double *X, int C)
     return scan_columns(X, sh.n);
 }
 
-int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns)
+int OzProduct::update_row_blocks(int n, int C, int sms, bool *wide)
 {
-    const int r1 = (sh.n + oz::kUpdateThreads - 1) / oz::kUpdateThreads;
-    const bool wide = (long long)((r1 + 3) / 4) * sh.C >= sms;
-    const int row_blocks = wide ? (r1 + 3) / 4 : r1;
+    const int r1 = (n + oz::kUpdateThreads - 1) / oz::kUpdateThreads;
+    *wide = (long long)((r1 + 3) / 4) * C >= sms;
+    return *wide ? (r1 + 3) / 4 : r1;
+}
+
+int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns,
+                    double *resid_part)
+{
+    bool wide = false;
+    const int row_blocks = update_row_blocks(sh.n, sh.C, sms, &wide);
     const long long grid = (long long)row_blocks * sh.C;
     if (want_norms && grid > ns->capacity) return IPT_CUDA_INVALID_ARGUMENT;
     const size_t set = (size_t)sh.groups * sh.cp;
@@ -1360,7 +1390,7 @@ int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms
     KernelTimerScope timer(kProfFp64Update, s);
     IPTGB_CHECK(launch_pdl(wide ? oz::oz_update_kernel<4> : oz::oz_update_kernel<1>,
                            dim3((unsigned)grid), dim3(oz::kUpdateThreads + 32), 0, s, partials(), m->H, d, g, X, Xn, colmax.ptr + (1 - cur) * set, row_blocks,
-                           want_norms, ns->partials, ns->counter, ns->norms));
+                           want_norms, ns->partials, ns->counter, ns->norms, resid_part));
     cur = 1 - cur;
     return IPT_CUDA_SUCCESS;
 }

@@ -78,7 +78,13 @@ struct OzProduct {
     // n x C), the maxima of Xn in the other set, and with ns (want_norms)
     // ||Xn - X||_F and ||X||_F in ns->norms.
     int begin(const double *X, int C);
-    int step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns);
+    // resid_part (optional): update_row_blocks parts per column of
+    // ||(H X)_c - X_c (H X)_cc||^2.
+    int step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns,
+             double *resid_part = nullptr);
+    static int update_row_blocks(int n, int C, int sms, bool *wide);
+    // the column maxima (bit patterns) the next step reads
+    unsigned long long *column_maxima() { return colmax.ptr + (size_t)cur * sh.groups * sh.cp; }
 
     // the kernel's error flag (non-zero: a bounded wait gave up)
     int read_error(int *host_err);
