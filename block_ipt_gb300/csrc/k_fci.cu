@@ -121,10 +121,19 @@ __host__ __device__ __forceinline__ float u53_to_float(uint64_t v)
 }
 
 // second stage of the pair hash: h1 = splitmix(key ^ lo), hm = hi * M;
-// u = float((h >> 11) | 1) 2^-53
+// u = float((h >> 11) | 1) 2^-53.  The | 1 lies below every rounding position,
+// so 32 leading bits with that one or-ed into the last of them round alike as
+// long as at least 26 of them are significant: one 32-bit conversion (h >>
+// 32, or h >> 25 below 2^57) unless the 14 top bits of h are zero.
 __host__ __device__ __forceinline__ float pair_uniform(uint64_t h1, uint64_t hm)
 {
     const uint64_t h = splitmix(h1 ^ hm);
+    const uint32_t hi = (uint32_t)(h >> 32);
+    if (hi >= (1u << 18)) {
+        const bool low = hi < (1u << 25);
+        const uint32_t q = (low ? (uint32_t)(h >> 25) : hi) | 1u;
+        return (float)q * (low ? 0x1p-39f : 0x1p-32f);
+    }
     return u53_to_float((h >> 11) | 1ULL) * 0x1p-53f;
 }
 
@@ -351,6 +360,7 @@ struct DevTables {
     int nsb, sA, sB, dA, dB;
     uint64_t k33a, k33b;
     float sigma;
+    uint32_t inv_sB;  // ceil(2^32 / sB), sB > 1
     const double *diag;
 };
 
@@ -401,13 +411,66 @@ struct SigmaAcc<XDF> {
     __device__ __forceinline__ double value() const { return (double)sh + (double)sl; }
 };
 
-// Y[:, c0:c0+KC] (column-major, ld n) = H X for the KC-column block of the
-// row-major Xr (row J holds X[J, c0:c0+KC]); one warp per row.  The lane
-// partials are summed in FP64.
+// Coupling q of row (ia, ib): the coupled strings (ja, jb).
+struct RowLinks {
+    const int *sa, *sb, *da, *db;
+    int ia, ib, b1, b2, b3, b4, total;
+    __device__ __forceinline__ RowLinks(const DevTables &t, int ia_, int ib_)
+        : sa(t.singA + (size_t)ia_ * t.sA),
+          sb(t.singB + (size_t)ib_ * t.sB),
+          da(t.doubA + (size_t)ia_ * t.dA),
+          db(t.doubB + (size_t)ib_ * t.dB),
+          ia(ia_),
+          ib(ib_),
+          b1(t.sA),
+          b2(b1 + t.sB),
+          b3(b2 + t.dA),
+          b4(b3 + t.dB),
+          total(b4 + t.sA * t.sB)
+    {
+    }
+    __device__ __forceinline__ void target(const DevTables &t, int q, int &ja, int &jb) const
+    {
+        if (q >= b4) {
+            // r / sB by a multiplication: exact for r sB < 2^32
+            const uint32_t r = (uint32_t)(q - b4);
+            const uint32_t a = t.sB > 1 ? __umulhi(r, t.inv_sB) : r;
+            ja = sa[a];
+            jb = sb[r - a * (uint32_t)t.sB];
+        } else if (q < b1) {
+            ja = sa[q];
+            jb = ib;
+        } else if (q < b2) {
+            ja = ia;
+            jb = sb[q - b1];
+        } else if (q < b3) {
+            ja = da[q - b2];
+            jb = ib;
+        } else {
+            ja = ia;
+            jb = db[q - b3];
+        }
+    }
+};
+
+// Y[:, c0:c0+8] (column-major, ld n) = H X for the 8-column block of the
+// row-major Xr (row J holds X[J, c0:c0+8]); one warp per row, 32 couplings at
+// a time.  Lane l generates the element of coupling q0 + l; then the warp
+// gathers four rows of X at a time, eight lanes (the columns) per row: lane
+// (g, c) takes couplings 4 u + g, u = 0..7, of column c, with one partial sum
+// per u, which is the sum a lane that handled its coupling's whole row of X
+// would form.  (That form read 64 bytes per lane from 32 unrelated rows: 128
+// L1 tag lookups per 32 couplings against 32 here.)  The partials are summed in
+// FP64, in a fixed order.
+//
+// Bound by the instructions that regenerate an element (hashes, Box-Muller,
+// exp); FP64-accurate, 12 orbitals (n = 853,776, 1.55 G couplings), 8 columns:
+// 56 ms before, 22.8 ms now (427 lane instructions per coupling, 77 % of the issue slots).
 template <typename XT, int KC>
 __global__ void __launch_bounds__(256)
 fci_sigma_kernel(DevTables t, const XT *__restrict__ Xr, int c0, int k, double *__restrict__ Y)
 {
+    static_assert(KC == 8, "eight lanes per row of X");
     const long long I = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (I >= t.n) return;
@@ -417,48 +480,50 @@ fci_sigma_kernel(DevTables t, const XT *__restrict__ Xr, int c0, int k, double *
     const uint64_t hI1 = splitmix(t.k33a ^ (uint64_t)I);
     const uint64_t hI2 = splitmix(t.k33b ^ (uint64_t)I);
     const uint64_t hIm = pair_mult((uint64_t)I);
-    SigmaAcc<XT> acc[KC];
-    const int *sa = t.singA + (size_t)ia * t.sA;
-    const int *sb = t.singB + (size_t)ib * t.sB;
-    const int *da = t.doubA + (size_t)ia * t.dA;
-    const int *db = t.doubB + (size_t)ib * t.dB;
-    const int b1 = t.sA, b2 = b1 + t.sB, b3 = b2 + t.dA, b4 = b3 + t.dB;
-    const int total = b4 + t.sA * t.sB;
-    for (int q = lane; q < total; q += 32) {
-        int ja, jb;
-        if (q < b1) {
-            ja = sa[q];
-            jb = ib;
-        } else if (q < b2) {
-            ja = ia;
-            jb = sb[q - b1];
-        } else if (q < b3) {
-            ja = da[q - b2];
-            jb = ib;
-        } else if (q < b4) {
-            ja = ia;
-            jb = db[q - b3];
-        } else {
-            const int r = q - b4;
-            const int a = r / t.sB;
-            ja = sa[a];
-            jb = sb[r - a * t.sB];
+    const RowLinks links(t, ia, ib);
+    const int c = lane & 7, g = lane >> 3;
+    SigmaAcc<XT> acc[8];
+    for (int q0 = 0; q0 < links.total; q0 += 32) {
+        const int q = q0 + lane;
+        float v = 0.f;
+        uint32_t J = (uint32_t)I;
+        if (q < links.total) {
+            int ja, jb;
+            links.target(t, q, ja, jb);
+            J = (uint32_t)ja * (uint32_t)t.nsb + (uint32_t)jb;
+            const float gap = F_ADD(F_SUB(t.occAf[ja], eIa), F_SUB(t.occBf[jb], eIb));
+            v = offdiag(t.k33a, t.k33b, (uint64_t)I, (uint64_t)J, hI1, hI2, hIm, gap, t.sigma);
         }
-        const long long J = (long long)ja * t.nsb + jb;
-        const float gap = F_ADD(F_SUB(t.occAf[ja], eIa), F_SUB(t.occBf[jb], eIb));
-        const float v = offdiag(t.k33a, t.k33b, (uint64_t)I, (uint64_t)J, hI1, hI2, hIm, gap,
-                                t.sigma);
-        const XT *x = Xr + (size_t)J * KC;
+        XT x[8];
+        float w[8];
 #pragma unroll
-        for (int j = 0; j < KC; ++j) acc[j].add(v, x[j]);
-    }
-    double out = 0.0;
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t Ju = __shfl_sync(0xffffffffu, J, 4 * u + g);
+            x[u] = Xr[(size_t)Ju * KC + c];
+            w[u] = __shfl_sync(0xffffffffu, v, 4 * u + g);
+        }
+        if (q0 + 32 <= links.total) {
 #pragma unroll
-    for (int j = 0; j < KC; ++j) {
-        double s = acc[j].value();
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        out = lane == j ? s : out;
+            for (int u = 0; u < 8; ++u) acc[u].add(w[u], x[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (q0 + 4 * u + g < links.total) acc[u].add(w[u], x[u]);
+            }
+        }
     }
+    // the couplings' lanes 4 u + g pairwise: bits 4, 3, 2 (u), then 1, 0 (g)
+    double s[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s[u] = acc[u].value();
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+#pragma unroll
+        for (int u = 0; u < off; ++u) s[u] += s[u + off];
+    }
+    double out = s[0];
+    out += __shfl_xor_sync(0xffffffffu, out, 16);
+    out += __shfl_xor_sync(0xffffffffu, out, 8);
     if (lane < KC && c0 + lane < k) {
         // the diagonal term in FP64
         const size_t e = (size_t)I * KC + lane;
@@ -488,33 +553,11 @@ fci_rowstats_kernel(DevTables t, double *__restrict__ rowabs, double *__restrict
     const uint64_t hI1 = splitmix(t.k33a ^ (uint64_t)I);
     const uint64_t hI2 = splitmix(t.k33b ^ (uint64_t)I);
     const uint64_t hIm = pair_mult((uint64_t)I);
-    const int *sa = t.singA + (size_t)ia * t.sA;
-    const int *sb = t.singB + (size_t)ib * t.sB;
-    const int *da = t.doubA + (size_t)ia * t.dA;
-    const int *db = t.doubB + (size_t)ib * t.dB;
-    const int b1 = t.sA, b2 = b1 + t.sB, b3 = b2 + t.dA, b4 = b3 + t.dB;
-    const int total = b4 + t.sA * t.sB;
+    const RowLinks links(t, ia, ib);
     double sabs = 0.0, s2 = 0.0;
-    for (int q = lane; q < total; q += 32) {
+    for (int q = lane; q < links.total; q += 32) {
         int ja, jb;
-        if (q < b1) {
-            ja = sa[q];
-            jb = ib;
-        } else if (q < b2) {
-            ja = ia;
-            jb = sb[q - b1];
-        } else if (q < b3) {
-            ja = da[q - b2];
-            jb = ib;
-        } else if (q < b4) {
-            ja = ia;
-            jb = db[q - b3];
-        } else {
-            const int r = q - b4;
-            const int a = r / t.sB;
-            ja = sa[a];
-            jb = sb[r - a * t.sB];
-        }
+        links.target(t, q, ja, jb);
         const long long J = (long long)ja * t.nsb + jb;
         const float gap = F_ADD(F_SUB(t.occAf[ja], eIa), F_SUB(t.occBf[jb], eIb));
         const double v = (double)offdiag(t.k33a, t.k33b, (uint64_t)I, (uint64_t)J, hI1, hI2, hIm,
@@ -619,6 +662,7 @@ struct FciOperator final : Fp64Apply {
         dev.k33a = fci::stream_key(seed, 33);
         dev.k33b = fci::stream_key(seed, 33 + 7919);
         dev.sigma = host.sigma;
+        dev.inv_sB = host.sB > 1 ? (uint32_t)(((1ULL << 32) + host.sB - 1) / host.sB) : 0;
         dev.diag = diag.ptr;
         fci::fci_diag_kernel<<<(unsigned)((host.n + 255) / 256), 256, 0, s>>>(
             dev, fci::stream_key(seed, 32), fci::stream_key(seed, 32 + 7919), diag.ptr);
