@@ -14,8 +14,9 @@
 //        a. conversion + shift + symmetrisation, many CTAs;
 //        b. Householder tridiagonalisation, one CTA (four barriers per
 //           column);
-//        c. bisection (Sturm counts) for every eigenvalue, one thread each,
-//           then inverse iteration with a partially pivoted tridiagonal LU,
+//        c. bisection (Sturm counts) for every eigenvalue, one warp each on
+//           many SMs, then inverse iteration with a partially pivoted
+//           tridiagonal LU,
 //           with modified Gram-Schmidt inside clusters of eigenvalues closer
 //           than 1e-3 ||T|| between iterations (block inverse iteration),
 //           so that clustered vectors span the cluster's invariant subspace;
@@ -214,8 +215,8 @@ eig_tridiag_kernel(const float *__restrict__ Af, int m, float *__restrict__ vh,
 }
 
 // ---------------------------------------------------------------------------
-// 1c. Eigenvalues of the tridiagonal (d, e) by bisection and eigenvectors by
-// inverse iteration, one CTA of 128 threads, thread i <-> eigenvalue i.
+// 1c. Eigenvalues of the tridiagonal (d, e) by bisection, one warp each, and
+// eigenvectors by inverse iteration.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int sturm_count(const float *d, const float *e2, int m, float x,
                                            float pivmin)
@@ -229,6 +230,116 @@ __device__ __forceinline__ int sturm_count(const float *d, const float *e2, int 
         cnt += q < 0.f;
     }
     return cnt;
+}
+
+// The tridiagonal scaled by 1 / its Gershgorin bound, in shared memory, by one
+// CTA: the pivot floors are then independent of the matrix scale (a zero
+// matrix gives one cluster at 0 and an orthonormal basis).  lo, hi: the scaled
+// Gershgorin interval; pivmin: the pivot floor of the Sturm counts.
+struct ScaledTri {
+    float d[kEigMax], e[kEigMax], e2[kEigMax];
+    float lo, hi, pivmin;
+};
+
+__device__ __forceinline__ void load_scaled(const float *__restrict__ dg,
+                                            const float *__restrict__ eg, int m, ScaledTri &T)
+{
+    const int tid = threadIdx.x;
+    for (int j = tid; j < m; j += blockDim.x) {
+        T.d[j] = dg[j];
+        T.e[j] = j + 1 < m ? eg[j] : 0.f;
+    }
+    __syncthreads();
+    __shared__ float scale_sh;
+    if (tid < 32) {
+        float lo = INFINITY, hi = -INFINITY;
+        for (int j = tid; j < m; j += 32) {
+            const float r = (j > 0 ? fabsf(T.e[j - 1]) : 0.f) + (j + 1 < m ? fabsf(T.e[j]) : 0.f);
+            lo = fminf(lo, T.d[j] - r);
+            hi = fmaxf(hi, T.d[j] + r);
+        }
+        for (int off = 16; off > 0; off >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+        }
+        if (tid == 0) {
+            const float bound = fmaxf(fabsf(lo), fabsf(hi));
+            const float scale = bound > 0.f ? 1.f / bound : 1.f;
+            scale_sh = scale;
+            T.lo = lo * scale;
+            T.hi = hi * scale;
+        }
+    }
+    __syncthreads();
+    const float scale = scale_sh;
+    for (int j = tid; j < m; j += blockDim.x) {
+        T.d[j] *= scale;
+        T.e[j] *= scale;
+        T.e2[j] = T.e[j] * T.e[j];
+    }
+    __syncthreads();
+    if (tid < 32) {
+        float emax = 0.f;
+        for (int j = tid; j < m; j += 32) emax = fmaxf(emax, T.e2[j]);
+        for (int off = 16; off > 0; off >>= 1) {
+            emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
+        }
+        if (tid == 0) T.pivmin = FLT_MIN * fmaxf(1.f, emax);
+    }
+    __syncthreads();
+}
+
+// Bisection for eigenvalue i, one warp: the 31 midpoints of the next five
+// levels of the bisection tree in one round (lane = node in heap order, its
+// interval formed by the same halvings), then the walk down those levels.  A
+// round is one chain of m dependent divisions, so an eigenvalue takes about 5
+// of them instead of 25, with the interval ends of plain bisection.  (One
+// thread per eigenvalue in the inverse-iteration CTA: 65 of its 127 us at m =
+// 96.  The warps here spread over m / 4 SMs: 16 us.)
+constexpr int kBisectWarps = 4;
+
+__global__ void __launch_bounds__(32 * kBisectWarps)
+eig_bisect_kernel(const float *__restrict__ dg, const float *__restrict__ eg, int m,
+                  float *__restrict__ lam)
+{
+    pdl_wait();  // programmatic dependent launch: predecessor done
+    pdl_trigger();
+    __shared__ ScaledTri T;
+    load_scaled(dg, eg, m, T);
+    const int lane = threadIdx.x & 31;
+    const int i = blockIdx.x * kBisectWarps + (threadIdx.x >> 5);
+    if (i >= m) return;
+    const float tol = 2.f * FLT_EPSILON;
+    float lo = T.lo - tol, hi = T.hi + tol;
+    const int depth = lane > 0 ? 31 - __clz(lane) : 0;
+    bool open = true;
+    for (int it = 0; open && it < 64 && hi - lo > tol;) {
+        float l = lo, h = hi;
+        for (int b = depth - 1; b >= 0; --b) {
+            const float mid = 0.5f * (l + h);
+            if ((lane >> b) & 1) l = mid;
+            else h = mid;
+        }
+        const unsigned above = __ballot_sync(
+            0xffffffffu, sturm_count(T.d, T.e2, m, 0.5f * (l + h), T.pivmin) > i);
+        int node = 1;
+        for (int level = 0; level < 5; ++level, ++it) {
+            if (!(it < 64 && hi - lo > tol)) break;
+            const float mid = 0.5f * (lo + hi);
+            if (mid <= lo || mid >= hi) {
+                open = false;
+                break;
+            }
+            if ((above >> node) & 1u) {
+                hi = mid;
+                node = 2 * node;
+            } else {
+                lo = mid;
+                node = 2 * node + 1;
+            }
+        }
+    }
+    if (lane == 0) lam[i] = 0.5f * (lo + hi);
 }
 
 __device__ __forceinline__ float start_value(int i, int l)
@@ -245,79 +356,40 @@ size_t tri_vectors_smem_bytes(int m)
     return ((size_t)m * kEigPad + 3 * (size_t)m * m) * sizeof(float);
 }
 
+// Inverse iteration, one CTA, thread i <-> eigenvalue i: (Tri - lam I) y = b by
+// Gaussian elimination with partial pivoting (U rows hold up to three entries,
+// the third only in exchanged rows, which one bit per row remembers), tiny
+// pivots replaced by eps ||T||.  The factorisation is made once, by the first
+// of the three iterations; the others reuse its multipliers.  Bound by the
+// chains of dependent divisions along m, one in each elimination and one in
+// each substitution: with the factors kept, four chains instead of six, and
+// the bisection above out of this CTA, 127 -> 65 us at m = 96 and 68 -> 36 at
+// m = 40.
 __global__ void __launch_bounds__(128)
-eig_tri_vectors_kernel(const float *__restrict__ dg, const float *__restrict__ eg, int m,
-                       float *__restrict__ Y, int *info)
+eig_tri_vectors_kernel(const float *__restrict__ dg, const float *__restrict__ eg,
+                       const float *__restrict__ lam_in, int m, float *__restrict__ Y, int *info)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
     // Ys: the vectors, column-major with ld kEigPad (thread i's right-hand
-    // side and solution live in column i); U0..U2: the U rows of every
-    // thread's factorisation, element l of thread i at [l * m + i]
+    // side and solution live in column i); U0, U1: the U rows of every
+    // thread's factorisation and LM its multipliers, element l of thread i at
+    // [l * m + i]
     extern __shared__ float Ys[];
     float *U0 = Ys + (size_t)m * kEigPad;
     float *U1 = U0 + (size_t)m * m;
-    float *U2 = U1 + (size_t)m * m;
-    __shared__ float d[kEigMax], e[kEigMax], e2[kEigMax], lam[kEigMax];
+    float *LM = U1 + (size_t)m * m;
+    __shared__ ScaledTri T;
+    __shared__ float lam[kEigMax];
     __shared__ int cstart[kEigMax], csize[kEigMax];
     __shared__ int ncl;
-    __shared__ float tnorm_sh, pivmin_sh, glo_sh, ghi_sh;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    for (int j = tid; j < m; j += blockDim.x) {
-        d[j] = dg[j];
-        const float ej = j + 1 < m ? eg[j] : 0.f;
-        e[j] = ej;
-        e2[j] = ej * ej;
-    }
-    __syncthreads();
-    // Gershgorin interval; the tridiagonal is then scaled by 1 / its bound so
-    // that the pivot floors below are independent of the matrix scale (a
-    // zero matrix gives one cluster at 0 and an orthonormal basis)
-    if (tid == 0) {
-        float lo = INFINITY, hi = -INFINITY;
-        for (int j = 0; j < m; ++j) {
-            const float r = (j > 0 ? fabsf(e[j - 1]) : 0.f) + (j + 1 < m ? fabsf(e[j]) : 0.f);
-            lo = fminf(lo, d[j] - r);
-            hi = fmaxf(hi, d[j] + r);
-        }
-        const float bound = fmaxf(fabsf(lo), fabsf(hi));
-        const float scale = bound > 0.f ? 1.f / bound : 1.f;
-        tnorm_sh = scale;
-        glo_sh = lo * scale;
-        ghi_sh = hi * scale;
-    }
-    __syncthreads();
-    {
-        const float scale = tnorm_sh;
-        for (int j = tid; j < m; j += blockDim.x) {
-            d[j] *= scale;
-            e[j] *= scale;
-            e2[j] = e[j] * e[j];
-        }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        float emax = 0.f;
-        for (int j = 0; j < m; ++j) emax = fmaxf(emax, e2[j]);
-        pivmin_sh = FLT_MIN * fmaxf(1.f, emax);
-    }
-    __syncthreads();
+    load_scaled(dg, eg, m, T);
+    const float *d = T.d, *e = T.e;
     const float tnorm = 1.f;
-    const float pivmin = pivmin_sh;
-    if (tid < m) {
-        float lo = glo_sh - 2.f * FLT_EPSILON * tnorm;
-        float hi = ghi_sh + 2.f * FLT_EPSILON * tnorm;
-        const float tol = 2.f * FLT_EPSILON * tnorm;
-        for (int it = 0; it < 64 && hi - lo > tol; ++it) {
-            const float mid = 0.5f * (lo + hi);
-            if (mid <= lo || mid >= hi) break;
-            if (sturm_count(d, e2, m, mid, pivmin) > tid) hi = mid;
-            else lo = mid;
-        }
-        lam[tid] = 0.5f * (lo + hi);
-    }
+    for (int j = tid; j < m; j += blockDim.x) lam[j] = lam_in[j];
     __syncthreads();
     // clusters of eigenvalues closer than 1e-3 ||T||; members' shifts are
     // pulled apart to at least 10 eps ||T|| so their factorisations differ
@@ -339,64 +411,88 @@ eig_tri_vectors_kernel(const float *__restrict__ dg, const float *__restrict__ e
         if (info != nullptr) *info = n;
     }
     __syncthreads();
-    // inverse iteration: (Tri - lam I) y = b by Gaussian elimination with
-    // partial pivoting (U rows hold up to three entries), tiny pivots
-    // replaced by eps ||T||
     const float shift = tid < m ? lam[tid] : 0.f;
     const float tiny = FLT_EPSILON * tnorm;
     float *rhs = Ys + (size_t)(tid < m ? tid : 0) * kEigPad;
+    float *u0 = U0 + tid, *u1 = U1 + tid, *lmp = LM + tid;
+    unsigned swapped[4] = {0u, 0u, 0u, 0u};  // bit j: rows j and j + 1 exchanged
     if (tid < m) {
         for (int l = 0; l < m; ++l) rhs[l] = start_value(tid, l);
     }
     for (int it = 0; it < 3; ++it) {
         if (tid < m) {
-            float *u0 = U0 + tid;
-            float *u1 = U1 + tid;
-            float *u2 = U2 + tid;
-            float a = d[0] - shift;  // working row: a at col j, b at col j+1
-            float b = m > 1 ? e[0] : 0.f;
             float w = rhs[0];
-            for (int j = 0; j + 1 < m; ++j) {
-                const float sub = e[j];
-                const float dn = d[j + 1] - shift;
-                const float sup = j + 2 < m ? e[j + 1] : 0.f;
-                const float rn = rhs[j + 1];
-                if (fabsf(a) >= fabsf(sub)) {
-                    const float piv = fabsf(a) < tiny ? copysignf(tiny, a) : a;
-                    const float lm = sub / piv;
-                    u0[j * m] = piv;
-                    u1[j * m] = b;
-                    u2[j * m] = 0.f;
-                    rhs[j] = w;
-                    a = dn - lm * b;
-                    b = sup;
-                    w = rn - lm * w;
-                } else {
-                    const float lm = a / sub;
-                    u0[j * m] = sub;
-                    u1[j * m] = dn;
-                    u2[j * m] = sup;
-                    rhs[j] = rn;
-                    a = b - lm * dn;
-                    b = -lm * sup;
-                    w = w - lm * rn;
+            if (it == 0) {
+                float a = d[0] - shift;  // working row: a at col j, b at col j+1
+                float b = m > 1 ? e[0] : 0.f;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    unsigned bits = 0u;
+                    for (int j = 32 * g; j < 32 * g + 32 && j + 1 < m; ++j) {
+                        const float sub = e[j];
+                        const float dn = d[j + 1] - shift;
+                        const float sup = j + 2 < m ? e[j + 1] : 0.f;
+                        const float rn = rhs[j + 1];
+                        if (fabsf(a) >= fabsf(sub)) {
+                            const float piv = fabsf(a) < tiny ? copysignf(tiny, a) : a;
+                            const float lm = sub / piv;
+                            u0[j * m] = piv;
+                            u1[j * m] = b;
+                            lmp[j * m] = lm;
+                            rhs[j] = w;
+                            a = fmaf(-lm, b, dn);
+                            b = sup;
+                            w = fmaf(-lm, w, rn);
+                        } else {
+                            const float lm = a / sub;
+                            u0[j * m] = sub;
+                            u1[j * m] = dn;
+                            lmp[j * m] = lm;
+                            bits |= 1u << (j & 31);
+                            rhs[j] = rn;
+                            a = fmaf(-lm, dn, b);
+                            b = -lm * sup;
+                            w = fmaf(-lm, rn, w);
+                        }
+                    }
+                    swapped[g] = bits;
+                }
+                u0[(m - 1) * m] = fabsf(a) < tiny ? copysignf(tiny, a) : a;
+            } else {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const unsigned bits = swapped[g];
+                    for (int j = 32 * g; j < 32 * g + 32 && j + 1 < m; ++j) {
+                        const float lm = lmp[j * m];
+                        const float rn = rhs[j + 1];
+                        const bool sw = ((bits >> (j & 31)) & 1u) != 0u;
+                        rhs[j] = sw ? rn : w;
+                        w = sw ? fmaf(-lm, rn, w) : fmaf(-lm, w, rn);
+                    }
                 }
             }
-            u0[(m - 1) * m] = fabsf(a) < tiny ? copysignf(tiny, a) : a;
             rhs[m - 1] = w;
             // back substitution, rescaled against overflow
-            float ymax = 0.f;
-            for (int j = m - 1; j >= 0; --j) {
-                float s = rhs[j];
-                if (j + 1 < m) s -= u1[j * m] * rhs[j + 1];
-                if (j + 2 < m) s -= u2[j * m] * rhs[j + 2];
-                const float y = s / u0[j * m];
-                rhs[j] = y;
-                ymax = fmaxf(ymax, fabsf(y));
-                if (ymax > 1e30f) {
-                    const float sc = 1.f / ymax;
-                    for (int l = j; l < m; ++l) rhs[l] *= sc;
-                    ymax = 1.f;
+            float ymax = 0.f, y1 = 0.f, y2 = 0.f;
+#pragma unroll
+            for (int g = 3; g >= 0; --g) {
+                const unsigned bits = swapped[g];
+                for (int j = min(m - 1, 32 * g + 31); j >= 32 * g; --j) {
+                    float s = rhs[j];
+                    if (j + 1 < m) s = fmaf(-u1[j * m], y1, s);
+                    if (j + 2 < m && ((bits >> (j & 31)) & 1u) != 0u) s = fmaf(-e[j + 1], y2, s);
+                    const float y = s / u0[j * m];
+                    rhs[j] = y;
+                    y2 = y1;
+                    y1 = y;
+                    ymax = fmaxf(ymax, fabsf(y));
+                    if (ymax > 1e30f) {
+                        const float sc = 1.f / ymax;
+                        for (int l = j; l < m; ++l) rhs[l] *= sc;
+                        y1 *= sc;
+                        y2 *= sc;
+                        ymax = 1.f;
+                    }
                 }
             }
             const float sc = ymax > 0.f ? 1.f / ymax : 1.f;
@@ -837,9 +933,12 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
         return IPT_CUDA_INVALID_ARGUMENT;
     }
     const size_t mm = (size_t)m * m;
-    const size_t nfloat = 3 * mm + 3 * (size_t)m;
+    const size_t nfloat = 3 * mm + 4 * (size_t)m;
     const size_t need = 8 * mm + m + kMaxConvBlocks + 2 * kMaxTiles + (nfloat + 1) / 2;
     if (eig_capacity < need) {
+        // without it the pool gives the workspace back at every
+        // synchronisation and the next call maps it anew
+        retain_pool_memory();
         if (eig_scratch != nullptr) {
             cudaFreeAsync(eig_scratch, stream);
             eig_scratch = nullptr;
@@ -866,6 +965,7 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
     float *tau = Yf + mm;
     float *dg = tau + m;
     float *eg = dg + m;
+    float *lamf = eg + m;
     KernelTimerScope timer(kProfSmallEig, stream);
 
     // 1. FP32 eigenvectors of T'
@@ -877,11 +977,15 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
                                     (int)tri_smem));
     IPTGB_CHECK(launch_pdl(eig_tridiag_kernel, dim3(1), dim3(512), tri_smem, stream, Af, m, vh,
                            tau, dg, eg));
+    IPTGB_CHECK(launch_pdl(eig_bisect_kernel, dim3((m + kBisectWarps - 1) / kBisectWarps),
+                           dim3(32 * kBisectWarps), 0, stream, (const float *)dg,
+                           (const float *)eg, m, lamf));
     const size_t vec_smem = tri_vectors_smem_bytes(m);
     IPTGB_CUDA(cudaFuncSetAttribute(eig_tri_vectors_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vec_smem));
-    IPTGB_CHECK(launch_pdl(eig_tri_vectors_kernel, dim3(1), dim3(128), vec_smem, stream, dg, eg, m,
-                           Yf, info_dev));
+    IPTGB_CHECK(launch_pdl(eig_tri_vectors_kernel, dim3(1), dim3(128), vec_smem, stream,
+                           (const float *)dg, (const float *)eg, (const float *)lamf, m, Yf,
+                           info_dev));
     const size_t bt_smem = ((size_t)m * m + m) * sizeof(float);
     IPTGB_CUDA(cudaFuncSetAttribute(eig_backtransform_kernel,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_smem));
