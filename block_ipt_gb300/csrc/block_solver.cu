@@ -349,8 +349,16 @@ int block_solve(const BlockSolveInput &in, double *X_out, double *values_out,
         if (m + nsel > maxb) {
             const int room = restart_keep > 0 ? std::min(restart_keep, maxb - nsel) : maxb - nsel;
             const int kr = std::max(k, std::min(m, room));
-            IPTGB_CHECK(ops.tall_gemm(V.ptr, n, Zm, m, Vt.ptr, n, n, m, kr));
-            IPTGB_CHECK(ops.tall_gemm(AV.ptr, n, Zm, m, AVt.ptr, n, n, m, kr));
+            // the first k columns are the Ritz block formed by the last
+            // Rayleigh-Ritz from the same V and Z (kr >= k)
+            const size_t ritz = (size_t)n * k;
+            IPTGB_CUDA(cudaMemcpyAsync(Vt.ptr, Xr.ptr, ritz * sizeof(double),
+                                       cudaMemcpyDeviceToDevice, s));
+            IPTGB_CUDA(cudaMemcpyAsync(AVt.ptr, AXr.ptr, ritz * sizeof(double),
+                                       cudaMemcpyDeviceToDevice, s));
+            const double *Zk = Zm + (size_t)m * k;
+            IPTGB_CHECK(ops.tall_gemm(V.ptr, n, Zk, m, Vt.ptr + ritz, n, n, m, kr - k));
+            IPTGB_CHECK(ops.tall_gemm(AV.ptr, n, Zk, m, AVt.ptr + ritz, n, n, m, kr - k));
             std::swap(V.ptr, Vt.ptr);
             std::swap(AV.ptr, AVt.ptr);
             m = kr;

@@ -106,6 +106,60 @@ __device__ __forceinline__ void df_acc(float &S, float &s, float ah, float al, f
     s = __fadd_rn(s, __fadd_rn(err, t));
 }
 
+// Two floats in one 64-bit register; each half of a packed instruction is an
+// ordinary round-to-nearest FP32 operation.  Measured on double-float sums: a
+// tall product of 96 x 80 over 63 504 rows takes 247 us with packed terms and
+// 290 with scalar ones, the sparse product 481 against 517.
+using f32x2 = unsigned long long;
+
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// df_acc on two sums at once, the same operations on each half
+__device__ __forceinline__ void df_acc2(f32x2 &S, f32x2 &s, f32x2 ah, f32x2 al, f32x2 bh, f32x2 bl)
+{
+    const f32x2 p = mul2(ah, bh);
+    const f32x2 pe = fma2(ah, bh, p ^ 0x8000000080000000ull);
+    const f32x2 t = fma2(ah, bl, fma2(al, bh, pe));
+    const f32x2 u = add2(S, p);
+    const f32x2 bp = sub2(u, S);
+    const f32x2 err = add2(sub2(S, sub2(u, bp)), sub2(p, bp));
+    S = u;
+    s = add2(s, add2(err, t));
+}
+
 // |h| = |hi| + sgn(hi) lo added to a double-float sum (S, C) on the FP32 pipe
 __device__ __forceinline__ void df_abs_add(float &S, float &C, float hi, float lo)
 {
@@ -118,9 +172,30 @@ __device__ __forceinline__ void df_abs_add(float &S, float &C, float hi, float l
     C = __fadd_rn(C, __fadd_rn(err, bl));
 }
 
-// exact conversions
+// exact conversions.  The leading part of the common case (|v| in [2^-74,
+// 2^127), so that the remainder's scale is a normal float) is the top 24 bits
+// of the significand rounded half to even in integers, the trailing part the
+// signed 29-bit remainder converted by the integer-to-float unit and scaled by
+// its power of two: 17 instructions, with the bits of split_double_bits (which
+// takes the others, 40 instructions).  A zero is common in a sparse problem's
+// vectors and would take the FP64 instructions.
 __device__ __forceinline__ dfloat df_from_double(double v)
 {
+    const uint32_t h32 = (uint32_t)((uint64_t)__double_as_longlong(v) >> 32);
+    const uint32_t l32 = (uint32_t)__double_as_longlong(v);
+    const uint32_t e = (h32 >> 20) & 0x7FFu;
+    if (e - 949u <= 200u) {
+        // exponent e - 896 and the top 23 mantissa bits, sign put back
+        const uint32_t f = ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) |
+                           (h32 & 0x80000000u);
+        const uint32_t rem = l32 & 0x1FFFFFFFu;
+        const uint32_t inc = (rem + (f & 1u) + 0x0FFFFFFFu) >> 29;
+        const int d = (int)rem - (int)(inc << 29);
+        const int sm = (int)h32 >> 31;
+        const float scale = __uint_as_float((e - 948u) << 23);
+        return {__uint_as_float(f + inc), __fmul_rn(__int2float_rn((d ^ sm) - sm), scale)};
+    }
+    if (((h32 & 0x7FFFFFFFu) | l32) == 0u) return {__uint_as_float(h32), 0.0f};
     uint32_t hb, lb;
     if (split_double_bits((uint64_t)__double_as_longlong(v), &hb, &lb)) {
         return {__uint_as_float(hb), __uint_as_float(lb)};

@@ -100,73 +100,114 @@ __global__ void reduce_slices_kernel(const double *__restrict__ P, int slices, s
 }
 
 // The same partial Gram products in double-float arithmetic on the FP32
-// pipe (BlockOps::df_products): tiles split into (hi, lo) floats when staged,
-// df_acc per term; GB300's FP32 pipe runs ~5x more of these terms per second
-// than its FP64 pipe runs FMAs.
-__global__ void __launch_bounds__(256)
+// pipe (BlockOps::df_products): TI x TJ tiles of the output, the operands
+// split into (hi, lo) floats when staged, df_acc2 per pair of columns; GB300's
+// FP32 pipe runs ~5x more of these terms per second than its FP64 pipe runs
+// FMAs.  Bound by that pipe: thread (li, lj) owns row li and the columns 2 lj,
+// 2 lj + 1 (+ 16 q) of the tile, a term is six packed instructions, and the
+// next rows are loaded while this chunk is summed.  TJ = 16 for the blocks of
+// 16 columns that a Davidson step adds (32 did half its work on padding), and
+// TI = 16 for their own Gram matrices.  At 63 504
+// rows a Davidson step's products took 101 us on average and take 53 (18 the
+// 16 x 16 ones).
+constexpr int kGramDfRows = 32;
+
+template <int TI, int TJ>
+__global__ void __launch_bounds__(8 * TI)
 gram_partial_df_kernel(const double *__restrict__ A, long long lda, int ma,
                        const double *__restrict__ B, long long ldb, int mb, int n,
                        int chunks_per_block, double *__restrict__ P)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
-    // (hi, lo) pairs: one 8-byte load per entry
-    __shared__ float2 as2[kGramRows][kGramTile + 1];
-    __shared__ float2 bs2[kGramRows][kGramTile + 1];
-    const int tiles_i = (ma + kGramTile - 1) / kGramTile;
+    constexpr int kThr = 8 * TI;
+    constexpr int kPairs = TJ / 2;
+    constexpr int kOwn = TJ / 16;  // column pairs per thread
+    // two stages of kGramDfRows rows: one is filled while the other is summed
+    __shared__ float2 as2[2][kGramDfRows][TI + 1];
+    // (hi_j, hi_j+1, lo_j, lo_j+1) per column pair, rows padded against bank
+    // conflicts of the staging stores
+    __shared__ ulonglong2 bs2[2][kGramDfRows][kPairs + 1];
+    const int tiles_i = (ma + TI - 1) / TI;
     const int ti = blockIdx.y % tiles_i;
     const int tj = blockIdx.y / tiles_i;
-    const int i0 = ti * kGramTile;
-    const int j0 = tj * kGramTile;
-    const int li = threadIdx.x % kGramTile;
-    const int lj = threadIdx.x / kGramTile;  // 0..7
-    float S[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < chunks_per_block; ++c) {
-        const int r0 = (blockIdx.x * chunks_per_block + c) * kGramRows;
-        if (r0 >= n) {
-            break;
-        }
-        __syncthreads();
-        // loads first (all in flight), then the splits into shared memory
-        constexpr int kPer = kGramRows * kGramTile / 256;
-        double av[kPer], bv[kPer];
+    const int i0 = ti * TI;
+    const int j0 = tj * TJ;
+    const int li = threadIdx.x % TI;
+    const int lj = threadIdx.x / TI;  // 0..7
+    f32x2 S[kOwn], sl[kOwn];
 #pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int e = threadIdx.x + q * 256;
-            const int r = e % kGramRows;
-            const int col = e / kGramRows;
-            const int row = r0 + r;
-            av[q] = (row < n && i0 + col < ma) ? A[(size_t)row + (size_t)(i0 + col) * lda] : 0.0;
-            bv[q] = (row < n && j0 + col < mb) ? B[(size_t)row + (size_t)(j0 + col) * ldb] : 0.0;
+    for (int q = 0; q < kOwn; ++q) S[q] = sl[q] = 0;
+    constexpr int kPerA = kGramDfRows * TI / kThr;
+    constexpr int kPerB = kGramDfRows * TJ / kThr;
+    double av[kPerA], bv[kPerB];
+    const int lr = threadIdx.x % kGramDfRows;  // staged row, first staged column
+    const int lc = threadIdx.x / kGramDfRows;
+    constexpr int kColStep = kThr / kGramDfRows;
+    auto load = [&](int row0) {
+        const int row = row0 + lr;
+#pragma unroll
+        for (int q = 0; q < kPerA; ++q) {
+            const int col = i0 + lc + q * kColStep;
+            av[q] = (row < n && col < ma) ? A[(size_t)row + (size_t)col * lda] : 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < kPer; ++q) {
-            const int e = threadIdx.x + q * 256;
-            const int r = e % kGramRows;
-            const int col = e / kGramRows;
+        for (int q = 0; q < kPerB; ++q) {
+            const int col = j0 + lc + q * kColStep;
+            bv[q] = (row < n && col < mb) ? B[(size_t)row + (size_t)col * ldb] : 0.0;
+        }
+    };
+    auto stage = [&](int buf) {
+#pragma unroll
+        for (int q = 0; q < kPerA; ++q) {
             const dfloat a = df_from_double(av[q]);
-            const dfloat b = df_from_double(bv[q]);
-            as2[r][col] = make_float2(a.hi, a.lo);
-            bs2[r][col] = make_float2(b.hi, b.lo);
+            as2[buf][lr][lc + q * kColStep] = make_float2(a.hi, a.lo);
         }
-        __syncthreads();
-#pragma unroll 4
-        for (int r = 0; r < kGramRows; ++r) {
-            const float2 a = as2[r][li];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float2 b = bs2[r][lj + 8 * q];
-                df_acc(S[q], sl[q], a.x, a.y, b.x, b.y);
+        for (int q = 0; q < kPerB; ++q) {
+            const int col = lc + q * kColStep;
+            const dfloat b = df_from_double(bv[q]);
+            float *o = reinterpret_cast<float *>(&bs2[buf][lr][col >> 1]) + (col & 1);
+            o[0] = b.hi;
+            o[2] = b.lo;
+        }
+    };
+    const int first = blockIdx.x * chunks_per_block * kGramRows;
+    const int last = min(first + chunks_per_block * kGramRows, n);
+    if (first < last) {
+        load(first);
+        stage(0);
+    }
+    int buf = 0;
+    for (int r0 = first; r0 < last; r0 += kGramDfRows, buf ^= 1) {
+        __syncthreads();
+        const bool more = r0 + kGramDfRows < last;
+        if (more) load(r0 + kGramDfRows);
+#pragma unroll(kOwn == 1 ? 16 : 8)
+        for (int r = 0; r < kGramDfRows; ++r) {
+            const float2 a = as2[buf][r][li];
+            const f32x2 ah = pack2(a.x, a.x), al = pack2(a.y, a.y);
+#pragma unroll
+            for (int q = 0; q < kOwn; ++q) {
+                const ulonglong2 b = bs2[buf][r][lj + 8 * q];
+                df_acc2(S[q], sl[q], ah, al, b.x, b.y);
             }
         }
+        if (more) stage(buf ^ 1);
     }
     const size_t mm = (size_t)ma * (size_t)mb;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int i = i0 + li;
-        const int j = j0 + lj + 8 * q;
-        if (i < ma && j < mb) {
-            P[(size_t)blockIdx.x * mm + (size_t)j * ma + i] = (double)S[q] + (double)sl[q];
+    for (int q = 0; q < kOwn; ++q) {
+        float hi[2], lo[2];
+        unpack2(S[q], hi[0], hi[1]);
+        unpack2(sl[q], lo[0], lo[1]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + li;
+            const int j = j0 + 2 * (lj + 8 * q) + u;
+            if (i < ma && j < mb) {
+                P[(size_t)blockIdx.x * mm + (size_t)j * ma + i] = (double)hi[u] + (double)lo[u];
+            }
         }
     }
 }
@@ -212,7 +253,13 @@ int BlockOps::gram(const double *A, long long lda, int ma, const double *B, long
     IPTGB_CHECK(ensure_partials((size_t)blocks_x * mm));
     KernelTimerScope timer(kProfGram, stream);
     if (df_products) {
-        IPTGB_CHECK(launch_pdl(gram_partial_df_kernel, dim3(blocks_x, tiles), dim3(256), 0, stream,
+        // (narrow tiles only where one covers the columns, so that `tiles` holds)
+        const bool narrow = mb <= 16;
+        const bool small = narrow && ma <= 16;
+        auto kernel = small ? gram_partial_df_kernel<16, 16>
+                      : narrow ? gram_partial_df_kernel<32, 16>
+                               : gram_partial_df_kernel<32, 32>;
+        IPTGB_CHECK(launch_pdl(kernel, dim3(blocks_x, tiles), dim3(small ? 128 : 256), 0, stream,
                                A, lda, ma, B, ldb, mb, n, per_block, partials));
         IPTGB_CHECK(launch_pdl(reduce_slices_warp_kernel, dim3(blocks_for(mm * 32)),
                                dim3(kThreads), 0, stream, (const double *)partials, blocks_x, mm, C,
@@ -284,64 +331,66 @@ __global__ void __launch_bounds__(kTallThreads)
     }
 }
 
-// tall_gemm_kernel in double-float arithmetic (BlockOps::df_products): the
-// B tile split into (hi, lo) floats in shared memory, interleaved so that one
-// 16-byte load brings two columns' pairs (every thread of the CTA reads the
-// same address: a broadcast), each A entry split once per row and used for TC
-// columns.
+// tall_gemm_kernel in double-float arithmetic (BlockOps::df_products), one row
+// and TC columns per thread: up to kTallDfK rows of B split into (hi, lo)
+// floats in shared memory, two columns' pairs in one 16-byte broadcast load;
+// each A entry split once per row and used for TC columns by df_acc2, the next
+// kTallDfRun in flight meanwhile.  Bound by the FP32 pipe (63 % busy): over
+// 63 504 rows, 96 x 80 took 427 us and takes 247; 96 x 16, 74 and 36.  More
+// resident warps (79 registers for 96) gave 1 %.
+constexpr int kTallDfK = 128;
+constexpr int kTallDfRun = 4;  // A entries of a row in flight per thread
+
 template <int TC>
-__global__ void __launch_bounds__(kTallThreads)
+__global__ void __launch_bounds__(kTallThreads, TC == 16 ? 6 : 8)
     tall_gemm_df_kernel(const double *__restrict__ A, long long lda, const double *__restrict__ B,
                         long long ldb, double *__restrict__ C, long long ldc, int n, int m, int p,
                         double alpha, double beta)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
-    __shared__ float4 bs4[kTallK][TC / 2];  // (hi_j, lo_j, hi_j+1, lo_j+1)
+    constexpr int kPairs = TC / 2;
+    __shared__ ulonglong2 bs2[kTallDfK][kPairs];  // (hi_j, hi_j+1), (lo_j, lo_j+1)
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     const int c0 = blockIdx.y * TC;
-    float S[TC], sl[TC];
+    f32x2 S[kPairs], sl[kPairs];
 #pragma unroll
-    for (int j = 0; j < TC; ++j) {
-        S[j] = 0.f;
-        sl[j] = 0.f;
-    }
-    for (int l0 = 0; l0 < m; l0 += kTallK) {
+    for (int j = 0; j < kPairs; ++j) S[j] = sl[j] = 0;
+    const double *Ar = A + (row < n ? row : 0);
+    for (int l0 = 0; l0 < m; l0 += kTallDfK) {
+        const int lc = min(kTallDfK, m - l0);
+        double av[kTallDfRun];
+        auto load = [&](int g) {
+#pragma unroll
+            for (int u = 0; u < kTallDfRun; ++u) {
+                av[u] = g + u < lc ? Ar[(size_t)(l0 + g + u) * lda] : 0.0;
+            }
+        };
+        load(0);
         __syncthreads();
-        for (int e = threadIdx.x; e < kTallK * TC / 2; e += blockDim.x) {
-            const int l = e % kTallK;
-            const int j = 2 * (e / kTallK);
-            const bool row_ok = l0 + l < m;
-            const dfloat b0 = df_from_double(
-                (row_ok && c0 + j < p) ? B[(size_t)(l0 + l) + (size_t)(c0 + j) * ldb] : 0.0);
-            const dfloat b1 = df_from_double(
-                (row_ok && c0 + j + 1 < p) ? B[(size_t)(l0 + l) + (size_t)(c0 + j + 1) * ldb]
-                                           : 0.0);
-            bs4[l][j / 2] = make_float4(b0.hi, b0.lo, b1.hi, b1.lo);
+        for (int e = threadIdx.x; e < kTallDfK * kPairs; e += blockDim.x) {
+            const int l = e % kTallDfK;
+            const int j = 2 * (e / kTallDfK);
+            if (l >= lc) continue;
+            const double *b = B + (size_t)(l0 + l);
+            const dfloat b0 = df_from_double(c0 + j < p ? b[(size_t)(c0 + j) * ldb] : 0.0);
+            const dfloat b1 = df_from_double(c0 + j + 1 < p ? b[(size_t)(c0 + j + 1) * ldb] : 0.0);
+            bs2[l][j / 2] = make_ulonglong2(pack2(b0.hi, b1.hi), pack2(b0.lo, b1.lo));
         }
         __syncthreads();
-        if (row < n) {
-            const int lc = min(kTallK, m - l0);
-            // groups of 8 A values in flight per thread: enough loads per
-            // warp without the register cost of a whole chunk (which limits
-            // the resident warps)
+        for (int g = 0; g < lc; g += kTallDfRun) {
+            dfloat a[kTallDfRun];
 #pragma unroll
-            for (int g = 0; g < kTallK; g += 8) {
-                double av[8];
+            for (int u = 0; u < kTallDfRun; ++u) a[u] = df_from_double(av[u]);
+            load(g + kTallDfRun);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    av[u] = g + u < lc ? A[(size_t)row + (size_t)(l0 + g + u) * lda] : 0.0;
-                }
+            for (int u = 0; u < kTallDfRun; ++u) {
+                if (g + u < lc) {
+                    const f32x2 ah = pack2(a[u].hi, a[u].hi), al = pack2(a[u].lo, a[u].lo);
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (g + u < lc) {
-                        const dfloat a = df_from_double(av[u]);
-#pragma unroll
-                        for (int q = 0; q < TC / 2; ++q) {
-                            const float4 b = bs4[g + u][q];
-                            df_acc(S[2 * q], sl[2 * q], a.hi, a.lo, b.x, b.y);
-                            df_acc(S[2 * q + 1], sl[2 * q + 1], a.hi, a.lo, b.z, b.w);
-                        }
+                    for (int q = 0; q < kPairs; ++q) {
+                        const ulonglong2 b = bs2[g + u][q];
+                        df_acc2(S[q], sl[q], ah, al, b.x, b.y);
                     }
                 }
             }
@@ -349,11 +398,18 @@ __global__ void __launch_bounds__(kTallThreads)
     }
     if (row < n) {
 #pragma unroll
-        for (int j = 0; j < TC; ++j) {
-            if (c0 + j < p) {
-                double *o = C + (size_t)row + (size_t)(c0 + j) * ldc;
-                const double v = (double)S[j] + (double)sl[j];
-                *o = beta == 0.0 ? alpha * v : alpha * v + beta * *o;
+        for (int q = 0; q < kPairs; ++q) {
+            float hi[2], lo[2];
+            unpack2(S[q], hi[0], hi[1]);
+            unpack2(sl[q], lo[0], lo[1]);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = 2 * q + u;
+                if (c0 + j < p) {
+                    double *o = C + (size_t)row + (size_t)(c0 + j) * ldc;
+                    const double v = (double)hi[u] + (double)lo[u];
+                    *o = beta == 0.0 ? alpha * v : alpha * v + beta * *o;
+                }
             }
         }
     }

@@ -124,9 +124,10 @@ int launch_csr64_spmm(const int *row_ptr, const int *col_ind, const double *vals
 // by the FP64 pipe at ~81 % of its peak; this one does ~5x more terms per
 // second and is limited by the gathers of X instead.
 // ---------------------------------------------------------------------------
-// Xr2[c * ldr + j] = split(X[c + j * n]) as float2 (hi, lo); 0 beyond k.
+// Row c of Xr2 holds split(X[c + j * n]), 0 beyond k, as (hi_j, hi_j+1, lo_j,
+// lo_j+1) for each pair of columns: the operand pairs of df_acc2.
 __global__ void rowmajor_split_kernel(const double *__restrict__ X, int n, int k,
-                                      float2 *__restrict__ Xr2, int ldr)
+                                      float *__restrict__ Xr2, int ldr)
 {
     __shared__ double t[32][33];
     pdl_wait();  // programmatic dependent launch: predecessor done
@@ -144,45 +145,89 @@ __global__ void rowmajor_split_kernel(const double *__restrict__ X, int n, int k
         const int j = c0 + threadIdx.x;
         if (r < n && j < ldr) {
             const dfloat v = df_from_double(t[threadIdx.x][y]);
-            Xr2[(size_t)r * ldr + j] = make_float2(v.hi, v.lo);
+            float *x = Xr2 + (size_t)r * (2 * ldr) + 4 * (j >> 1) + (j & 1);
+            x[0] = v.hi;
+            x[2] = v.lo;
         }
     }
 }
 
+// Bound by the gathers of X (128 bytes a nonzero for 16 columns, few of them
+// found in L1): a lane's four columns come as one 32-byte load (two 16-byte
+// ones touch each line twice, and the L1's lines per clock were the bound),
+// two nonzeros of a lane per round, the values and columns of the next round
+// already in flight.  582 -> 485 us for 57 million nonzeros (16 TB/s of
+// gathers) at 8 blocks of 4 warps an SM; 4 blocks of 8: 493; without the
+// register limit, at 48 registers: 527; one nonzero per round: 550.
+constexpr int kCsrDfWarps = 4;
+
 template <int BN>
-__global__ void __launch_bounds__(kCsrWarpsPerBlock * 32)
+__global__ void __launch_bounds__(kCsrDfWarps * 32, 8)
 csr_df_spmm_kernel(const int *__restrict__ row_ptr, const int *__restrict__ col_ind,
                    const float *__restrict__ vh, const float *__restrict__ vl, int n,
-                   const float2 *__restrict__ Xr2, int ldr, int k, double *__restrict__ Y)
+                   const float *__restrict__ Xr2, int ldr, int k, double *__restrict__ Y)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
     constexpr int LPN = BN / 4;          // lanes per nonzero
     constexpr int STREAMS = 32 / LPN;    // nonzeros in flight per warp
     const int lane = threadIdx.x & 31;
-    const int row = blockIdx.x * kCsrWarpsPerBlock + (threadIdx.x >> 5);
+    const int row = blockIdx.x * kCsrDfWarps + (threadIdx.x >> 5);
     if (row >= n) {
         return;
     }
     const int sub = lane % LPN;
     const int q = lane / LPN;
     const int col0 = blockIdx.y * BN + 4 * sub;
-    float S[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+    f32x2 S01 = 0, S23 = 0, s01 = 0, s23 = 0;
     const int pbeg = row_ptr[row];
     const int pend = row_ptr[row + 1];
-    const float2 *xb = Xr2 + col0;
-    for (int p = pbeg + q; p < pend; p += STREAMS) {
-        const float h = __ldg(vh + p);
-        const float l = __ldg(vl + p);
-        const int c = __ldg(col_ind + p);
-        const float4 *x = reinterpret_cast<const float4 *>(xb + (size_t)c * ldr);
-        const float4 x01 = __ldg(x);      // (hi, lo) of columns col0, col0 + 1
-        const float4 x23 = __ldg(x + 1);  // and col0 + 2, col0 + 3
-        df_acc(S[0], s[0], h, l, x01.x, x01.y);
-        df_acc(S[1], s[1], h, l, x01.z, x01.w);
-        df_acc(S[2], s[2], h, l, x23.x, x23.y);
-        df_acc(S[3], s[3], h, l, x23.z, x23.w);
+    const float *xb = Xr2 + 2 * col0;
+    auto gather = [&](int c, ulonglong2 &a, ulonglong2 &b) {
+        // (hi, hi), (lo, lo) of columns col0, col0 + 1 and col0 + 2, col0 + 3
+        asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+            : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
+            : "l"(xb + (size_t)c * (2 * ldr)));
+    };
+    auto term = [&](float h, float l, const ulonglong2 &a, const ulonglong2 &b) {
+        const f32x2 hh = pack2(h, h), ll = pack2(l, l);
+        df_acc2(S01, s01, hh, ll, a.x, a.y);
+        df_acc2(S23, s23, hh, ll, b.x, b.y);
+    };
+    int p = pbeg + q;
+    if (p + STREAMS < pend) {
+        float h0 = __ldg(vh + p), h1 = __ldg(vh + p + STREAMS);
+        float l0 = __ldg(vl + p), l1 = __ldg(vl + p + STREAMS);
+        int c0 = __ldg(col_ind + p), c1 = __ldg(col_ind + p + STREAMS);
+        do {
+            ulonglong2 a0, b0, a1, b1;
+            gather(c0, a0, b0);
+            gather(c1, a1, b1);
+            p += 2 * STREAMS;
+            const float g0 = h0, g1 = h1, m0 = l0, m1 = l1;
+            if (p + STREAMS < pend) {
+                h0 = __ldg(vh + p);
+                h1 = __ldg(vh + p + STREAMS);
+                l0 = __ldg(vl + p);
+                l1 = __ldg(vl + p + STREAMS);
+                c0 = __ldg(col_ind + p);
+                c1 = __ldg(col_ind + p + STREAMS);
+            }
+            term(g0, m0, a0, b0);
+            term(g1, m1, a1, b1);
+        } while (p + STREAMS < pend);
     }
+    if (p < pend) {
+        ulonglong2 a, b;
+        gather(__ldg(col_ind + p), a, b);
+        term(__ldg(vh + p), __ldg(vl + p), a, b);
+    }
+    float S[4], s[4];
+    unpack2(S01, S[0], S[1]);
+    unpack2(S23, S[2], S[3]);
+    unpack2(s01, s[0], s[1]);
+    unpack2(s23, s[2], s[3]);
+    __syncwarp();
 #pragma unroll
     for (int off = 16; off >= LPN; off >>= 1) {
 #pragma unroll
@@ -212,17 +257,17 @@ int launch_csr_df_spmm(const int *row_ptr, const int *col_ind, const float *vh, 
     const int bn = k <= 4 ? 4 : (k <= 8 ? 8 : 16);
     const int nblk = (k + bn - 1) / bn;
     const int ldr = nblk * bn;
-    DeviceBuffer<float2> Xr2;
-    IPTGB_CHECK(Xr2.alloc((size_t)n * ldr, stream));
+    DeviceBuffer<float> Xr2;
+    IPTGB_CHECK(Xr2.alloc((size_t)n * ldr * 2, stream));
     IPTGB_CHECK(launch_pdl(rowmajor_split_kernel, dim3((n + 31) / 32, (ldr + 31) / 32),
                            dim3(32, 8), 0, stream, X, n, k, Xr2.ptr, ldr));
-    dim3 grid((n + kCsrWarpsPerBlock - 1) / kCsrWarpsPerBlock, nblk);
-    const dim3 threads(kCsrWarpsPerBlock * 32);
+    dim3 grid((n + kCsrDfWarps - 1) / kCsrDfWarps, nblk);
+    const dim3 threads(kCsrDfWarps * 32);
     auto kernel = bn == 4 ? csr_df_spmm_kernel<4>
                   : bn == 8 ? csr_df_spmm_kernel<8>
                             : csr_df_spmm_kernel<16>;
     return launch_pdl(kernel, grid, threads, 0, stream, row_ptr, col_ind, vh, vl, n,
-                      (const float2 *)Xr2.ptr, ldr, k, Y);
+                      (const float *)Xr2.ptr, ldr, k, Y);
 }
 
 int launch_ipt_update_from_y(const double *Y, int n, int k, const double *X, const double *d,

@@ -34,16 +34,9 @@ __global__ void df_split_kernel(const double *__restrict__ A, size_t count,
     pdl_trigger();
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
-    const double a = A[e];
-    uint32_t hb, lb;
-    if (split_double_bits((unsigned long long)__double_as_longlong(a), &hb, &lb)) {
-        hi[e] = __uint_as_float(hb);
-        lo[e] = __uint_as_float(lb);
-    } else {
-        const float h = __double2float_rn(a);
-        hi[e] = h;
-        lo[e] = __double2float_rn(a - (double)h);
-    }
+    const dfloat v = df_from_double(A[e]);
+    hi[e] = v.hi;
+    lo[e] = v.lo;
 }
 
 __device__ __forceinline__ void df_term(float &S, float &s, float hh, float hl, float xh, float xl)
