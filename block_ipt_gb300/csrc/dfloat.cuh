@@ -179,22 +179,30 @@ __device__ __forceinline__ void df_abs_add(float &S, float &C, float hi, float l
 // its power of two: 17 instructions, with the bits of split_double_bits (which
 // takes the others, 40 instructions).  A zero is common in a sparse problem's
 // vectors and would take the FP64 instructions.
+__device__ __forceinline__ bool df_common_exponent(uint32_t h32)
+{
+    return ((h32 >> 20) & 0x7FFu) - 949u <= 200u;
+}
+
+__device__ __forceinline__ dfloat df_from_common(uint32_t h32, uint32_t l32)
+{
+    const uint32_t e = (h32 >> 20) & 0x7FFu;
+    // exponent e - 896 and the top 23 mantissa bits, sign put back
+    const uint32_t f =
+        ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) | (h32 & 0x80000000u);
+    const uint32_t rem = l32 & 0x1FFFFFFFu;
+    const uint32_t inc = (rem + (f & 1u) + 0x0FFFFFFFu) >> 29;
+    const int d = (int)rem - (int)(inc << 29);
+    const int sm = (int)h32 >> 31;
+    const float scale = __uint_as_float((e - 948u) << 23);
+    return {__uint_as_float(f + inc), __fmul_rn(__int2float_rn((d ^ sm) - sm), scale)};
+}
+
 __device__ __forceinline__ dfloat df_from_double(double v)
 {
     const uint32_t h32 = (uint32_t)((uint64_t)__double_as_longlong(v) >> 32);
     const uint32_t l32 = (uint32_t)__double_as_longlong(v);
-    const uint32_t e = (h32 >> 20) & 0x7FFu;
-    if (e - 949u <= 200u) {
-        // exponent e - 896 and the top 23 mantissa bits, sign put back
-        const uint32_t f = ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) |
-                           (h32 & 0x80000000u);
-        const uint32_t rem = l32 & 0x1FFFFFFFu;
-        const uint32_t inc = (rem + (f & 1u) + 0x0FFFFFFFu) >> 29;
-        const int d = (int)rem - (int)(inc << 29);
-        const int sm = (int)h32 >> 31;
-        const float scale = __uint_as_float((e - 948u) << 23);
-        return {__uint_as_float(f + inc), __fmul_rn(__int2float_rn((d ^ sm) - sm), scale)};
-    }
+    if (df_common_exponent(h32)) return df_from_common(h32, l32);
     if (((h32 & 0x7FFFFFFFu) | l32) == 0u) return {__uint_as_float(h32), 0.0f};
     uint32_t hb, lb;
     if (split_double_bits((uint64_t)__double_as_longlong(v), &hb, &lb)) {

@@ -925,18 +925,14 @@ struct alignas(2 * sizeof(LP)) LpPair {  // two adjacent Delta entries, one stor
 // of the power-of-two scale).
 __device__ __forceinline__ float sym_entry(double h, int s2, double scale, float &hi, float &lo)
 {
-    uint32_t hb, lb;
-    if (split_double_bits((unsigned long long)__double_as_longlong(h), &hb, &lb)) {
-        hi = __uint_as_float(hb);
-        lo = __uint_as_float(lb);
-        const int ex = (int)((hb >> 23) & 0xFFu) + s2;
-        if (ex >= 1 && ex <= 254) {
-            return __uint_as_float(hb + ((uint32_t)s2 << 23));
-        }
-    } else {
-        hi = __double2float_rn(h);
-        lo = __double2float_rn(h - (double)hi);
-    }
+    const dfloat v = df_from_double(h);
+    hi = v.hi;
+    lo = v.lo;
+    const uint32_t hb = __float_as_uint(v.hi);
+    const uint32_t e = (hb >> 23) & 0xFFu;
+    const int ex = (int)e + s2;
+    if (e - 1u <= 253u && ex >= 1 && ex <= 254) return __uint_as_float(hb + ((uint32_t)s2 << 23));
+    if (((unsigned long long)__double_as_longlong(h) << 1) == 0ull) return hi;
     return (float)(scale * h);
 }
 
@@ -1022,123 +1018,160 @@ __global__ void __launch_bounds__(256)
 
 // Fused setup of a symmetric H: one CTA per column c (= row c of Delta).
 // Pass 0 reads the column (writing the FP64 device copy when the source is
-// host memory) and finds its largest off-diagonal |h| (integer max of the bit
-// patterns); the row's FP16 scale is the largest power of two 2^s2 with
-// 2^s2 max <= 16384 (BF16/TF32: 1).  Pass 1 re-reads the column from device
-// memory (L2-resident by then: the source over the host link is read once)
-// and writes row c of Delta and the double-FP32 split of column c, and forms
-// the exact double-float column sum.  The CTA's thread 0 then stores 2^-s2, the
-// diagonal entry, the column sum (atomic max: hnorm), its maximum and whether
-// d_{c+1} < d_c.  No FP64 arithmetic per entry (the conversions run on the
-// integer pipe), so the pass streams at memory (or host link) speed.
+// host memory) and finds its largest off-diagonal |h|; the row's FP16 scale is
+// the largest power of two 2^s2 with 2^s2 max <= 16384 (BF16/TF32: 1).  Pass 1
+// writes row c of Delta, its digit words and the double-FP32 split of column
+// c, and forms the double-float column sum.  The CTA's thread 0 then stores
+// 2^-s2, the diagonal entry, the column sum (atomic max: hnorm), its maximum
+// and whether d_{c+1} < d_c.
+//
+// Bound by the integer pipe (the conversions run there: the FP64 pipe would
+// take longer), so every step of an entry is kept short: pass 0 compares the
+// high words alone and looks at the low ones only where they can matter, the
+// split is df_from_double's, the scaled value one FP32 multiplication, and the
+// diagonal pair, zeros and the end of the column take a branch of their own.
+// Two entry pairs per round: the registers that takes leave five CTAs on an SM,
+// whose columns L2 still holds in pass 1 (eight read 0.4 GB more from memory).
+// n = 8192, FP16 with digit words: 373 -> 285 us, 1.23 GB, the integer pipe
+// 66 % busy; keeping the column in shared memory (three CTAs) took 321.
+constexpr int kSetupThreads = 256;
+
 template <typename LP>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kSetupThreads)
     fused_setup_kernel(const double *__restrict__ src, int n, int ldp, int fp16_scale,
                        double *__restrict__ copy, LP *__restrict__ delta, float *__restrict__ hi,
                        float *__restrict__ lo, float *__restrict__ inv_row,
                        double *__restrict__ diag, DenseStats *__restrict__ stats, int vec,
                        int *__restrict__ oz_rowexp, uint4 *__restrict__ oz_words, int c0)
 {
-    __shared__ unsigned long long wmax[8];
+    __shared__ uint32_t wmax[8];
+    __shared__ uint32_t wlow[8];
     __shared__ float wS[8], wC[8];
-    __shared__ int s2_sh;
     const int c = c0 + blockIdx.x;
     const int tid = threadIdx.x;
+    const int cpair = c & ~1;
     const double *scol = src + (size_t)c * n;
     double *ccol = copy != nullptr ? copy + (size_t)c * n : nullptr;
-    unsigned long long m = 0;
-    if (vec) {  // n even, src (and copy) 16-byte aligned
-        const double2 *s2v = reinterpret_cast<const double2 *>(scol);
-        for (int q = tid; q < n / 2; q += 256) {
-            const double2 v = s2v[q];
-            if (ccol != nullptr) reinterpret_cast<double2 *>(ccol)[q] = v;
-            const int l = 2 * q;
-            const unsigned long long a0 =
-                (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFULL;
-            const unsigned long long a1 =
-                (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFULL;
-            if (l != c && a0 > m) m = a0;
-            if (l + 1 != c && a1 > m) m = a1;
+    // the largest high word of the off-diagonal |h|, NaNs and infinities too
+    uint32_t m = 0;
+    auto abs_hi = [](double v) { return (uint32_t)__double2hiint(v) & 0x7FFFFFFFu; };
+#pragma unroll 8
+    for (int l = 2 * tid; l < n; l += 2 * kSetupThreads) {
+        double2 v = make_double2(0.0, 0.0);
+        if (vec) {  // n even, src (and copy) 16-byte aligned
+            v = *reinterpret_cast<const double2 *>(scol + l);
+            if (ccol != nullptr) *reinterpret_cast<double2 *>(ccol + l) = v;
+        } else {
+            v.x = scol[l];
+            if (l + 1 < n) v.y = scol[l + 1];
+            if (ccol != nullptr) {
+                ccol[l] = v.x;
+                if (l + 1 < n) ccol[l + 1] = v.y;
+            }
         }
-    } else {
-        for (int l = tid; l < n; l += 256) {
-            const double v = scol[l];
-            if (ccol != nullptr) ccol[l] = v;
-            const unsigned long long a =
-                (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
-            if (l != c && a > m) m = a;
+        uint32_t a0 = abs_hi(v.x), a1 = abs_hi(v.y);
+        if (l == cpair) {
+            if (c & 1) a1 = 0;
+            else a0 = 0;
         }
+        m = max(m, max(a0, a1));
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
-        if (o > m) m = o;
-    }
+    m = __reduce_max_sync(0xffffffffu, m);
     if ((tid & 31) == 0) wmax[tid >> 5] = m;
     __syncthreads();
-    if (tid == 0) {
-        unsigned long long mx = 0;
-        for (int w = 0; w < 8; ++w) mx = wmax[w] > mx ? wmax[w] : mx;
-        wmax[0] = mx;
-        int s2 = 0;
-        const double mv = __longlong_as_double((long long)mx);
-        if (fp16_scale && mv > 0.0 && isfinite(mv)) {
-            s2 = (int)floor(log2(16384.0 / mv));
-            s2 = min(max(s2, -40), 40);
-        }
-        s2_sh = s2;
-    }
-    __syncthreads();
-    const int s2 = s2_sh;
-    const double scale = ldexp(1.0, s2);
-    // exponent and digit words of row c (symmetric H: column c is row c)
-    const int oz_e = oz_exponent(wmax[0]);
-    const int oz_nst = (n + 31) / 32;
-    // the block's pass-0 writes of the copy are visible after the barrier;
-    // pass 1 reads with ld.global.cg (coherent at L2), never through the
-    // read-only path, since the copy is written by this kernel
+    uint32_t mh = wmax[0];
+    for (int w = 1; w < 8; ++w) mh = max(mh, wmax[w]);
+    // the passes below read with ld.global.cg (coherent at L2), never through
+    // the read-only path, since the copy is written by this kernel
     const double *rcol = ccol != nullptr ? ccol : scol;
+    auto pair_at = [&](int l) {
+        double2 v = make_double2(0.0, 0.0);
+        if (vec && l + 1 < n) {
+            v = __ldcg(reinterpret_cast<const double2 *>(rcol + l));
+        } else {
+            if (l < n) v.x = __ldcg(rcol + l);
+            if (l + 1 < n) v.y = __ldcg(rcol + l + 1);
+        }
+        return v;
+    };
+    // the low word of the maximum: for the scale where the high word alone is
+    // a power of two or subnormal, and for the matrix's maximum where this
+    // column may hold it
+    const uint32_t known =
+        (uint32_t)(*(volatile unsigned long long *)&stats->maxabs_bits >> 32);
+    uint32_t ml = 0;
+    if (__syncthreads_or((mh & 0xFFFFFu) == 0u || mh < 0x00100000u || mh >= known)) {
+        for (int l = 2 * tid; l < n; l += 2 * kSetupThreads) {
+            const double2 v = pair_at(l);
+            if (l != c && abs_hi(v.x) == mh) ml = max(ml, (uint32_t)__double2loint(v.x));
+            if (l + 1 < n && l + 1 != c && abs_hi(v.y) == mh) {
+                ml = max(ml, (uint32_t)__double2loint(v.y));
+            }
+        }
+        ml = __reduce_max_sync(0xffffffffu, ml);
+        if ((tid & 31) == 0) wlow[tid >> 5] = ml;
+        __syncthreads();
+        for (int w = 0; w < 8; ++w) ml = max(ml, wlow[w]);
+    }
+    const unsigned long long mx = ((unsigned long long)mh << 32) | ml;
+    int s2 = 0;
+    if (fp16_scale && mx > 0 && mh < 0x7FF00000u) {
+        s2 = 14 + 1023 - (int)(mh >> 20) - ((mx & 0xFFFFFFFFFFFFFULL) != 0 ? 1 : 0);
+        s2 = min(max(s2, -40), 40);
+    }
+    const float scale = __uint_as_float((uint32_t)(127 + s2) << 23);
+    // exponent and digit words of row c (symmetric H: column c is row c)
+    const int oz_e = oz_exponent(mx);
+    const int oz_nst = (n + 31) / 32;
+    const int nb = oz_shift_base<kOzSlices>(oz_e);
+    const bool oz_fast = oz_e == kOzNonFinite || oz_e >= kOzFastExp;
     LP *orow = delta + (size_t)c * ldp;
     float S = 0.0f, C = 0.0f;
-    for (int l = 2 * tid; l < ldp; l += 512) {  // ldp is a multiple of 64: l + 1 < ldp
-        double h0 = 0.0, h1 = 0.0;
-        if (vec && l + 1 < n) {
-            const double2 v = __ldcg(reinterpret_cast<const double2 *>(rcol + l));
-            h0 = v.x;
-            h1 = v.y;
-        } else {
-            if (l < n) h0 = __ldcg(rcol + l);
-            if (l + 1 < n) h1 = __ldcg(rcol + l + 1);
+    // a thread's next pair lies 2 kSetupThreads / 32 stages further on
+    uint4 *wp = oz_words != nullptr ? oz_words + oz_word_index(c, 2 * tid, oz_nst) : nullptr;
+    constexpr size_t kWordStep = (size_t)(2 * kSetupThreads / 32) * 128 * 16;
+#pragma unroll 2
+    for (int l = 2 * tid; l < ldp; l += 2 * kSetupThreads) {  // ldp is a multiple of 64
+        const double2 h = pair_at(l);
+        dfloat x, y;
+        uint64_t w0, w1;
+        const uint32_t u0 = (uint32_t)__double2hiint(h.x), u1 = (uint32_t)__double2hiint(h.y);
+        const bool in0 = l < n && l != c, in1 = l + 1 < n && l + 1 != c;
+        if (df_common_exponent(u0) && df_common_exponent(u1) && l != cpair && oz_fast) {
+            x = df_from_common(u0, (uint32_t)__double2loint(h.x));
+            y = df_from_common(u1, (uint32_t)__double2loint(h.y));
+            w0 = oz_biased<kOzSlices>(h.x, nb);
+            w1 = oz_biased<kOzSlices>(h.y, nb);
+        } else {  // zeros (and the end of the column) among them
+            x = df_from_double(h.x);
+            y = df_from_double(h.y);
+            w0 = oz_biased_any<kOzSlices>(in0 ? h.x : 0.0, oz_e);
+            w1 = oz_biased_any<kOzSlices>(in1 ? h.y : 0.0, oz_e);
         }
-        float a0, a1, b0, b1;
-        float v0 = sym_entry(h0, s2, scale, a0, b0);
-        float v1 = sym_entry(h1, s2, scale, a1, b1);
-        if (!(l < n && l != c)) v0 = 0.0f;
-        if (!(l + 1 < n && l + 1 != c)) v1 = 0.0f;
+        // 2^s2 hi: FP16 rounds it as it does RN(2^s2 h), for a subnormal one
+        // is zero there; the other types have s2 = 0
+        const float v0 = l != c ? __fmul_rn(x.hi, scale) : 0.0f;
+        const float v1 = l + 1 != c ? __fmul_rn(y.hi, scale) : 0.0f;
         *reinterpret_cast<LpPair<LP> *>(orow + l) = LpPair<LP>{to_lp<LP>(v0), to_lp<LP>(v1)};
-        if (oz_words != nullptr && l < 32 * oz_nst) {
-            oz_words[oz_word_index(c, l, oz_nst)] = oz_pack_pair<kOzSlices>(
-                oz_biased_any<kOzSlices>((l < n && l != c) ? h0 : 0.0, oz_e),
-                oz_biased_any<kOzSlices>((l + 1 < n && l + 1 != c) ? h1 : 0.0, oz_e));
+        if (wp != nullptr) {
+            if (l < 32 * oz_nst) *wp = oz_pack_pair<kOzSlices>(w0, w1);
+            wp += kWordStep;
         }
-        df_abs_add(S, C, a0, b0);  // entries beyond n are zero
-        df_abs_add(S, C, a1, b1);
-        const size_t o = (size_t)c * n + l;
-        if (vec && l + 1 < n) {
-            if (hi != nullptr) {
-                *reinterpret_cast<float2 *>(hi + o) = make_float2(a0, a1);
-                *reinterpret_cast<float2 *>(lo + o) = make_float2(b0, b1);
-            }
-        } else {
-            if (l < n) {
-                if (hi != nullptr) {
-                    hi[o] = a0;
-                    lo[o] = b0;
+        df_abs_add(S, C, x.hi, x.lo);  // entries beyond n are zero
+        df_abs_add(S, C, y.hi, y.lo);
+        if (hi != nullptr) {
+            const size_t o = (size_t)c * n + l;
+            if (vec && l + 1 < n) {
+                *reinterpret_cast<float2 *>(hi + o) = make_float2(x.hi, y.hi);
+                *reinterpret_cast<float2 *>(lo + o) = make_float2(x.lo, y.lo);
+            } else {
+                if (l < n) {
+                    hi[o] = x.hi;
+                    lo[o] = x.lo;
                 }
-            }
-            if (l + 1 < n) {
-                if (hi != nullptr) {
-                    hi[o + 1] = a1;
-                    lo[o + 1] = b1;
+                if (l + 1 < n) {
+                    hi[o + 1] = y.hi;
+                    lo[o + 1] = y.lo;
                 }
             }
         }
@@ -1159,15 +1192,27 @@ __global__ void __launch_bounds__(256)
         if (colsum > 0.0) {
             atomicMax(&stats->hnorm_bits, (unsigned long long)__double_as_longlong(colsum));
         }
-        if (wmax[0] > 0) atomicMax(&stats->maxabs_bits, wmax[0]);
+        if (mx > 0) atomicMax(&stats->maxabs_bits, mx);
         const double dc = __ldcg(rcol + c);
         diag[c] = dc;
         if (c + 1 < n && src[(size_t)(c + 1) * ((size_t)n + 1)] < dc) {
             atomicAdd(&stats->descents, 1ULL);
         }
-        inv_row[c] = (float)ldexp(1.0, -s2);
+        inv_row[c] = __uint_as_float((uint32_t)(127 - s2) << 23);
         if (oz_rowexp != nullptr) oz_rowexp[c] = oz_e;
     }
+}
+
+template <typename LP>
+int launch_fused_setup(const double *src, int n, int ldp, int fp16_scale, double *copy, LP *delta,
+                       float *hi, float *lo, float *inv_row, double *diag, DenseStats *stats,
+                       int vec, int *oz_rowexp, uint4 *oz_words, int c0, int c1, cudaStream_t s)
+{
+    fused_setup_kernel<LP><<<c1 - c0, kSetupThreads, 0, s>>>(
+        src, n, ldp, fp16_scale, copy, delta, hi, lo, inv_row, diag, stats, vec, oz_rowexp,
+        oz_words, c0);
+    IPTGB_LAUNCH();
+    return IPT_CUDA_SUCCESS;
 }
 
 // Upper triangle of a symmetric H (column-major, ld = n) in pinned host
@@ -1929,7 +1974,6 @@ struct LowpDense final : LowpDenseOperator {
         if (su.fused_src != nullptr && symmetric && n <= kFusedSetupMaxN && su.diag != nullptr &&
             su.stats != nullptr) {
             IPTGB_CHECK(inv_rows.alloc((size_t)n, s));
-            auto kfn = fused_setup_kernel<LP>;
             const int vec = (n % 2 == 0) &&
                             ((reinterpret_cast<uintptr_t>(su.fused_src) & 15) == 0) &&
                             ((reinterpret_cast<uintptr_t>(split_hi) & 7) == 0) &&
@@ -1938,11 +1982,10 @@ struct LowpDense final : LowpDenseOperator {
             if (su.upper_host != nullptr && su.fused_copy != nullptr) {
                 IPTGB_CHECK(upper_pipeline(su, split_hi, split_lo));
             } else {
-                kfn<<<n, 256, 0, s>>>(su.fused_src, n, ldp,
-                                         LowpTypes<LP>::kind == kLowpF16 ? 1 : 0, su.fused_copy,
-                                         delta.ptr, split_hi, split_lo, inv_rows.ptr, su.diag,
-                                         su.stats, vec, su.oz_rowexp, su.oz_words, 0);
-                IPTGB_LAUNCH();
+                IPTGB_CHECK(launch_fused_setup<LP>(
+                    su.fused_src, n, ldp, LowpTypes<LP>::kind == kLowpF16 ? 1 : 0, su.fused_copy,
+                    delta.ptr, split_hi, split_lo, inv_rows.ptr, su.diag, su.stats, vec,
+                    su.oz_rowexp, su.oz_words, 0, n, s));
             }
             scale = 1.0;  // per-row scales in inv_rows
             per_row_scales = true;
@@ -2062,14 +2105,14 @@ struct LowpDense final : LowpDenseOperator {
                 break;
             }
             count_launch();
-            fused_setup_kernel<LP><<<c1 - c0, 256, 0, s2>>>(
+            const int setup = launch_fused_setup<LP>(
                 su.fused_copy, n, ldp, LowpTypes<LP>::kind == kLowpF16 ? 1 : 0, nullptr, delta.ptr,
-                split_hi, split_lo, inv_rows.ptr, su.diag, su.stats, vec, su.oz_rowexp, su.oz_words, c0);
-            if (cudaGetLastError() != cudaSuccess) {
-                fail(IPT_CUDA_CUDA_ERROR);
+                split_hi, split_lo, inv_rows.ptr, su.diag, su.stats, vec, su.oz_rowexp,
+                su.oz_words, c0, c1, s2);
+            if (setup != IPT_CUDA_SUCCESS) {
+                fail(setup);
                 break;
             }
-            count_launch();
         }
         trace_mark("upper:setups_done", s2);
         // s continues after the last setup
