@@ -670,46 +670,63 @@ small_gemm64_kernel(SmallGemmJob j0, SmallGemmJob j1, int m)
 // (Z <- Z (I + R/2), a first-order Z (Z^T Z)^{-1/2}).  Block 0 writes the
 // eigenvalue estimates l.
 // ---------------------------------------------------------------------------
-__global__ void oa_e_kernel(const double *__restrict__ G, const double *__restrict__ S,
-                            const double *__restrict__ fro_part, int nfro,
-                            const double *__restrict__ r_part, const double *__restrict__ s_part,
-                            int ntiles, int m, double ebound, double *__restrict__ E,
-                            double *__restrict__ lam)
+struct RefineStats {
+    const double *fro_part;
+    const double *r_part;
+    const double *s_part;
+    int nfro;
+    int ntiles;
+};
+
+// delta and the eigenvalue estimates l_i = S_ii / G_ii of a CTA of at least
+// 256 threads: warp 0 sums the partials (its three sums and square roots share
+// the FP64 pipe's lanes), the others divide, once per eigenvalue.
+struct RefineScalars {
+    double delta;
+    double l[kEigMax];
+};
+
+__device__ __forceinline__ void oa_scalars(const double *G, const double *S, const RefineStats &st,
+                                           int m, RefineScalars &out)
 {
-    pdl_wait();  // programmatic dependent launch: predecessor done
-    pdl_trigger();
-    __shared__ double delta_sh;
     const int tid = threadIdx.x;
     if (tid < 32) {
         double f = 0.0, rr = 0.0, ss = 0.0;
-        for (int x = tid; x < nfro; x += 32) f += fro_part[x];
-        for (int x = tid; x < ntiles; x += 32) {
-            rr += r_part[x];
-            ss += s_part[x];
+        for (int x = tid; x < st.nfro; x += 32) f += st.fro_part[x];
+        for (int x = tid; x < st.ntiles; x += 32) {
+            rr += st.r_part[x];
+            ss += st.s_part[x];
         }
-        f = warp_sum_d(f);
-        rr = warp_sum_d(rr);
-        ss = warp_sum_d(ss);
-        if (tid == 0) delta_sh = 2.0 * (sqrt(ss) + sqrt(f) * sqrt(rr));
+        const bool up8 = (tid & 8) != 0;
+        const double a = pair_fold16(f, rr);
+        const double b = ss + __shfl_xor_sync(0xffffffffu, ss, 16);
+        double v = (up8 ? b : a) + __shfl_xor_sync(0xffffffffu, up8 ? a : b, 8);
+        for (int off = 4; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        const double q = sqrt(v);  // lane 0: f, lane 16: rr, lane 8: ss
+        const double qf = __shfl_sync(0xffffffffu, q, 0);
+        const double qr = __shfl_sync(0xffffffffu, q, 16);
+        const double qs = __shfl_sync(0xffffffffu, q, 8);
+        if (tid == 0) out.delta = 2.0 * (qs + qf * qr);
+    } else {
+        for (int i = tid - 32; i < m; i += blockDim.x - 32) {
+            const size_t o = (size_t)i * m + i;
+            out.l[i] = S[o] / G[o];
+        }
     }
     __syncthreads();
-    if (blockIdx.x == 0) {
-        for (int i = tid; i < m; i += blockDim.x) {
-            const size_t o = (size_t)i * m + i;
-            lam[i] = S[o] / G[o];
-        }
-    }
-    const int x = blockIdx.x * blockDim.x + tid;
-    if (x >= m * m) return;
+}
+
+__device__ __forceinline__ double oa_entry(const double *G, const double *S,
+                                           const RefineScalars &sc, int m, double ebound, int x)
+{
     const int j = x / m;
     const int i = x - j * m;
     const double r = (i == j ? 1.0 : 0.0) - G[x];
     double val = 0.5 * r;
     if (i != j && ebound > 0.0) {
-        const double li = S[(size_t)i * m + i] / G[(size_t)i * m + i];
-        const double lj = S[(size_t)j * m + j] / G[(size_t)j * m + j];
+        const double li = sc.l[i], lj = sc.l[j];
         const double gap = lj - li;
-        if (fabs(gap) > delta_sh) {
+        if (fabs(gap) > sc.delta) {
             const double num = S[x] + lj * r;
             // the transposed entry's numerator, for a symmetric decision
             const double num_t = S[(size_t)i * m + j] + li * r;
@@ -718,7 +735,20 @@ __global__ void oa_e_kernel(const double *__restrict__ G, const double *__restri
             }
         }
     }
-    E[x] = val;
+    return val;
+}
+
+__global__ void __launch_bounds__(256)
+oa_e_kernel(const double *__restrict__ G, const double *__restrict__ S, RefineStats st, int m,
+            double ebound, double *__restrict__ E, double *__restrict__ lam)
+{
+    pdl_wait();  // programmatic dependent launch: predecessor done
+    pdl_trigger();
+    __shared__ RefineScalars sc;
+    oa_scalars(G, S, st, m, sc);
+    if (blockIdx.x == 0 && threadIdx.x < m) lam[threadIdx.x] = sc.l[threadIdx.x];
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x < m * m) E[x] = oa_entry(G, S, sc, m, ebound, x);
 }
 
 // ---------------------------------------------------------------------------
@@ -996,6 +1026,7 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
     const int tiles = (m + 7) / 8;
     const int ntiles = tiles * tiles;
     const int egrid = blocks_for(mm);
+    const RefineStats stats = {fro_part, r_part, s_part, cgrid, ntiles};
     auto gemm = [&](SmallGemmJob a, SmallGemmJob b, int count) -> int {
         return launch_pdl(small_gemm64_kernel, dim3(tiles, tiles, count), dim3(64), 0, stream, a,
                           b, m);
@@ -1004,8 +1035,8 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
         IPTGB_CHECK((gemm({cur, cur, nullptr, G, 1, 1, nullptr, r_part},      // G = Z^T Z, ||R||
                           {Tp, cur, nullptr, TZ, 0, 0, nullptr, nullptr}, 2)));  // TZ = T' Z
         IPTGB_CHECK((gemm({cur, TZ, nullptr, S, 1, 2, G, s_part}, {}, 1)));  // S = Z^T T' Z
-        IPTGB_CHECK(launch_pdl(oa_e_kernel, dim3(egrid), dim3(kThreads), 0, stream, G, S,
-                               fro_part, cgrid, r_part, s_part, ntiles, m, ebound, E, lam));
+        IPTGB_CHECK(launch_pdl(oa_e_kernel, dim3(egrid), dim3(kThreads), 0, stream,
+                               (const double *)G, (const double *)S, stats, m, ebound, E, lam));
         IPTGB_CHECK((gemm({cur, E, cur, nxt, 0, 0, nullptr, nullptr}, {}, 1)));  // Z <- Z + Z E
         return IPT_CUDA_SUCCESS;
     };
