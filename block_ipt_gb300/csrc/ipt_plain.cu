@@ -44,6 +44,12 @@ int DenseFp64Operator::step(const double *X, double *Xn, const double *d, int wa
     return product.step(X, g.ptr, Xn, want_norms, ns);
 }
 
+int DenseFp64Operator::step_ahead(const double *X, double *Xn, const double *d, NormScratch *ns)
+{
+    (void)d;
+    return product.step(X, g.ptr, Xn, 1, ns, nullptr, true);
+}
+
 int DenseFp64Operator::diag_values(const double *X, double *values)
 {
     return launch_dense64_diag_values(H, n, n, X, k, values, stream);
@@ -217,7 +223,7 @@ int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, 
         double *slot = slots + 2 * (launched % kNormSlots);
         arm_slot(reinterpret_cast<volatile uint64_t *>(slot));
         scratch->ns.norms = slot;
-        IPTGB_CHECK(op.step(X[launched & 1], X[(launched + 1) & 1], d, 1, &scratch->ns));
+        IPTGB_CHECK(op.step_ahead(X[launched & 1], X[(launched + 1) & 1], d, &scratch->ns));
         ++launched;
         return IPT_CUDA_SUCCESS;
     };
@@ -230,6 +236,7 @@ int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, 
             status = launch();
         }
         const double *slot = slots + 2 * (done % kNormSlots);
+        if (status == IPT_CUDA_SUCCESS && launched == done + 1) status = op.flush_norms();
         if (status == IPT_CUDA_SUCCESS) {
             status = wait_slot(reinterpret_cast<const volatile uint64_t *>(slot), stream);
         }
@@ -249,9 +256,12 @@ int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, 
     if (status != IPT_CUDA_SUCCESS) {
         cudaStreamSynchronize(stream);
     } else if (launched > done) {
-        status = wait_slot(reinterpret_cast<const volatile uint64_t *>(
-                               slots + 2 * ((launched - 1) % kNormSlots)),
-                           stream);
+        status = op.flush_norms();
+        if (status == IPT_CUDA_SUCCESS) {
+            status = wait_slot(reinterpret_cast<const volatile uint64_t *>(
+                                   slots + 2 * ((launched - 1) % kNormSlots)),
+                               stream);
+        }
     }
     scratch->ns.norms = device_norms;
     IPTGB_CHECK(status);

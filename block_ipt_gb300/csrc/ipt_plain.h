@@ -18,6 +18,13 @@ struct Fp64Operator {
     // Xn = F(X); with want_norms the step leaves ||Xn - X||_F, ||X||_F in ns->norms.
     virtual int step(const double *X, double *Xn, const double *d, int want_norms,
                      NormScratch *ns) = 0;
+    // The same, where the norms may reach ns->norms only with the next step or
+    // with flush_norms().
+    virtual int step_ahead(const double *X, double *Xn, const double *d, NormScratch *ns)
+    {
+        return step(X, Xn, d, 1, ns);
+    }
+    virtual int flush_norms() { return IPT_CUDA_SUCCESS; }
     // values[j] = (H X)_jj.
     virtual int diag_values(const double *X, double *values) = 0;
 };
@@ -43,6 +50,8 @@ struct DenseFp64Operator final : Fp64Operator {
     int start(const double *X, int k, const double *d) override;
     int step(const double *X, double *Xn, const double *d, int want_norms,
              NormScratch *ns) override;
+    int step_ahead(const double *X, double *Xn, const double *d, NormScratch *ns) override;
+    int flush_norms() override { return product.flush_norms(); }
     int diag_values(const double *X, double *values) override;
 };
 

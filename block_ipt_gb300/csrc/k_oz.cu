@@ -787,14 +787,49 @@ __global__ void oz_colmax_kernel(const double *__restrict__ X, long long ldx, in
 // c >= C.  Grid (padded column, K chunk); colexp[c] records the column's
 // exponent; colmax_next (may be null) is cleared for the pass that writes
 // the next block.
+//
+// With norms.count > 0 an extra block (x = the number of padded columns)
+// finishes the norms of the update before, whose blocks only left their parts:
+// finished there, by the block with the last ticket, they held up the next
+// step by 3 us.
+struct PendingNorms {
+    const double2 *parts;
+    int count;
+    double *out;
+};
+
+__device__ __forceinline__ void finish_norms(const PendingNorms &p)
+{
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < p.count; i += blockDim.x) {
+        const double2 v = p.parts[i];
+        a += v.x;
+        b += v.y;
+    }
+    write_norms2(block_sum2(a, b), p.out);
+}
+
+// The same where no next step follows.
+__global__ void __launch_bounds__(256) oz_norms_kernel(PendingNorms norms)
+{
+    pdl_wait();
+    pdl_trigger();
+    finish_norms(norms);
+}
+
 template <int S>
-__global__ void oz_slice_x_kernel(const double *__restrict__ X, long long ldx, int n, int C,
-                                  int cp, int ldp, const unsigned long long *__restrict__ colmax,
-                                  unsigned long long *__restrict__ colmax_next,
-                                  __half *__restrict__ B, int *__restrict__ colexp)
+__global__ void __launch_bounds__(256)
+oz_slice_x_kernel(const double *__restrict__ X, long long ldx, int n, int C, int cp, int ldp,
+                  const unsigned long long *__restrict__ colmax,
+                  unsigned long long *__restrict__ colmax_next, __half *__restrict__ B,
+                  int *__restrict__ colexp, PendingNorms norms)
 {
     pdl_wait();
     const int c = blockIdx.x;
+    if (norms.count > 0 && c == (int)gridDim.x - 1) {
+        if (blockIdx.y == 0) finish_norms(norms);
+        return;
+    }
     const int e = c < C ? oz_exponent(colmax[c]) : 0;
     if (blockIdx.y == 0 && threadIdx.x == 0 && c < C) {
         colexp[c] = e;
@@ -919,13 +954,13 @@ oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
 // n = 8192, k = 32: 13 us per step together with the digit pass of X.
 constexpr int kUpdateThreads = 256;
 
-template <int R>
+template <int R, bool RESID>
 __global__ void __launch_bounds__(kUpdateThreads + 32)
 oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ H,
                  const double *__restrict__ d, const double *__restrict__ g,
                  const double *__restrict__ X, double *__restrict__ Xn,
                  unsigned long long *__restrict__ colmax_next, int row_blocks, int want_norms,
-                 double2 *partials, unsigned int *counter, double *norms,
+                 int defer_norms, double2 *partials, unsigned int *counter, double *norms,
                  double *__restrict__ resid_part)
 {
     constexpr int kRows = kUpdateThreads * R;
@@ -972,13 +1007,13 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     const bool failed = *p.err != 0;
     double dsq = 0.0, xsq = 0.0, rsq = 0.0;
     unsigned long long m = 0;
-    const double hcc = resid_part != nullptr ? fma(d[c], xc[c], cj) : 0.0;  // (H X)_cc
+    const double hcc = RESID ? fma(d[c], xc[c], cj) : 0.0;  // (H X)_cc
     if (t < kUpdateThreads) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int i = row0 + q * kUpdateThreads + t;
             if (i < n) {
-                if (resid_part != nullptr) {
+                if (RESID) {
                     const double r = fma(x[q], d[i] - hcc, y[q]);
                     rsq = fma(r, r, rsq);
                 }
@@ -997,11 +1032,17 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     }
     m = warp_max(m);
     if ((t & 31) == 0 && m != 0) atomicMax(colmax_next + c, m);
-    if (resid_part != nullptr) {
+    if (RESID) {
         const double2 r = block_sum2(rsq, 0.0);
         if (t == 0) resid_part[blockIdx.x] = r.x;
     }
-    if (want_norms) grid_finish_norms2(block_sum2(dsq, xsq), partials, counter, norms);
+    if (!want_norms) return;
+    const double2 sq = block_sum2(dsq, xsq);
+    if (!defer_norms) {
+        grid_finish_norms2(sq, partials, counter, norms);
+    } else if (t == 0) {
+        partials[blockIdx.x] = sq;
+    }
 }
 
 __global__ void gap_reciprocals_kernel(const double *__restrict__ d, int n, int k,
@@ -1015,20 +1056,21 @@ __global__ void gap_reciprocals_kernel(const double *__restrict__ d, int n, int 
 }
 
 // Row maxima of |H_il| (l != i) of a column-major H, as bit patterns, and its
-// diagonal: 256 rows x kScanCols columns per block, two neighbouring rows per
+// diagonal: 256 rows x `cols` columns per block, two neighbouring rows per
 // thread (16-byte loads when n is even and H aligned), eight columns in flight.
 constexpr int kScanThreads = 128;
-constexpr int kScanCols = 64;
+constexpr int kScanCols = 64;     // columns of a block, fewer (a multiple of 8)
+constexpr int kScanMinCols = 8;  // while the grid is small: n = 1024 16.7 -> 7.4 us
 
 template <bool VEC>
 __global__ void __launch_bounds__(kScanThreads)
-oz_rowmax_kernel(const double *__restrict__ H, int n, unsigned long long *__restrict__ rowmax,
-                 double *__restrict__ diag)
+oz_rowmax_kernel(const double *__restrict__ H, int n, int cols,
+                 unsigned long long *__restrict__ rowmax, double *__restrict__ diag)
 {
     const int i = (blockIdx.y * kScanThreads + threadIdx.x) * 2;
     if (i >= n) return;
-    const int l0 = blockIdx.x * kScanCols;
-    const int l1 = min(n, l0 + kScanCols);
+    const int l0 = blockIdx.x * cols;
+    const int l1 = min(n, l0 + cols);
     unsigned long long m0 = 0, m1 = 0;
     for (int l = l0; l < l1; l += 8) {
         double v0[8], v1[8];
@@ -1156,10 +1198,16 @@ int OzMatrix::scan_rows(const double *H_, int n_, double *diag, cudaStream_t s)
     IPTGB_CHECK(rm.alloc((size_t)n, s));
     IPTGB_CUDA(cudaMemsetAsync(rm.ptr, 0, (size_t)n * sizeof(unsigned long long), s));
     const int rows = 2 * oz::kScanThreads;
-    const dim3 grid((n + oz::kScanCols - 1) / oz::kScanCols, (n + rows - 1) / rows);
+    const int row_blocks = (n + rows - 1) / rows;
+    int cols = oz::kScanCols;
+    const int enough = 3 * device_sm_count();
+    while (cols > oz::kScanMinCols && (long long)((n + cols - 1) / cols) * row_blocks < enough) {
+        cols /= 2;
+    }
+    const dim3 grid((n + cols - 1) / cols, row_blocks);
     const bool vec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(H) & 15) == 0;
     auto scan = vec ? oz::oz_rowmax_kernel<true> : oz::oz_rowmax_kernel<false>;
-    scan<<<grid, oz::kScanThreads, 0, s>>>(H, n, rm.ptr, diag);
+    scan<<<grid, oz::kScanThreads, 0, s>>>(H, n, cols, rm.ptr, diag);
     IPTGB_LAUNCH();
     oz::oz_rowexp_kernel<<<blocks_for((size_t)n), kThreads, 0, s>>>(rm.ptr, n, rowexp.ptr);
     IPTGB_LAUNCH();
@@ -1299,10 +1347,13 @@ int OzProduct::slice_and_multiply(const double *X, long long ldx, int clear_othe
     const int pc = q.groups * q.cp;
     const int ychunks = std::max(1, std::min((q.ldp + 1023) / 1024, (8 * sms + pc - 1) / pc));
     auto slice = slices == 7 ? oz::oz_slice_x_kernel<7> : oz::oz_slice_x_kernel<6>;
-    IPTGB_CHECK(launch_pdl(slice, dim3(pc, ychunks), dim3(256), 0, s, X, ldx, q.n, q.C, q.cp,
-                           q.ldp, (const unsigned long long *)(colmax.ptr + cur * set),
+    const oz::PendingNorms norms = {pending_parts, pending_count, pending_out};
+    IPTGB_CHECK(launch_pdl(slice, dim3(pc + (pending_count > 0 ? 1 : 0), ychunks), dim3(256), 0, s,
+                           X, ldx, q.n, q.C, q.cp, q.ldp,
+                           (const unsigned long long *)(colmax.ptr + cur * set),
                            clear_other ? colmax.ptr + (1 - cur) * set : nullptr, B.ptr,
-                           colexp.ptr));
+                           colexp.ptr, norms));
+    pending_count = 0;
     oz::Params prm = {};
     prm.H = m->H;
     prm.words = m->words.ptr;
@@ -1375,8 +1426,16 @@ int OzProduct::update_row_blocks(int n, int C, int sms, bool *wide)
     return *wide ? (r1 + 3) / 4 : r1;
 }
 
+int OzProduct::flush_norms()
+{
+    if (pending_count == 0) return IPT_CUDA_SUCCESS;
+    const oz::PendingNorms norms = {pending_parts, pending_count, pending_out};
+    pending_count = 0;
+    return launch_pdl(oz::oz_norms_kernel, dim3(1), dim3(256), 0, s, norms);
+}
+
 int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns,
-                    double *resid_part)
+                    double *resid_part, bool defer_norms)
 {
     bool wide = false;
     const int row_blocks = update_row_blocks(sh.n, sh.C, sms, &wide);
@@ -1388,9 +1447,19 @@ int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms
         IPTGB_CHECK(slice_and_multiply(X, sh.n, 1));
     }
     KernelTimerScope timer(kProfFp64Update, s);
-    IPTGB_CHECK(launch_pdl(wide ? oz::oz_update_kernel<4> : oz::oz_update_kernel<1>,
-                           dim3((unsigned)grid), dim3(oz::kUpdateThreads + 32), 0, s, partials(), m->H, d, g, X, Xn, colmax.ptr + (1 - cur) * set, row_blocks,
-                           want_norms, ns->partials, ns->counter, ns->norms, resid_part));
+    auto update = resid_part == nullptr
+                      ? (wide ? oz::oz_update_kernel<4, false> : oz::oz_update_kernel<1, false>)
+                      : (wide ? oz::oz_update_kernel<4, true> : oz::oz_update_kernel<1, true>);
+    IPTGB_CHECK(launch_pdl(update,
+                           dim3((unsigned)grid), dim3(oz::kUpdateThreads + 32), 0, s, partials(),
+                           m->H, d, g, X, Xn, colmax.ptr + (1 - cur) * set, row_blocks,
+                           want_norms, defer_norms ? 1 : 0, ns->partials, ns->counter, ns->norms,
+                           resid_part));
+    if (want_norms && defer_norms) {
+        pending_parts = ns->partials;
+        pending_count = (int)grid;
+        pending_out = ns->norms;
+    }
     cur = 1 - cur;
     return IPT_CUDA_SUCCESS;
 }

@@ -66,6 +66,10 @@ struct OzProduct {
     DeviceBuffer<int> colexp;
     DeviceBuffer<unsigned long long> colmax;  // two sets of C column maxima
     int cur = 0;                              // the set the next product reads
+    // deferred norms of the last step: parts, their number (0: none), target
+    const double2 *pending_parts = nullptr;
+    int pending_count = 0;
+    double *pending_out = nullptr;
     DeviceBuffer<double> P;
     DeviceBuffer<int> err;
     CUtensorMap mapB;
@@ -80,8 +84,11 @@ struct OzProduct {
     int begin(const double *X, int C);
     // resid_part (optional): update_row_blocks parts per column of
     // ||(H X)_c - X_c (H X)_cc||^2.
+    // defer_norms: the norms reach ns->norms with the next step, or with
+    // flush_norms() where none follows.
     int step(const double *X, const double *g, double *Xn, int want_norms, NormScratch *ns,
-             double *resid_part = nullptr);
+             double *resid_part = nullptr, bool defer_norms = false);
+    int flush_norms();
     static int update_row_blocks(int n, int C, int sms, bool *wide);
     // the column maxima (bit patterns) the next step reads
     unsigned long long *column_maxima() { return colmax.ptr + (size_t)cur * sh.groups * sh.cp; }

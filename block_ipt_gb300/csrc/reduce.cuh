@@ -91,6 +91,16 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// out[0] = sqrt(t.x), out[1] = sqrt(t.y) of a t valid in thread 0, by one warp
+// (one square root's instructions for both).  Called by the whole block.
+__device__ __forceinline__ void write_norms2(double2 t, double *out)
+{
+    if (threadIdx.x >= 32) return;
+    const double y = __shfl_sync(0xffffffffu, t.y, 0);
+    const double v = sqrt(threadIdx.x == 0 ? t.x : y);
+    if (threadIdx.x < 2) out[threadIdx.x] = v;
+}
+
 // Deterministic grid-wide finish of per-block (a, b) sums.  `mine` must be
 // valid in thread 0.  The last block writes out[0] = sqrt(sum a) and
 // out[1] = sqrt(sum b) and re-arms *counter for the next launch.
@@ -115,12 +125,8 @@ __device__ __forceinline__ void grid_finish_norms2(double2 mine, double2 *partia
         a += p.x;
         b += p.y;
     }
-    const double2 t = block_sum2(a, b);
-    if (threadIdx.x == 0) {
-        out[0] = sqrt(t.x);
-        out[1] = sqrt(t.y);
-        *counter = 0u;
-    }
+    write_norms2(block_sum2(a, b), out);
+    if (threadIdx.x == 0) *counter = 0u;
 }
 
 }  // namespace iptgb
