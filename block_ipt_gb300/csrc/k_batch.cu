@@ -41,7 +41,10 @@
 // barrier, every CTA adds the cluster's sums in rank order from distributed
 // shared memory, so all of them take the same (bitwise identical) decisions.
 // Once the counter passes the team instances, every CTA takes the remaining
-// instances on its own.  Without the split, one CTA of ~2 FP64 FMAs per clock
+// instances on its own.  The cluster size and the fraction are those of the
+// shortest estimated schedule where it beats the largest clusters at 25 % by 5
+// %: for 256 instances up to n = 2048 with FP32 sweeps four CTAs and 10 %, 9.6
+// -> 7.7 ms; 200 up to 1500 in FP64 eight and 10 %, 34.4 -> 33.2.  Without the split, one CTA of ~2 FP64 FMAs per clock
 // holds an n = 2048, k = 16 instance for ~100 ms and sets the makespan.
 //
 // Within a CTA, a thread owns one row and all k columns of Y, k padded to a
@@ -54,7 +57,9 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <type_traits>
 #include <vector>
 
@@ -722,11 +727,16 @@ inline size_t batch_floats(int n, int k)
     return 2 * (size_t)n * kp + (((2 * (size_t)n * k + (size_t)n * n) + 3) & ~(size_t)3);
 }
 
+// Instances up to which launch shapes are compared by estimate (25 schedules of
+// the whole batch, 20 ms at this count; larger batches balance by themselves).
+constexpr int kMaxEstimated = 16384;
+
 struct BatchPlan {
     int count = 0;
     std::vector<batch::Inst> host_inst;
     std::vector<double> cost;  // n^2 k of order[q]
     std::vector<int> order_n;  // n of order[q]
+    std::vector<int> order_k;  // k of order[q]
     batch::Inst *inst = nullptr;
     int *order = nullptr;
     int *counter = nullptr;
@@ -742,8 +752,9 @@ struct BatchPlan {
     int threads = 512;
     int chunk = 128;
     // instances above team_pct % of the average load of one CTA go to a
-    // whole cluster (0: every instance on one CTA)
-    int team_pct = 25;
+    // whole cluster (0: every instance on one CTA; < 0: cluster size and
+    // threshold of the shortest estimated schedule)
+    int team_pct = -1;
     int cluster = 1;  // cluster size of the launch
     int n_team = 0;
     int ctas = 0;
@@ -768,55 +779,109 @@ struct BatchPlan {
         cluster = 1;
         ctas = std::min(count, full);
         n_team = 0;
-        if (team_pct <= 0) return IPT_CUDA_SUCCESS;
-        // the largest cluster size that keeps nearly every CTA slot of the
-        // device busy (clusters are placed within one GPC)
+        if (team_pct == 0) return IPT_CUDA_SUCCESS;
         const int forced = env_int("IPT_GB300_BATCH_CLUSTER", 0);
-        const int sizes[3] = {8, 4, 2};
-        for (int c : sizes) {
-            if (forced > 0 && c != forced) continue;
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)(full / c * c));
-            cfg.blockDim = dim3((unsigned)threads);
-            cfg.dynamicSmemBytes = chunk == 64 ? sizeof(batch::Shared<64>)
-                                               : sizeof(batch::Shared<128>);
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = (unsigned)c;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            cudaError_t e;
-            if (chunk == 64) {
-                e = cudaOccupancyMaxActiveClusters(&clusters, batch::batch_ipt_kernel<64>, &cfg);
-            } else {
-                e = cudaOccupancyMaxActiveClusters(&clusters, batch::batch_ipt_kernel<128>, &cfg);
-            }
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                continue;
-            }
-            if (clusters * c >= (forced > 0 ? 1 : (9 * full) / 10)) {
-                cluster = c;
-                ctas = clusters * c;
-                break;
-            }
-        }
-        if (cluster == 1) return IPT_CUDA_SUCCESS;
         double total = 0.0;
         for (double c : cost) total += c;
-        const double thr = (double)team_pct / 100.0 * total / ctas;
-        while (n_team < count && cost[(size_t)n_team] > thr &&
-               order_n[(size_t)n_team] >= 32 * cluster) {
-            ++n_team;
-        }
-        if (n_team == 0) {
-            cluster = 1;
-            ctas = std::min(count, full);
+        // a fixed threshold (25 unless set) on the largest cluster size; without
+        // a set one, another size or threshold where the estimated schedule is
+        // clearly shorter (the estimate is good to about 5 %)
+        const int base_pct = team_pct > 0 ? team_pct : 25;
+        const bool fixed = team_pct > 0 || count > kMaxEstimated;
+        double base = -1.0, best = INFINITY;
+        for (int c : {8, 4, 2}) {
+            if (forced > 0 && c != forced) continue;
+            int clusters = 0;
+            if (!max_clusters(c, full / c * c, &clusters)) continue;
+            // the sizes that keep nearly every CTA slot of the device busy
+            // (clusters are placed within one GPC)
+            if (clusters * c < (forced > 0 ? 1 : (9 * full) / 10)) continue;
+            for (int pct : {base_pct, 5, 10, 15, 40, 60, 100, 150}) {
+                const double thr = (double)pct / 100.0 * total / (clusters * c);
+                int teams = 0;
+                while (teams < count && cost[(size_t)teams] > thr &&
+                       order_n[(size_t)teams] >= 32 * c) {
+                    ++teams;
+                }
+                const int size = teams > 0 ? c : 1;
+                const int slots = teams > 0 ? clusters * c : std::min(count, full);
+                const double t = fixed ? 0.0 : makespan(size, slots, teams);
+                const bool first = base < 0.0;
+                if (first) base = t;
+                if (first || (t < 0.95 * base && t < best)) {
+                    if (!first) best = t;
+                    cluster = size;
+                    ctas = slots;
+                    n_team = teams;
+                }
+                if (fixed) return IPT_CUDA_SUCCESS;
+            }
         }
         return IPT_CUDA_SUCCESS;
+    }
+
+    bool max_clusters(int c, int grid, int *clusters)
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = chunk == 64 ? sizeof(batch::Shared<64>)
+                                           : sizeof(batch::Shared<128>);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)c;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e =
+            chunk == 64
+                ? cudaOccupancyMaxActiveClusters(clusters, batch::batch_ipt_kernel<64>, &cfg)
+                : cudaOccupancyMaxActiveClusters(clusters, batch::batch_ipt_kernel<128>, &cfg);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return true;
+    }
+
+    // Estimated time of instance order[q] on `team` CTAs, in columns of H of one
+    // row block: a sweep walks all n columns for each block of `threads` rows,
+    // at the loads' latency however few the rows (1 per block), plus the
+    // arithmetic of its rows and KP columns, for 256 rows and KP = 16 four
+    // times that with FP32 and double-float sweeps and 33 times on the FP64
+    // pipe; a team also meets at barriers.
+    double estimate(int q, int team) const
+    {
+        const int n = order_n[(size_t)q];
+        const int kp = (order_k[(size_t)q] + 3) & ~3;
+        const int rows = ((n + team - 1) / team + 31) & ~31;
+        const double work = certify_df ? 4.0 : 33.0;
+        return n * ((rows + threads - 1) / threads + work * kp / 16.0 * rows / 256.0) +
+               (team > 1 ? 100.0 : 0.0);
+    }
+
+    // End of the kernel's own schedule: clusters take the team instances in
+    // order, then every CTA takes the next one as it becomes free.
+    double makespan(int team, int slots, int teams) const
+    {
+        std::priority_queue<double, std::vector<double>, std::greater<double>> at;
+        for (int g = 0; g < slots / team; ++g) at.push(0.0);
+        double end = 0.0;
+        auto take = [&](int q, int size) {
+            const double t = at.top() + estimate(q, size);
+            at.pop();
+            at.push(t);
+            end = std::max(end, t);
+        };
+        for (int q = 0; q < teams; ++q) take(q, team);
+        if (team > 1) {
+            std::vector<double> free_at;
+            for (; !at.empty(); at.pop()) free_at.insert(free_at.end(), team, at.top());
+            for (double t : free_at) at.push(t);
+        }
+        for (int q = teams; q < count; ++q) take(q, 1);
+        return end;
     }
 
     int launch(cudaStream_t s)
@@ -940,7 +1005,7 @@ IPT_API int ipt_block_batch_plan_create(const IPTBatchInstance *instances, int c
     P->lowp_tol = opt.lowp_tol;
     P->threads = opt.threads != 0 ? opt.threads : 256;
     P->chunk = opt.chunk != 0 ? opt.chunk : 128;
-    P->team_pct = std::max(0, env_int("IPT_GB300_BATCH_TEAM_PCT", 25));
+    P->team_pct = env_int("IPT_GB300_BATCH_TEAM_PCT", -1);
     int st = IPT_CUDA_SUCCESS;
     if (cudaMalloc((void **)&P->pool, pool * sizeof(double)) != cudaSuccess ||
         (pool32 > 0 && cudaMalloc((void **)&P->pool32, pool32 * sizeof(float)) != cudaSuccess) ||
@@ -991,9 +1056,11 @@ IPT_API int ipt_block_batch_plan_create(const IPTBatchInstance *instances, int c
                          [&](int a, int b) { return cost_of(a) > cost_of(b); });
         P->cost.resize(count);
         P->order_n.resize(count);
+        P->order_k.resize(count);
         for (int q = 0; q < count; ++q) {
             P->cost[(size_t)q] = cost_of(order[(size_t)q]);
             P->order_n[(size_t)q] = instances[order[(size_t)q]].n;
+            P->order_k[(size_t)q] = instances[order[(size_t)q]].k;
         }
         if (cudaMemcpy(P->inst, P->host_inst.data(), count * sizeof(batch::Inst),
                        cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -1035,13 +1102,13 @@ IPT_API int ipt_block_batch_plan_autotune(void *plan, void *stream, int *threads
     IPTGB_CUDA(cudaEventCreate(&e1));
     const int cand_threads[3] = {128, 256, 512};
     const int cand_chunk[2] = {64, 128};
-    const int cand_team[3] = {0, 25, 100};
+    const int cand_team[4] = {-1, 0, 25, 100};
     double best = INFINITY;
     int bt = P->threads, bc = P->chunk, bp = P->team_pct;
     int st = P->launch(s);  // warm-up
     for (int ti = 0; ti < 3 && st == IPT_CUDA_SUCCESS; ++ti) {
         for (int ci = 0; ci < 2 && st == IPT_CUDA_SUCCESS; ++ci) {
-            for (int pi = 0; pi < 3 && st == IPT_CUDA_SUCCESS; ++pi) {
+            for (int pi = 0; pi < 4 && st == IPT_CUDA_SUCCESS; ++pi) {
                 P->threads = cand_threads[ti];
                 P->chunk = cand_chunk[ci];
                 P->team_pct = cand_team[pi];

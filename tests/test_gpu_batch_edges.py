@@ -35,3 +35,36 @@ def test_batch_column_pairs_and_row_edges(cuda, precision, threads):
         assert r.max() <= 1e-8 * max(1.0, hn)
         assert np.abs(np.sort(v) - np.linalg.eigvalsh(H)[:k]).max() <= 1e-10 * hn
     plan.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_batch_estimated_launch_shape_matches_single_cta(cuda, monkeypatch, precision):
+    """The launch shape picked by the estimated schedule gives the blocks and
+    sweep counts of one CTA per instance."""
+    torch = cuda
+    rng = np.random.default_rng(3)
+    specs = [(int(rng.integers(64, 420)), int(rng.integers(1, 17))) for _ in range(90)]
+    results = {}
+    for pct in (None, "0"):
+        if pct is None:
+            monkeypatch.delenv("IPT_GB300_BATCH_TEAM_PCT", raising=False)
+        else:
+            monkeypatch.setenv("IPT_GB300_BATCH_TEAM_PCT", pct)
+        keep, inst = [], []
+        for s, (n, k) in enumerate(specs):
+            H, _ = workloads.batch_instance(n, 0.05, 400 + s)
+            dH = torch.from_numpy(np.asfortranarray(H).T.copy()).cuda()
+            dX = torch.zeros((k, n), dtype=torch.float64, device="cuda")
+            dv = torch.zeros(k, dtype=torch.float64, device="cuda")
+            keep.append((dH, dX, dv))
+            inst.append((dH.data_ptr(), n, k, dX.data_ptr(), dv.data_ptr()))
+        plan = api.BatchPlan(inst, precision)
+        assert plan.shape()["cluster"] in ((1, 2, 4, 8) if pct is None else (1,))
+        plan.run()
+        torch.cuda.synchronize()
+        results[pct] = [(dX.cpu().numpy(), rep["iterations"], rep["converged"])
+                        for (_, dX, _), rep in zip(keep, plan.reports())]
+        plan.close()
+    for (Xa, ia, ca), (Xb, ib, cb) in zip(results[None], results["0"]):
+        assert ca == 1 and cb == 1 and ia == ib
+        assert np.abs(Xa - Xb).max() <= 1e-12
