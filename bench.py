@@ -61,9 +61,8 @@ NCU_TRAFFIC = {("dense64_partial", 8192, 32, "fp16"): 567.5e6,
                ("tc_stream", 8192, "default"): 95.7e6,
                ("tc_stream", 8192, "0"): 141.9e6,
                ("tc_stream", 16384, "default"): 554.4e6,
-               # one cold launch at n = 8192, 32 columns
-               # (profiles/oz_product_n4096_n8192_c32.md)
-               ("oz_product", 8192, 32, "fp16"): 811.5e6}
+               # a launch inside the solve (profiles/oz_product_digit_words.md)
+               ("oz_product", 8192, 32, "fp16"): 537.8e6}
 
 
 def parse():
@@ -980,19 +979,21 @@ def run_ours(args):
                      "avg_launch_ms": lp_ms / max(1, lp_cnt),
                      "algorithmic_bytes_per_launch": lp_bytes,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"}
-    # the FP64-accurate products of the refinement (k columns each): six FP16
-    # digit slices of Delta streamed once per product, the X slices written
-    # and read, X read and H X written (k_oz.cu); bound: HBM.  Its timer spans
+    # the FP64-accurate products of the refinement (k columns each): the digit
+    # words of Delta (8 bytes an entry) streamed once per product, the six FP16
+    # X slices written and read, X read and H X written (k_oz.cu); measured
+    # against HBM (the expansion of the words in shared memory comes before it).  Its timer spans
     # the X split, the tensor-core product and the finish kernel.
     fp_ms, fp_cnt = prof["fp64_product"]
     cp = (k + 15) // 16 * 16
-    acc_bytes = 12 * n * ldp + 24 * cp * ldp + 16 * n * k
+    acc_bytes = (8 * ((n + 127) // 128 * 128) * ((n + 31) // 32 * 32) + 24 * cp * ldp
+                 + 16 * n * k)
     acc_ach = acc_bytes / (fp_ms / max(1, fp_cnt) * 1e-3) / 1e9 if fp_cnt else None
     # MMA work: slice s times B rows (6 - s) cp, over every (row, K) pair
     mma_flops = 2.0 * ((n + 127) // 128 * 128) * ldp * sum((6 - s) * cp for s in range(6))
     roofline_accurate = {
-        "kernel": "oz_product_kernel (FP64-accurate product: 6+6 FP16 digit slices, tcgen05 "
-                  "+ TMA, persistent)",
+        "kernel": "oz_product_kernel (FP64-accurate product: 6+6 FP16 digits from packed words, "
+                  "tcgen05 + TMA, persistent)",
         "bound": "hbm", "achieved": acc_ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": (acc_ach / peaks["hbm_gbs"]) if acc_ach else None,
         "traffic": NCU_TRAFFIC.get(("oz_product", n, k, args.precision)),

@@ -1,8 +1,11 @@
-// k_dense64.cu - FP64 kernels of the plain dense IPT path.
+// k_dense64.cu - split-K SIMT block product and update in FP64 and FP32.
 //
-// The per-iteration block product Y = H X (reference: cublasDgemm in
-// IPT_C_GPU/src/ipt_cuda.cu:1649,1888) is written for GB300's FP64 pipe,
-// which retires ~1.2 TFLOP/s: a split-K SIMT kernel keeps every SM's DFMA
+// The block product Y = H X (reference: cublasDgemm in
+// IPT_C_GPU/src/ipt_cuda.cu:1649,1888) of the allocation-free entry, of the
+// block solver's dense solves that ask for FP64 FMAs, and of the FP32 stage of
+// the mixed ACX; the plain path multiplies on the tensor cores (k_oz.cu).
+// Written for GB300's FP64 pipe, which retires ~1.2 TFLOP/s: a split-K SIMT
+// kernel keeps every SM's DFMA
 // pipe busy (the skinny N = k product has too few output tiles otherwise),
 // writes per-slice partial blocks, and a second kernel sums the partials in a
 // fixed order and applies the IPT update (reference kernels

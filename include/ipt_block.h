@@ -33,7 +33,8 @@ extern "C" {
 
 /* Precision of the IPT stage's block product Delta X. */
 enum {
-    IPT_BLOCK_FP64 = 0, /* FP64 SIMT product (the plain path) */
+    IPT_BLOCK_FP64 = 0, /* FP64-accurate product on the FP16 tensor cores (dense),
+                           FP64 or double-float gather (CSR) */
     IPT_BLOCK_FP16 = 1, /* FP16 tensor cores (tcgen05), FP32 accumulation */
     IPT_BLOCK_BF16 = 2, /* BF16 tensor cores (tcgen05), FP32 accumulation */
     IPT_BLOCK_TF32 = 3, /* TF32 tensor cores (tcgen05), FP32 accumulation */
@@ -473,8 +474,9 @@ int ipt_block_split_double_host(const double *in, long long count, float *hi, fl
  * Numer. Algorithms 59 (2012); the fixed-point form of Mukunoki et al., ISC
  * 2020).  The error of an entry is below about 2^-46 times
  * max_l |H_il| max_l |X_lc| times the number of terms, plus the rounding of
- * |H_ii X_ic|.  The solver splits H once per solve; this entry splits it on
- * every call (for checking and one-off products).  Runs on `stream`
+ * |H_ii X_ic|.  The solver lays the digits out once per solve; this entry
+ * extracts them from H while it multiplies (for one-off products).  Runs on
+ * `stream`
  * (cudaStream_t, NULL = legacy default stream) and synchronises it. */
 int ipt_block_accurate_product(const double *d_H, int n, const double *d_X, int c,
                                double *d_Y, void *stream);
