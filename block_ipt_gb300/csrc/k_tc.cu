@@ -1419,9 +1419,42 @@ __device__ __forceinline__ void hist_add(double *hist, int step, double2 t)
     }
 }
 
+// The sums over a product's partial slots of one row and of the column's
+// diagonal row, in slot order; the first kSlotsUnrolled slots' loads are in
+// flight together.
+constexpr int kSlotsUnrolled = 8;
+
+__device__ __forceinline__ void sum_slots1(const float *__restrict__ P, int S, int p, int n,
+                                           int col, int row, float &y, float &c)
+{
+    float v[kSlotsUnrolled], d[kSlotsUnrolled];
+#pragma unroll
+    for (int s = 0; s < kSlotsUnrolled; ++s) {
+        if (s < S) {
+            const float *base = P + ((size_t)s * p + col) * (size_t)n;
+            v[s] = base[row];
+            d[s] = base[col];
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < kSlotsUnrolled; ++s) {
+        if (s < S) {
+            y += v[s];
+            c += d[s];
+        }
+    }
+    for (int s = kSlotsUnrolled; s < S; ++s) {
+        const float *base = P + ((size_t)s * p + col) * (size_t)n;
+        y += base[row];
+        c += base[col];
+    }
+}
+
 // Low-precision IPT update (see file header); Delta has a zero diagonal so
 // c_j = (Delta X)_jj is read straight from the product.
-template <typename LP>
+// Index: 32 bits below 2^31 entries.  n = 3001, 21 columns: 12.6 -> 6.3 us with
+// that and the slots' loads together.
+template <typename LP, typename Index>
 __global__ void lowp_update_kernel(const float *__restrict__ P, int S, int n, int p,
                                    float inv_scale, const float *__restrict__ inv_row,
                                    const float *__restrict__ G,
@@ -1433,33 +1466,28 @@ __global__ void lowp_update_kernel(const float *__restrict__ P, int S, int n, in
     pdl_wait();  // P and X come from the previous grids
     pdl_trigger();
     // grid-stride over the block (a few CTAs per SM)
-    const size_t elems = (size_t)n * (size_t)p;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const Index elems = (Index)n * (Index)p;
+    const Index stride = (Index)gridDim.x * blockDim.x;
     if (hist_stopped(hist, step, stop_tol)) {
         // stopped: pass the block through to the next buffer pair
-        for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < elems;
-             idx += stride) {
+        for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
             const float x = X[idx];
             Xn[idx] = x;
-            Xlp[(idx % (size_t)n) + (idx / (size_t)n) * (size_t)ldx] = to_lp<LP>(x);
+            Xlp[(idx % (Index)n) + (size_t)(idx / (Index)n) * ldx] = to_lp<LP>(x);
         }
         hist_carry(hist, step);
         return;
     }
     want_norms = want_norms || hist != nullptr;
     double dsq = 0.0, xsq = 0.0;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
-        const int row = (int)(idx % (size_t)n);
-        const int col = (int)(idx / (size_t)n);
+    for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
+        const int col = (int)(idx / (Index)n);
+        const int row = (int)(idx - (Index)col * (Index)n);
         const float x = X[idx];
         float out = 1.0f;
         if (row != col) {
             float y = 0.0f, c = 0.0f;
-            for (int s = 0; s < S; ++s) {
-                const size_t base = ((size_t)s * p + col) * (size_t)n;
-                y += P[base + row];
-                c += P[base + col];
-            }
+            sum_slots1(P, S, p, n, col, row, y, c);
             const float ir = inv_row != nullptr ? inv_row[row] : inv_scale;
             const float ic = inv_row != nullptr ? inv_row[col] : inv_scale;
             out = (y * ir - x * (c * ic)) * G[idx];
@@ -1535,7 +1563,6 @@ __device__ __forceinline__ float &f4_at(float4 &v, int i)
 // column col, and of the diagonal entry (col, col), in slot order: the loads
 // of up to kSlotsUnrolled slots are issued together (the update is bound by
 // their latency, not by bandwidth), the adds keep the fixed order.
-constexpr int kSlotsUnrolled = 8;
 
 __device__ __forceinline__ void sum_slots4(const float *__restrict__ P, int S, int p, int n,
                                            int col, int row0, float4 &y, float &c)
@@ -1681,7 +1708,7 @@ __global__ void refine_begin_kernel(const double *__restrict__ R0, const double 
     dlp[(size_t)row + (size_t)col * ldx] = to_lp<LP>(r * sg);
 }
 
-template <typename LP>
+template <typename LP, typename Index>
 __global__ void refine_update_kernel(const float *__restrict__ P, int S, int n, int p,
                                      float inv_scale, const float *__restrict__ inv_row,
                                      const float *__restrict__ sig,
@@ -1694,34 +1721,29 @@ __global__ void refine_update_kernel(const float *__restrict__ P, int S, int n, 
 {
     pdl_wait();  // P and X come from the previous grids
     pdl_trigger();
-    const size_t elems = (size_t)n * (size_t)p;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    const Index elems = (Index)n * (Index)p;
+    const Index stride = (Index)gridDim.x * blockDim.x;
     if (hist_stopped(hist, step, stop_tol)) {
         // stopped: pass the correction through to the next buffer pair
-        for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < elems;
-             idx += stride) {
+        for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
             const float cur = dcur[idx];
-            const int col = (int)(idx / (size_t)n);
+            const int col = (int)(idx / (Index)n);
             dnext[idx] = cur;
-            dlp[(idx % (size_t)n) + (size_t)col * (size_t)ldx] = to_lp<LP>(cur * sig[col]);
+            dlp[(idx % (Index)n) + (size_t)col * ldx] = to_lp<LP>(cur * sig[col]);
         }
         hist_carry(hist, step);
         return;
     }
     want_norms = want_norms || hist != nullptr;
     double dsq = 0.0, xsq = 0.0;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
-        const int row = (int)(idx % (size_t)n);
-        const int col = (int)(idx / (size_t)n);
+    for (Index idx = (Index)blockIdx.x * blockDim.x + threadIdx.x; idx < elems; idx += stride) {
+        const int col = (int)(idx / (Index)n);
+        const int row = (int)(idx - (Index)col * (Index)n);
         const float cur = dcur[idx];
         float out = 0.0f;
         if (row != col) {
             float y = 0.0f, b = 0.0f;
-            for (int s = 0; s < S; ++s) {
-                const size_t base = ((size_t)s * p + col) * (size_t)n;
-                y += P[base + row];
-                b += P[base + col];
-            }
+            sum_slots1(P, S, p, n, col, row, y, b);
             const float ir = inv_row != nullptr ? inv_row[row] : inv_scale;
             const float ic = inv_row != nullptr ? inv_row[col] : inv_scale;
             y *= ir * sig_inv[col];
@@ -2362,6 +2384,10 @@ struct LowpDense final : LowpDenseOperator {
 
     int product() override { return product_until(nullptr, 0, 0.0); }
 
+    // the one-row updates' indices need 64 bits (whose divisions take longer
+    // than the update's loads)
+    bool wide_index() const { return (size_t)n * p >= (size_t)1 << 31; }
+
     // update grid: grid-stride over the block with a few CTAs per SM (four
     // rows per thread when n % 4 == 0); tuning knob IPT_GB300_UPDATE_CTAS_PER_SM
     int update_grid() const
@@ -2421,7 +2447,9 @@ struct LowpDense final : LowpDenseOperator {
                                        mixed ? Gring[kf].ptr : nullptr,
                                        fused ? mix_part.ptr : nullptr));
             } else {
-                IPTGB_CHECK(launch_pdl(lowp_update_kernel<LP>, dim3(grid), dim3(kThreads), 0, s,
+                auto kernel = wide_index() ? lowp_update_kernel<LP, size_t>
+                                           : lowp_update_kernel<LP, unsigned>;
+                IPTGB_CHECK(launch_pdl(kernel, dim3(grid), dim3(kThreads), 0, s,
                                        (const float *)P.ptr, splits, n, p, (float)(1.0 / scale),
                                        (const float *)inv_rows.ptr, (const float *)G.ptr,
                                        (const float *)X32[cur].ptr, X32[nxt].ptr, Xlp[nxt].ptr,
@@ -2555,7 +2583,9 @@ struct LowpDense final : LowpDenseOperator {
                                        mixed ? Gring[kf].ptr : nullptr,
                                        fused ? mix_part.ptr : nullptr));
             } else {
-                IPTGB_CHECK(launch_pdl(refine_update_kernel<LP>, dim3(grid), dim3(kThreads), 0, s,
+                auto kernel = wide_index() ? refine_update_kernel<LP, size_t>
+                                           : refine_update_kernel<LP, unsigned>;
+                IPTGB_CHECK(launch_pdl(kernel, dim3(grid), dim3(kThreads), 0, s,
                                        (const float *)P.ptr, splits, n, p, (float)(1.0 / scale),
                                        (const float *)inv_rows.ptr,
                                        (const float *)(small.ptr + p),
@@ -2687,7 +2717,7 @@ struct LowpDenseSimtF32 final : LowpDenseOperator {
         if (want_norms && grid > ns->capacity) return IPT_CUDA_INVALID_ARGUMENT;
         const int nxt = cur ^ 1;
         KernelTimerScope timer(kProfLowpUpdate, s);
-        lowp_update_kernel<float><<<grid, kThreads, 0, s>>>(
+        lowp_update_kernel<float, size_t><<<grid, kThreads, 0, s>>>(
             P.ptr, splits, n, p, 1.0f, nullptr, G.ptr, X32[cur].ptr, X32[nxt].ptr, X32[nxt].ptr, n,
             want_norms, ns->partials, ns->counter, ns->norms, hm ? ns->hist : nullptr, ns->step,
             ns->stop_tol);
@@ -2745,7 +2775,7 @@ struct LowpDenseSimtF32 final : LowpDenseOperator {
         if (want_norms && grid > ns->capacity) return IPT_CUDA_INVALID_ARGUMENT;
         const int nxt = cur ^ 1;
         KernelTimerScope timer(kProfLowpUpdate, s);
-        refine_update_kernel<float><<<grid, kThreads, 0, s>>>(
+        refine_update_kernel<float, size_t><<<grid, kThreads, 0, s>>>(
             P.ptr, splits, n, p, 1.0f, nullptr, small.ptr + p, small.ptr + 2 * p, G.ptr, R32.ptr,
             Xref32.ptr, small.ptr, X32[cur].ptr, X32[nxt].ptr, X32[nxt].ptr, n, want_norms,
             ns->partials, ns->counter, ns->norms, hm ? ns->hist : nullptr, ns->step,
