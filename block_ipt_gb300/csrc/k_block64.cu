@@ -22,40 +22,53 @@ namespace iptgb {
 
 // ---------------------------------------------------------------------------
 // Gram-type products C = A^T B (A: n x ma, B: n x mb, column-major).
-// Grid: (row chunks, output tiles of 32x32).  Partials [chunk][mb][ma].
+// Grid: (row chunks, output tiles of TI x TJ).  Partials [chunk][mb][ma].  Bound
+// by the FP64 pipe, which takes as long for padding as for columns: tiles 8 or
+// 16 wide where a block has no more columns, as in a Davidson step (15 876 rows,
+// 16 pairs: the solve 30.1 -> 26.4 ms with that and tall products of four columns
+// where eight would be padded).
 // ---------------------------------------------------------------------------
 constexpr int kGramRows = 64;
 constexpr int kGramTile = 32;
 
-__global__ void __launch_bounds__(256)
+template <int TI, int TJ>
+__global__ void __launch_bounds__(8 * TI)
 gram_partial_kernel(const double *__restrict__ A, long long lda, int ma,
                     const double *__restrict__ B, long long ldb, int mb, int n, int chunks_per_block,
                     double *__restrict__ P)
 {
     pdl_wait();  // programmatic dependent launch: predecessor done
     pdl_trigger();
-    __shared__ double as[kGramRows][kGramTile + 1];
-    __shared__ double bs[kGramRows][kGramTile + 1];
-    const int tiles_i = (ma + kGramTile - 1) / kGramTile;
+    __shared__ double as[kGramRows][TI + 1];
+    __shared__ double bs[kGramRows][TJ + 1];
+    const int tiles_i = (ma + TI - 1) / TI;
     const int ti = blockIdx.y % tiles_i;
     const int tj = blockIdx.y / tiles_i;
-    const int i0 = ti * kGramTile;
-    const int j0 = tj * kGramTile;
-    // thread -> 4 outputs: (li, lj + 8q), q = 0..3
-    const int li = threadIdx.x % kGramTile;
-    const int lj = threadIdx.x / kGramTile;  // 0..7
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const int i0 = ti * TI;
+    const int j0 = tj * TJ;
+    // thread -> TJ / 8 outputs: (li, lj + 8q)
+    constexpr int kOwn = TJ / 8;
+    const int li = threadIdx.x % TI;
+    const int lj = threadIdx.x / TI;  // 0..7
+    double acc[kOwn];
+#pragma unroll
+    for (int q = 0; q < kOwn; ++q) acc[q] = 0.0;
     for (int c = 0; c < chunks_per_block; ++c) {
         const int r0 = (blockIdx.x * chunks_per_block + c) * kGramRows;
         if (r0 >= n) {
             break;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < kGramRows * kGramTile; e += blockDim.x) {
+        for (int e = threadIdx.x; e < kGramRows * TI; e += 8 * TI) {
             const int r = e % kGramRows;
             const int col = e / kGramRows;
             const int row = r0 + r;
             as[r][col] = (row < n && i0 + col < ma) ? A[(size_t)row + (size_t)(i0 + col) * lda] : 0.0;
+        }
+        for (int e = threadIdx.x; e < kGramRows * TJ; e += 8 * TI) {
+            const int r = e % kGramRows;
+            const int col = e / kGramRows;
+            const int row = r0 + r;
             bs[r][col] = (row < n && j0 + col < mb) ? B[(size_t)row + (size_t)(j0 + col) * ldb] : 0.0;
         }
         __syncthreads();
@@ -63,14 +76,14 @@ gram_partial_kernel(const double *__restrict__ A, long long lda, int ma,
         for (int r = 0; r < kGramRows; ++r) {
             const double a = as[r][li];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
+            for (int q = 0; q < kOwn; ++q) {
                 acc[q] = fma(a, bs[r][lj + 8 * q], acc[q]);
             }
         }
     }
     const size_t mm = (size_t)ma * (size_t)mb;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kOwn; ++q) {
         const int i = i0 + li;
         const int j = j0 + lj + 8 * q;
         if (i < ma && j < mb) {
@@ -252,10 +265,10 @@ int BlockOps::gram(const double *A, long long lda, int ma, const double *B, long
     const size_t mm = (size_t)ma * (size_t)mb;
     IPTGB_CHECK(ensure_partials((size_t)blocks_x * mm));
     KernelTimerScope timer(kProfGram, stream);
+    // (narrow tiles only where one covers the columns, so that `tiles` holds)
+    const bool narrow = mb <= 16;
+    const bool small = narrow && ma <= 16;
     if (df_products) {
-        // (narrow tiles only where one covers the columns, so that `tiles` holds)
-        const bool narrow = mb <= 16;
-        const bool small = narrow && ma <= 16;
         auto kernel = small ? gram_partial_df_kernel<16, 16>
                       : narrow ? gram_partial_df_kernel<32, 16>
                                : gram_partial_df_kernel<32, 32>;
@@ -266,8 +279,11 @@ int BlockOps::gram(const double *A, long long lda, int ma, const double *B, long
                                ldc, ma, alpha, beta));
         return IPT_CUDA_SUCCESS;
     }
-    IPTGB_CHECK(launch_pdl(gram_partial_kernel, dim3(blocks_x, tiles), dim3(256), 0, stream, A,
-                           lda, ma, B, ldb, mb, n, per_block, partials));
+    auto kernel = mb <= 8 ? (small ? gram_partial_kernel<16, 8> : gram_partial_kernel<32, 8>)
+                  : narrow ? (small ? gram_partial_kernel<16, 16> : gram_partial_kernel<32, 16>)
+                           : gram_partial_kernel<32, 32>;
+    IPTGB_CHECK(launch_pdl(kernel, dim3(blocks_x, tiles), dim3(small ? 128 : 256), 0, stream, A, lda, ma,
+                           B, ldb, mb, n, per_block, partials));
     IPTGB_CHECK(launch_pdl(reduce_slices_kernel, dim3(blocks_for(mm)), dim3(kThreads), 0, stream,
                            (const double *)partials, blocks_x, mm, C, ldc, ma, alpha, beta));
     return IPT_CUDA_SUCCESS;
@@ -447,6 +463,10 @@ int BlockOps::tall_gemm(const double *A, long long lda, const double *B, long lo
     } else if ((long long)row_blocks * ((p + 15) / 16) >= want) {
         tc = 16;
         kernel = tall_gemm_kernel<16>;
+    } else if ((p + 7) / 8 * 8 > (p + 3) / 4 * 4) {
+        // the FP64 pipe takes as long for padding as for columns
+        tc = 4;
+        kernel = tall_gemm_kernel<4>;
     } else {
         tc = 8;
         kernel = tall_gemm_kernel<8>;
