@@ -472,10 +472,10 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
     // Delta (k_oz.cu): six slices (48 bits) in the mixed solve, seven (56
     // bits) in the plain FP64 solve.  Tuning knob IPT_GB300_ACCURATE_PRODUCT
     // = df selects double-FP32 arithmetic on the FP32 pipe for the mixed solve
-    // instead, fp64 (or IPT_GB300_FP64_DFMA=1) FP64 FMAs.
+    // instead, fp64 (or IPT_GB300_FP64_DFMA=1) FP64 FMAs, in the IPT steps of
+    // the plain FP64 solve as well.
     const char *ap = getenv("IPT_GB300_ACCURATE_PRODUCT");
-    const bool want_fp64 = env_flag("IPT_GB300_FP64_DFMA", 0) ||
-                           (ap != nullptr && strcmp(ap, "fp64") == 0);
+    const bool want_fp64 = fp64_fma_wanted();
     const bool want_df = ap != nullptr && strcmp(ap, "df") == 0;
     const bool use_oz = !want_fp64 && (!lowp_mode || !want_df);
     DeviceBuffer<float> Hsplit;

@@ -44,6 +44,7 @@ struct DenseFp64Operator final : Fp64Operator {
     DeviceBuffer<double> g;  // n x k gap reciprocals
     const double *H = nullptr;
     int n = 0, k = 0;
+    int slices = 7;  // 0: FP64 FMAs, where the environment asks for them
     cudaStream_t stream = nullptr;
     // scans H (column-major n x n); d (optional) receives its diagonal
     int bind(const double *H, int n, double *d, cudaStream_t s);

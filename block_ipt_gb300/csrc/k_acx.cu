@@ -98,7 +98,7 @@ acx_products_kernel(const double *__restrict__ X, const double *__restrict__ F1,
     const double2 s = block_sum2(num, den);
     if (threadIdx.x == 0) {
         part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
-        if (blockIdx.x == 0) colmax[blockIdx.y] = 0;
+        if (blockIdx.x == 0 && colmax != nullptr) colmax[blockIdx.y] = 0;
     }
 }
 
@@ -138,10 +138,12 @@ acx_update_kernel(double *__restrict__ X, const double *__restrict__ F1,
             v = x + fma(3.0 * g, d1, fma(3.0 * g2, d2, g3 * d3));
         }
         X[base + i] = v;
+        if (colmax == nullptr) continue;
         const unsigned long long a =
             (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFULL;
         m = a > m ? a : m;
     }
+    if (colmax == nullptr) return;
     for (int off = 16; off > 0; off >>= 1) {
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, m, off);
         m = o > m ? o : m;
@@ -410,7 +412,13 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
         };
         if (status == ACX_CUDA_SUCCESS) {
             cuda_ok(cudaMemsetAsync(flags.ptr, 0, 2 * sizeof(int), s));
-            if (lib_ok(F.matrix.scan_rows(H, n, d, s)) && lib_ok(F.matrix.build_words(7, s))) {
+            if (fp64_fma_wanted()) {
+                F.matrix.reference(H, n);
+                if (lib_ok(launch_extract_diagonal(H, n, n, d, s))) {
+                    lib_ok(F.product.bind(&F.matrix, d, 0, s));
+                }
+            } else if (lib_ok(F.matrix.scan_rows(H, n, d, s)) &&
+                       lib_ok(F.matrix.build_words(7, s))) {
                 lib_ok(F.product.bind(&F.matrix, d, 7, s));
             }
             if (initial == nullptr) {
@@ -467,7 +475,7 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                 result->f_calls += 1;
             }
             const double *f3 = order == 3 ? F3.ptr : nullptr;
-            unsigned long long *maxima = F.product.column_maxima();
+            unsigned long long *maxima = F.product.column_maxima();  // null with FP64 FMAs
             lib_ok(launch_pdl(acx_products_kernel, dim3(ext_blocks, k), dim3(kAcxThreads), 0, s,
                               (const double *)X.ptr, (const double *)f1, (const double *)F2.ptr,
                               f3, n, ext.ptr, maxima));

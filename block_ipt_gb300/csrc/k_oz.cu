@@ -48,6 +48,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -861,12 +862,15 @@ struct Partials {
     const int *colexp;
     int n, cp, tiles, periods, maxslots, out;  // out: OzSplit::kOut
     long long items, G;
+    // FP64 FMAs: the partials are `maxslots` n x C blocks of H X
+    int fma, C;
     const int *err;  // set by a product whose bounded wait gave up: its results are NaN
 };
 
 // Number of partials of column c's group in a tile.
 __device__ __forceinline__ int slots_of(const Partials &p, int c, int tile)
 {
+    if (p.fma) return p.maxslots;
     if (tile >= p.tiles) return 0;
     const long long gt = (long long)(c / p.cp) * p.tiles + tile;
     return (int)(owner_of(gt * p.periods + p.periods - 1, p.items, p.G) -
@@ -896,6 +900,17 @@ __device__ __forceinline__ double delta_entry(const Partials &p, int i, int c, i
 #pragma unroll 4
     for (int u = 0; u < slots; ++u) s += q[u * stride];
     return scale2(s, ei + fc + p.out);
+}
+
+// (H X)_ic from the K slices of an FP64 FMA product, in order.
+__device__ __forceinline__ double fma_entry(const Partials &p, int i, int c)
+{
+    const size_t stride = (size_t)p.n * p.C;
+    const double *q = p.P + (size_t)i + (size_t)c * p.n;
+    double s = 0.0;
+#pragma unroll 4
+    for (int u = 0; u < p.maxslots; ++u) s += q[u * stride];
+    return s;
 }
 
 constexpr int kFinishRows = 256;  // rows of one column a finish block covers
@@ -944,7 +959,8 @@ oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
 // want_norms ||X' - X||_F, ||X||_F (ipt_cuda.cu:1457-1467,1663-1688); with
 // resid_part also the block's part of ||(H X)_c - X_c (H X)_cc||^2 (ACX).  A
 // row of H or column of X that is not finite takes the FP64 sums the map is
-// defined by, so Inf and NaN travel as there.
+// defined by, so Inf and NaN travel as there.  The partials of an FP64 FMA
+// product hold H X: the diagonal's part is taken off here.
 //
 // A block of 8 warps takes 256 R rows of one column, R per thread; a ninth
 // warp forms c_j while the others load.  With R = 4 the shuffle sums of the
@@ -976,14 +992,16 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     pdl_wait();
     pdl_trigger();
     const double *xc = X + (size_t)c * n;
-    const int fc = p.colexp[c];
+    const int fc = p.fma ? 0 : p.colexp[c];
     // (H X)_rc - d_r X_rc by the plain FP64 sum
     auto direct = [&](int r) {
         double y = 0.0;
         for (int l = 0; l < n; ++l) y = fma(H[(size_t)r + (size_t)l * n], xc[l], y);
         return y - d[r] * xc[r];
     };
-    auto delta = [&](int r, int er, int count) {
+    auto delta = [&](int r, int count) {
+        if (p.fma) return fma(-d[r], xc[r], fma_entry(p, r, c));
+        const int er = p.rowexp[r];
         return (er == kOzNonFinite || fc == kOzNonFinite) ? direct(r)
                                                           : delta_entry(p, r, c, count, er, fc);
     };
@@ -996,11 +1014,11 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
             if (i < n) {
                 x[q] = xc[i];
                 gi[q] = g[(size_t)i + (size_t)c * n];
-                y[q] = delta(i, p.rowexp[i], slots[(q * kUpdateThreads + t) / kBM]);
+                y[q] = delta(i, slots[(q * kUpdateThreads + t) / kBM]);
             }
         }
     } else if (t == kUpdateThreads) {
-        cj_sh = delta(c, p.rowexp[c], slots[kTiles]);
+        cj_sh = delta(c, slots[kTiles]);
     }
     __syncthreads();
     const double cj = cj_sh;
@@ -1030,8 +1048,10 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
             }
         }
     }
-    m = warp_max(m);
-    if ((t & 31) == 0 && m != 0) atomicMax(colmax_next + c, m);
+    if (!p.fma) {
+        m = warp_max(m);
+        if ((t & 31) == 0 && m != 0) atomicMax(colmax_next + c, m);
+    }
     if (RESID) {
         const double2 r = block_sum2(rsq, 0.0);
         if (t == 0) resid_part[blockIdx.x] = r.x;
@@ -1158,6 +1178,12 @@ oz_words_kernel(const double *__restrict__ H, int n, int nst, const int *__restr
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+void OzMatrix::reference(const double *H_, int n_)
+{
+    H = H_;
+    n = n_;
+}
+
 int OzMatrix::init_storage(int n_, cudaStream_t s)
 {
     n = n_;
@@ -1293,6 +1319,13 @@ int OzProduct::shape_for(int C)
     OzShape q;
     q.n = n;
     q.C = C;
+    if (slices == 0) {
+        q.maxslots = dense64_split_for(n, C, sms);
+        const size_t need = (size_t)q.maxslots * n * C;
+        if (P.count < need) IPTGB_CHECK(P.alloc(need, s));
+        sh = q;
+        return IPT_CUDA_SUCCESS;
+    }
     q.cp = group_cols(slices, C);
     q.groups = (C + q.cp - 1) / q.cp;
     q.tiles = (n + oz::kBM - 1) / oz::kBM;
@@ -1378,6 +1411,8 @@ oz::Partials OzProduct::partials() const
 {
     oz::Partials p;
     p.P = P.ptr;
+    p.fma = slices == 0;
+    p.C = sh.C;
     p.rowexp = m->rowexp.ptr;
     p.colexp = colexp.ptr;
     p.n = sh.n;
@@ -1416,7 +1451,7 @@ int OzProduct::apply(const double *X, long long ldx, int C, double *Y, long long
 int OzProduct::begin(const double *X, int C)
 {
     IPTGB_CHECK(shape_for(C));
-    return scan_columns(X, sh.n);
+    return slices == 0 ? IPT_CUDA_SUCCESS : scan_columns(X, sh.n);
 }
 
 int OzProduct::update_row_blocks(int n, int C, int sms, bool *wide)
@@ -1444,7 +1479,13 @@ int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms
     const size_t set = (size_t)sh.groups * sh.cp;
     {
         KernelTimerScope timer(kProfFp64Product, s);
-        IPTGB_CHECK(slice_and_multiply(X, sh.n, 1));
+        if (slices == 0) {
+            IPTGB_CHECK(launch_dense64_partial(m->H, sh.n, sh.n, X, sh.n, sh.C, P.ptr,
+                                               sh.maxslots, s));
+            defer_norms = false;  // (there is no digit pass to finish them)
+        } else {
+            IPTGB_CHECK(slice_and_multiply(X, sh.n, 1));
+        }
     }
     KernelTimerScope timer(kProfFp64Update, s);
     auto update = resid_part == nullptr
@@ -1469,6 +1510,12 @@ int OzProduct::read_error(int *host_err)
     IPTGB_CUDA(cudaMemcpyAsync(host_err, err.ptr, sizeof(int), cudaMemcpyDeviceToHost, s));
     IPTGB_CUDA(cudaStreamSynchronize(s));
     return IPT_CUDA_SUCCESS;
+}
+
+bool fp64_fma_wanted()
+{
+    const char *ap = getenv("IPT_GB300_ACCURATE_PRODUCT");
+    return env_flag("IPT_GB300_FP64_DFMA", 0) != 0 || (ap != nullptr && strcmp(ap, "fp64") == 0);
 }
 
 int launch_gap_reciprocals(const double *d, int n, int k, double *g, cudaStream_t s)

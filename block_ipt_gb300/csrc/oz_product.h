@@ -24,6 +24,8 @@ struct OzMatrix {
     int words_slices = 0;  // digits per entry in `words` (0: none)
     DeviceBuffer<int> rowexp;
     DeviceBuffer<uint4> words;  // oz_word_index
+    // H alone, for products in FP64 FMAs
+    void reference(const double *H, int n);
     int init_storage(int n, cudaStream_t s);
     // storage of the words only (the mixed solve's fused setup writes them)
     int alloc_words(int slices, cudaStream_t s);
@@ -45,13 +47,14 @@ constexpr size_t kMaxWordBytes = (size_t)16 << 30;
 struct OzShape {
     int n = 0, C = 0, cp = 0, groups = 0, tiles = 0, periods = 0, ldp = 0, grid = 0;
     int spp = 0;       // 32-element K stages per item
-    int maxslots = 0;  // partials a (group, tile) can have
+    int maxslots = 0;  // partials a (group, tile) can have; FP64 FMAs: K slices
     long long items = 0;
 };
 
 // Y = (diag(d) + Delta) X for an n x C block X (column-major, ld ldx); d may
 // be null (Y = Delta X).  slices = 6: the 48-bit split; 7: the 56-bit split
-// of the plain FP64 path (oz.cuh).
+// of the plain FP64 path (oz.cuh); 0: no split, FP64 FMAs (k_dense64.cu; step()
+// only).
 namespace oz {
 struct Partials;
 }
@@ -91,7 +94,11 @@ struct OzProduct {
     int flush_norms();
     static int update_row_blocks(int n, int C, int sms, bool *wide);
     // the column maxima (bit patterns) the next step reads
-    unsigned long long *column_maxima() { return colmax.ptr + (size_t)cur * sh.groups * sh.cp; }
+    // (null with FP64 FMAs)
+    unsigned long long *column_maxima()
+    {
+        return slices == 0 ? nullptr : colmax.ptr + (size_t)cur * sh.groups * sh.cp;
+    }
 
     // the kernel's error flag (non-zero: a bounded wait gave up)
     int read_error(int *host_err);
@@ -102,6 +109,10 @@ struct OzProduct {
     int slice_and_multiply(const double *X, long long ldx, int clear_other);
     oz::Partials partials() const;
 };
+
+// Does the caller's environment ask for FP64 FMAs (IPT_GB300_FP64_DFMA=1 or
+// IPT_GB300_ACCURATE_PRODUCT=fp64)?
+bool fp64_fma_wanted();
 
 // g_ij = 1 / (d_j - d_i) for the n x k block (NaN for a zero or non-finite
 // gap, as the reference's build_g_kernel with min_gap_allowed = 0).
