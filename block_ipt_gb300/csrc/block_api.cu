@@ -108,7 +108,6 @@ struct Fp64Stage final : IptStage {
     CsrFp64Operator *csr = nullptr;
     const double *d = nullptr;
     int n = 0;
-    int sms = 148;
     cudaStream_t s = nullptr;
     DeviceBuffer<double> Y, Xb;
 
@@ -180,18 +179,21 @@ struct Fp64Stage final : IptStage {
     }
 };
 
-IptStage *make_fp64_dense_stage(const double *dH, int n, const double *d, cudaStream_t stream)
+IptStage *make_fp64_dense_stage(const double *dH, int n, const double *d, const OzMatrix *matrix,
+                                cudaStream_t stream, int *status)
 {
     auto *st = new Fp64Stage();
     auto *op = new DenseFp64Operator();
     st->op.reset(op);
-    if (op->bind(dH, n, nullptr, stream) != IPT_CUDA_SUCCESS) {
+    *status = IPT_CUDA_SUCCESS;
+    if (matrix != nullptr) op->share(matrix, stream);
+    else *status = op->bind(dH, n, nullptr, stream);
+    if (*status != IPT_CUDA_SUCCESS) {
         delete st;
         return nullptr;
     }
     st->d = d;
     st->n = n;
-    st->sms = device_sm_count();
     st->s = stream;
     return st;
 }
@@ -210,7 +212,6 @@ IptStage *make_fp64_csr_stage(const int *row_ptr, const int *col_ind, const doub
     st->csr = op;
     st->d = d;
     st->n = n;
-    st->sms = device_sm_count();
     st->s = stream;
     return st;
 }
@@ -622,8 +623,9 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         trace_mark("dense:operator_done", s);
         stage.reset(make_lowp_stage_on(lowp.get(), d.ptr, n, s));
     } else {
-        stage.reset(make_fp64_dense_stage(dH, n, d.ptr, s));
-        if (stage == nullptr) return IPT_CUDA_CUDA_ERROR;
+        // the steps read the digits laid out above
+        stage.reset(make_fp64_dense_stage(dH, n, d.ptr, use_oz ? &ozm : nullptr, s, &st));
+        if (stage == nullptr) return st;
     }
     std::unique_ptr<LearnedCorrection> learned;
     DeviceBuffer<double> coupling;

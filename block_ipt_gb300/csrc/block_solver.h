@@ -10,6 +10,8 @@
 
 namespace iptgb {
 
+struct OzMatrix;
+
 // FP64-accurate block product AV = H V (V, AV: n x c, ld = n).
 struct Fp64Apply {
     virtual ~Fp64Apply() = default;
@@ -161,7 +163,9 @@ IptStage *make_lowp_dense_stage(const double *dH, int n, const double *d, int pr
                                 cudaStream_t stream, int *status);
 
 // FP64 IPT stages on the plain operators.
-IptStage *make_fp64_dense_stage(const double *dH, int n, const double *d, cudaStream_t stream);
+// matrix: the digits of dH where the caller has laid them out, or null
+IptStage *make_fp64_dense_stage(const double *dH, int n, const double *d, const OzMatrix *matrix,
+                                cudaStream_t stream, int *status);
 IptStage *make_fp64_csr_stage(const int *row_ptr, const int *col_ind, const double *vals, int n,
                               const double *d, cudaStream_t stream);
 

@@ -26,17 +26,26 @@ int DenseFp64Operator::bind(const double *H_, int n_, double *d, cudaStream_t s)
     stream = s;
     slices = fp64_fma_wanted() ? 0 : 7;
     if (slices == 0) {
-        matrix.reference(H, n);
+        own.reference(H, n);
         return d != nullptr ? launch_extract_diagonal(H, n, n, d, s) : IPT_CUDA_SUCCESS;
     }
-    IPTGB_CHECK(matrix.scan_rows(H, n, d, s));
-    return matrix.build_words(7, s);
+    IPTGB_CHECK(own.scan_rows(H, n, d, s));
+    return own.build_words(7, s);
+}
+
+void DenseFp64Operator::share(const OzMatrix *scanned, cudaStream_t s)
+{
+    matrix = scanned;
+    H = scanned->H;
+    n = scanned->n;
+    stream = s;
+    slices = 7;
 }
 
 int DenseFp64Operator::start(const double *X, int k_, const double *d)
 {
     k = k_;
-    IPTGB_CHECK(product.bind(&matrix, d, slices, stream));
+    IPTGB_CHECK(product.bind(matrix, d, slices, stream));
     if (g.count < (size_t)n * k) IPTGB_CHECK(g.alloc((size_t)n * k, stream));
     IPTGB_CHECK(launch_gap_reciprocals(d, n, k, g.ptr, stream));
     return product.begin(X, k);

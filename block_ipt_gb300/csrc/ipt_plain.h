@@ -39,7 +39,8 @@ struct Fp64Operator {
 // k = 1501 8e-16 against 7e-14 in the 2-norm: the diagonal, which the FP64
 // product carried through y and the map took off again, is left out).
 struct DenseFp64Operator final : Fp64Operator {
-    OzMatrix matrix;
+    OzMatrix own;
+    const OzMatrix *matrix = &own;
     OzProduct product;
     DeviceBuffer<double> g;  // n x k gap reciprocals
     const double *H = nullptr;
@@ -48,6 +49,8 @@ struct DenseFp64Operator final : Fp64Operator {
     cudaStream_t stream = nullptr;
     // scans H (column-major n x n); d (optional) receives its diagonal
     int bind(const double *H, int n, double *d, cudaStream_t s);
+    // the same on a matrix the caller has scanned and laid out (and keeps)
+    void share(const OzMatrix *scanned, cudaStream_t s);
     int start(const double *X, int k, const double *d) override;
     int step(const double *X, double *Xn, const double *d, int want_norms,
              NormScratch *ns) override;

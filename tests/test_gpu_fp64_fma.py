@@ -106,19 +106,34 @@ def pool_peak(torch, call):
     return value.value
 
 
-@pytest.mark.parametrize("knob", KNOBS)
-def test_block_solver_lays_out_no_digits(cuda, monkeypatch, knob):
-    torch = cuda
-    monkeypatch.setenv(*knob)
-    n, k = 2048, 8
+def block_case(torch, n, k):
     rng = np.random.default_rng(2)
     A = rng.standard_normal((n, n)) * (0.05 / np.sqrt(n))
     H = A + A.T + np.diag(np.arange(1.0, n + 1))
     dH = torch.from_numpy(H).cuda()
     X = torch.empty(k, n, dtype=torch.float64, device="cuda")
     w = torch.empty(k, dtype=torch.float64, device="cuda")
-    peak = pool_peak(torch, lambda: api.block_solve_dense_device(
-        dH.data_ptr(), n, k, X.data_ptr(), w.data_ptr(), "fp64"))
-    assert peak < 8 * n * n
+
+    def solve():
+        api.block_solve_dense_device(dH.data_ptr(), n, k, X.data_ptr(), w.data_ptr(), "fp64")
+
+    return H, solve, w
+
+
+def test_block_solver_lays_the_digits_out_once(cuda):
+    """8 n^2 bytes of digit words, and less than half of that for the rest."""
+    n, k = 4096, 8
+    H, solve, w = block_case(cuda, n, k)
+    peak = pool_peak(cuda, solve)
+    assert 8 * n * n <= peak < 12 * n * n
+    assert np.abs(w.cpu().numpy() - np.linalg.eigvalsh(H)[:k]).max() <= 1e-10 * np.abs(H).sum(1).max()
+
+
+@pytest.mark.parametrize("knob", KNOBS)
+def test_block_solver_lays_out_no_digits(cuda, monkeypatch, knob):
+    monkeypatch.setenv(*knob)
+    n, k = 2048, 8
+    H, solve, w = block_case(cuda, n, k)
+    assert pool_peak(cuda, solve) < 8 * n * n
     # eigenvalues to the solver's residual tolerance
     assert np.abs(w.cpu().numpy() - np.linalg.eigvalsh(H)[:k]).max() <= 1e-10 * np.abs(H).sum(1).max()
