@@ -572,8 +572,11 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
                                  : "r"(src + (uint32_t)(((4 * g0 + j) ^ (r & 7)) << 4))
                                  : "memory");
                 }
-                // the slot may be refilled: every lane's reads precede the
-                // arrival (a release)
+                // the slot may be refilled once every lane's words have arrived:
+                // the arrival alone does not wait for loads under way (with more
+                // work in the drain warps rows came out wrong, and otherwise in
+                // the next run)
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(raw_empty(rq));
             } else {
