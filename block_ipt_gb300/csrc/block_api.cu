@@ -478,7 +478,7 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
     const char *ap = getenv("IPT_GB300_ACCURATE_PRODUCT");
     const bool want_fp64 = fp64_fma_wanted();
     const bool want_df = ap != nullptr && strcmp(ap, "df") == 0;
-    const bool use_oz = !want_fp64 && (!lowp_mode || !want_df);
+    bool use_oz = !want_fp64 && (!lowp_mode || !want_df);
     DeviceBuffer<float> Hsplit;
     OzMatrix ozm;
     OzProduct ozp;
@@ -587,7 +587,10 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         if (!fused) {
             IPTGB_CHECK(ozm.scan_rows(dH, n, nullptr, s));
             IPTGB_CHECK(ozm.build_words(lowp_mode ? kOzSlices : 7, s));
+            use_oz = !ozm.wide;
         }
+    }
+    if (use_oz) {
         IPTGB_CHECK(ozp.bind(&ozm, d.ptr, lowp_mode ? kOzSlices : 7, s));
         apply.oz = &ozp;
     }
@@ -624,7 +627,7 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         stage.reset(make_lowp_stage_on(lowp.get(), d.ptr, n, s));
     } else {
         // the steps read the digits laid out above
-        stage.reset(make_fp64_dense_stage(dH, n, d.ptr, use_oz ? &ozm : nullptr, s, &st));
+        stage.reset(make_fp64_dense_stage(dH, n, d.ptr, want_fp64 ? nullptr : &ozm, s, &st));
         if (stage == nullptr) return st;
     }
     std::unique_ptr<LearnedCorrection> learned;

@@ -30,7 +30,9 @@ int DenseFp64Operator::bind(const double *H_, int n_, double *d, cudaStream_t s)
         return d != nullptr ? launch_extract_diagonal(H, n, n, d, s) : IPT_CUDA_SUCCESS;
     }
     IPTGB_CHECK(own.scan_rows(H, n, d, s));
-    return own.build_words(7, s);
+    IPTGB_CHECK(own.build_words(7, s));
+    if (own.wide) slices = 0;
+    return IPT_CUDA_SUCCESS;
 }
 
 void DenseFp64Operator::share(const OzMatrix *scanned, cudaStream_t s)
@@ -39,7 +41,7 @@ void DenseFp64Operator::share(const OzMatrix *scanned, cudaStream_t s)
     H = scanned->H;
     n = scanned->n;
     stream = s;
-    slices = 7;
+    slices = scanned->wide ? 0 : 7;
 }
 
 int DenseFp64Operator::start(const double *X, int k_, const double *d)

@@ -32,12 +32,21 @@ struct Fp64Operator {
 // Dense H: Delta X by the 56-bit digit-slice product on the tensor cores
 // (k_oz.cu), whose consumer applies the map.  It replaces a split-K FP64 SIMT
 // product (GB300 runs FP64 FMAs at 1/64 of the FP32 rate; on a matrix of few
-// row blocks most SMs stood idle as well): a step takes 140 us instead of 3.7
-// ms at n = 8192, k = 32, 17 us instead of 105 us at n = 1024, k = 8 and 12 us
-// at n = 256, k = 4, so no size keeps the old one; 0.45 instead of 6.1 ms with
-// all n = 1501 columns.  Its error is the smaller one (after 12 steps at n =
-// k = 1501 8e-16 against 7e-14 in the 2-norm: the diagonal, which the FP64
-// product carried through y and the map took off again, is left out).
+// row blocks most SMs stood idle as well): a step takes 172 us instead of 3.7
+// ms at n = 8192, k = 32, 29 us instead of 105 us at n = 1024, k = 8, so no
+// size keeps the old one for its time; 0.35 instead of 6.1 ms with all n = 1501
+// columns.
+//
+// Its error: in the 2-norm it is the smaller one (after 12 steps at n = k =
+// 1501 8e-16 against 7e-14: the diagonal, which the FP64 product carried
+// through y and the map took off again, is left out).  Entry by entry, a block
+// of 128 columns adds up to 128 2^-54 max_l |Delta_il| max_l |X_lc| (l in the
+// block) to an entry of Delta X, where FP64 FMAs stay relative to the terms
+// themselves.  So a matrix with rows whose entries span many binades within a
+// block (graded ones, sparse or banded ones stored as dense, couplings that
+// decay within tens of rows) keeps the FP64 FMAs, found out when the digits are
+// laid out (OzMatrix::wide): every entry of the vectors is then as accurate as
+// theirs.
 struct DenseFp64Operator final : Fp64Operator {
     OzMatrix own;
     const OzMatrix *matrix = &own;

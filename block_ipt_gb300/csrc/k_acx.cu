@@ -419,7 +419,7 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                 }
             } else if (lib_ok(F.matrix.scan_rows(H, n, d, s)) &&
                        lib_ok(F.matrix.build_words(7, s))) {
-                lib_ok(F.product.bind(&F.matrix, d, 7, s));
+                lib_ok(F.product.bind(&F.matrix, d, F.matrix.wide ? 0 : 7, s));
             }
             if (initial == nullptr) {
                 lib_ok(launch_set_identity(X.ptr, n, k, s));

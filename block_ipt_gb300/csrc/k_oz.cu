@@ -25,8 +25,10 @@
 //    costs its issuing thread tens of cycles;
 //  * warps 8-15 drain the level accumulators after every period (two sets, so
 //    the next period's MMAs run meanwhile, when they fit in TMEM).  S = 7 adds
-//    the levels as 96-bit integers, exactly; S = 6 combines them in
-//    double-float arithmetic.  A CTA leaving a tile writes one FP64 partial.
+//    the levels as 96-bit integers, moved to the largest of the scales that
+//    the row's and the column's blocks of 128 entries have; S = 6 combines
+//    them in double-float arithmetic.  A CTA leaving a tile writes one FP64
+//    partial.
 // The consumer of the partials (oz_finish_kernel or oz_update_kernel) adds
 // those of a tile in a fixed order, so the product is deterministic.
 //
@@ -35,13 +37,14 @@
 // the MMAs read the digit rows of X 34 times 2 KB: 265 KB, 2070 cycles at 128
 // bytes per cycle, against 1090 cycles of MMA and 32 KB of HBM traffic (79 us
 // per product of n = 8192 at the measured 6.8 TB/s).  Measured at n = 8192, 32
-// columns: 127 us per product (2240 cycles per stage; tensor pipe 50 %, HBM
-// 54 %); the split-K FP64 SIMT product it replaces in the plain path 3.6 ms
-// (95 % of the FP64 pipe).  Digit slices stored as FP16 (14 bytes per entry
-// with 7 slices) would need 139 us of HBM time; extracting the digits from H
-// in every product took 205 us (55 instructions per entry); A operands
-// in TMEM instead of shared memory 137 us (their tcgen05.st wait for the
-// MMAs, and only one accumulator set fits).
+// columns: 132 us per product with one scale per row and column (2240 cycles
+// per stage; tensor pipe 50 %, HBM 54 %), 157 us with those of S = 7 (35 more
+// instructions per sum in the drain); the split-K FP64 SIMT product it replaces
+// in the plain path 3.6 ms (95 % of the FP64 pipe).  With one scale: digit
+// slices stored as FP16 (14 bytes per entry with 7 slices) would need 139 us of
+// HBM time; extracting the digits from H in every product took 205 us (55
+// instructions per entry); A operands in TMEM instead of shared memory 137 us
+// (their tcgen05.st wait for the MMAs, and only one accumulator set fits).
 //
 // Every mbarrier wait is bounded; a timeout sets the error flag, the CTA
 // drains its own copies and MMAs (bounded), frees TMEM and returns.
@@ -93,7 +96,12 @@ enum Mode { kRows = 0, kWords = 1 };
 struct Params {
     const double *H;
     const uint4 *words;
-    const int *rowexp;
+    const int *rowexp;    // S = 6: per row
+    // S = 7: biased exponents (oz_pack_exponent) of Delta, [block][row], and of
+    // X, [group][block][CP], two to a word
+    const uint16_t *blockexp;
+    const uint32_t *xexp;
+    int blocks;           // of kOzBlock K elements
     int n, groups, tiles, periods, nstages;  // nstages: K stages of a row
     int spp;         // stages per period (item): at most kMaxStagesPerItem
     long long items;
@@ -170,12 +178,13 @@ __device__ __forceinline__ uint64_t l2_normal_policy()
 // periods + per, stage st of its period.
 struct Walk {
     long long it;
-    int tile, per, st, count;  // count: stages of this period
+    int grp, tile, per, st, count;  // count: stages of this period
     __device__ __forceinline__ void start(long long first, const Params &p)
     {
         it = first;
         per = (int)(first % p.periods);
         tile = (int)((first / p.periods) % p.tiles);
+        grp = (int)(first / ((long long)p.periods * p.tiles));
         st = 0;
         count = min(p.spp, p.nstages - per * p.spp);
     }
@@ -186,9 +195,18 @@ struct Walk {
         ++it;
         if (++per == p.periods) {
             per = 0;
-            if (++tile == p.tiles) tile = 0;
+            if (++tile == p.tiles) {
+                tile = 0;
+                ++grp;
+            }
         }
         count = min(p.spp, p.nstages - per * p.spp);
+    }
+    // to the next item
+    __device__ __forceinline__ void skip(const Params &p)
+    {
+        st = count - 1;
+        next(p);
     }
 };
 
@@ -219,7 +237,7 @@ __device__ __forceinline__ void fetch8(const Params &p, const Walk &w, int r, in
     }
 }
 
-__device__ __forceinline__ void tmem_ld_4cols(uint32_t taddr, uint32_t (&r)[4])
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[4])
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -228,60 +246,129 @@ __device__ __forceinline__ void tmem_ld_4cols(uint32_t taddr, uint32_t (&r)[4])
 
 // Waits for the TMEM loads issued so far; naming the registers they fill keeps
 // every use of them behind the wait.
-template <int V>
-__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[V][4])
+template <int V, int N>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[V][N])
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int l = 0; l < V; ++l) {
-        asm volatile("" : "+r"(r[l][0]), "+r"(r[l][1]), "+r"(r[l][2]), "+r"(r[l][3])::"memory");
+#pragma unroll
+        for (int j = 0; j < N; ++j) asm volatile("" : "+r"(r[l][j])::"memory");
     }
+}
+
+// v 2^e; one multiplication where 2^e is a normal number.
+__device__ __forceinline__ double scale2(double v, int e)
+{
+    if (e > -1022 && e < 1023) return v * __hiloint2double((e + 1023) << 20, 0);
+    return ldexp(v, e);
 }
 
 // Running sums of a thread's columns over the periods of a tile.
 template <int S, int NC>
 struct Sums;
-// 56-bit split: exact 96-bit integers (three words; a pair of 64-bit sums
-// would not leave the drain's loads enough registers).  Per period the levels
-// 0-3 and 4-7 are each combined by one wide multiply-add per level into 64
-// bits (below 2^48), with weights 2^24, 2^16, 2^8, 1.
+// 56-bit split: 96-bit integers (three words; a pair of 64-bit sums would not
+// leave the drain's loads enough registers) in units of 2^(E + kOut), E at
+// least the exponent of every product so far.  Per period the levels 0-3 and
+// 4-7 are each combined by one wide multiply-add per level into 64 bits (below
+// 2^48), with weights 2^24, 2^16, 2^8, 1; the sum, below 2^80, moves down to
+// the unit.  Exponents are pairs of biased 16-bit ones (two columns;
+// oz_pack_exponent), so that one addition or subtraction serves both.
 template <int NC>
 struct Sums<7, NC> {
     uint32_t w[NC][3];
+    uint32_t E[NC / 2];
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
         for (int j = 0; j < NC; ++j) w[j][0] = w[j][1] = w[j][2] = 0;
-    }
-    __device__ __forceinline__ void add(int j, const uint32_t (&l)[8])
-    {
-        constexpr int kWeight[4] = {1 << 24, 1 << 16, 1 << 8, 1};
-        long long part[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            part[h] = __float2int_rn(__uint_as_float(l[4 * h + 3]));
+        for (int j = 0; j < NC / 2; ++j) E[j] = 0;
+    }
+    // columns 4, 5, ... become columns 0, 1, ...
+    __device__ __forceinline__ void rotate()
+    {
+        uint32_t t[4][3];
+        const uint32_t e0 = E[0], e1 = E[1];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                const int v = __float2int_rn(__uint_as_float(l[4 * h + q]));
-                asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(part[h]) : "r"(v), "r"(kWeight[q]));
+                if (j < 4) t[j][q] = w[j][q];
+                w[j][q] = j + 4 < NC ? w[j + 4 < NC ? j + 4 : j][q] : t[j + 4 - NC][q];
             }
         }
-        asm("{\n\t.reg .u32 a, b, c, d, e;\n\t"
-            "mov.b64 {a, b}, %3;\n\t"
-            "mov.b64 {c, d}, %4;\n\t"
-            "shr.s32 e, d, 31;\n\t"
-            "add.cc.u32 %0, %0, c;\n\t"
-            "addc.cc.u32 %1, %1, d;\n\t"
-            "addc.u32 %2, %2, e;\n\t"
-            "add.cc.u32 %1, %1, a;\n\t"
-            "addc.u32 %2, %2, b;\n\t}"
+#pragma unroll
+        for (int j = 0; j + 2 < NC / 2; ++j) E[j] = E[j + 2];
+        E[NC / 2 - 2] = e0;
+        E[NC / 2 - 1] = e1;
+    }
+    // x down by `bits` (at most 95)
+    static __device__ __forceinline__ void shift(uint32_t (&x)[3], uint32_t bits)
+    {
+        const uint32_t sign = (uint32_t)((int)x[2] >> 31);
+        const bool two = bits >= 64, one = (bits & 32) != 0;
+        const uint32_t u0 = two ? x[2] : x[0], u1 = two ? sign : x[1], u2 = two ? sign : x[2];
+        const uint32_t v0 = one ? u1 : u0, v1 = one ? u2 : u1, v2 = one ? sign : u2;
+        x[0] = __funnelshift_r(v0, v1, bits);
+        x[1] = __funnelshift_r(v1, v2, bits);
+        x[2] = (uint32_t)((int)v2 >> (bits & 31));
+    }
+    // Units for products of exponents e(j) (pairs).  One that has to rise goes
+    // kSpare binades beyond: the next rise is seldom then (entries that grow
+    // towards the diagonal), and 2^-66 is far below the operands' 2^-56.
+    static constexpr uint32_t kSpare = 6u | 6u << 16;
+    template <typename F>
+    __device__ __forceinline__ void raise(F e)
+    {
+        uint32_t above = 0;  // (e() is warp-collective)
+#pragma unroll
+        for (int j = 0; j < NC / 2; ++j) above |= __vmaxu2(E[j], e(j)) ^ E[j];
+        if (!__any_sync(0xffffffffu, above != 0)) return;
+#pragma unroll
+        for (int j = 0; j < NC / 2; ++j) {
+            // (0 or the new unit, per half)
+            const uint32_t ej = e(j);
+            const uint32_t up = __vcmpgtu2(ej, E[j]);
+            const uint32_t now = ((ej + kSpare) & up) | (E[j] & ~up);
+            const uint32_t by = __vminu2(now - E[j], 95u | 95u << 16);
+            E[j] = now;
+            shift(w[2 * j], by & 0xFFFFu);
+            shift(w[2 * j + 1], by >> 16);
+        }
+    }
+    // v + x w, on the multiply pipe (the integer one is the converters')
+    static __device__ __forceinline__ long long mad(int x, int w, long long v)
+    {
+        asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(v) : "r"(x), "r"(w));
+        return v;
+    }
+    static __device__ __forceinline__ long long combine(uint32_t l0, uint32_t l1, uint32_t l2,
+                                                        uint32_t l3)
+    {
+        long long v = mad(__float2int_rn(__uint_as_float(l3)), 1, 0);
+        v = mad(__float2int_rn(__uint_as_float(l2)), 1 << 8, v);
+        v = mad(__float2int_rn(__uint_as_float(l1)), 1 << 16, v);
+        return mad(__float2int_rn(__uint_as_float(l0)), 1 << 24, v);
+    }
+    // column j: hi 2^32 + lo, `down` bits (at most 95) below the unit
+    __device__ __forceinline__ void add(int j, long long hi, long long lo, uint32_t down)
+    {
+        const long long top = mad((int)(lo >> 32), 1, hi);
+        uint32_t x[3] = {(uint32_t)lo, (uint32_t)top, (uint32_t)(top >> 32)};
+        shift(x, down);
+        asm("add.cc.u32 %0, %0, %3;\n\t"
+            "addc.cc.u32 %1, %1, %4;\n\t"
+            "addc.u32 %2, %2, %5;"
             : "+r"(w[j][0]), "+r"(w[j][1]), "+r"(w[j][2])
-            : "l"(part[0]), "l"(part[1]));
+            : "r"(x[0]), "r"(x[1]), "r"(x[2]));
     }
     __device__ __forceinline__ double value(int j) const
     {
         const long long hi = (long long)(((uint64_t)w[j][2] << 32) | w[j][1]);
-        return (double)hi * 4294967296.0 + (double)w[j][0];
+        const int e = (int)((j & 1) != 0 ? E[j >> 1] >> 16 : E[j >> 1] & 0xFFFFu);
+        return scale2((double)hi * 4294967296.0 + (double)w[j][0],
+                      e + 2 * kOzZeroExp + OzSplit<7>::kOut);
     }
 };
 // 48-bit split: double-float (H, L).
@@ -402,7 +489,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
                 }
                 const uint32_t dst = b0 + (uint32_t)q * kBBytes;
                 const int x = (w.per * prm.spp + w.st) * kStageK;
-                const int y = (int)(w.it / ((long long)prm.tiles * prm.periods)) * S * CP;
+                const int y = w.grp * S * CP;
                 tc::mbar_expect_tx(b_full(q), prm.b_bytes);
                 tc::tma_load_2d(dst, &tmB, x, y, b_full(q));
                 if (prm.b_loads == 2) {
@@ -554,7 +641,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
         }
         int q = 0, rq = 0, done = 0;
         uint32_t par = 0, rpar = 0;
-        int e_row = 0, e_tile = -1;
+        int e_row = 0, e_tile = -1, e_block = -1;
         bool good = true;
         // the packed digits of this thread's 16 K entries of the stage at w,
         // which then moves on
@@ -580,12 +667,19 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(raw_empty(rq));
             } else {
-                if (w.tile != e_tile) {
-                    e_tile = w.tile;
-                    const int row = w.tile * kBM + r;
-                    e_row = row < prm.n ? __ldg(prm.rowexp + row) : kOzNonFinite;
-                }
                 const int k0 = (w.per * prm.spp + w.st) * kStageK;
+                const int block = S == 7 ? k0 / kOzBlock : 0;
+                if (w.tile != e_tile || block != e_block) {
+                    e_tile = w.tile;
+                    e_block = block;
+                    const int row = w.tile * kBM + r;
+                    e_row = kOzNonFinite;
+                    if (row < prm.n) {
+                        e_row = S == 7 ? oz_unpack_exponent(
+                                             __ldg(prm.blockexp + (size_t)block * prm.n + row))
+                                       : __ldg(prm.rowexp + row);
+                    }
+                }
                 const bool on_diag = k0 < w.tile * kBM + kBM && k0 + kStageK > w.tile * kBM;
                 asm volatile("cp.async.wait_group %0;" ::"n"(kRawStages - 1) : "memory");
 #pragma unroll
@@ -684,9 +778,30 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
         const int dcol = ((warp - kConvWarps) >> 2) * NC;
         Sums<S, NC> sums;
         sums.clear();
+        if (S == 7) pdl_wait();  // the exponents of X
         int k = 0;
+        Walk w;
+        w.start(it0, prm);
+        // S = 7: the exponents of the next item's operands (biased: two columns'
+        // per word, one word per lane), read one item ahead
+        uint32_t er_next = 0, ex_next = 0;
+        auto exponents = [&]() {
+            if (w.it >= it1) return;
+            const int block = w.per * prm.spp / (kOzBlock / kStageK);
+            const int row = min(w.tile * kBM + drow, prm.n - 1);
+            er_next = (uint32_t)__ldg(prm.blockexp + (size_t)block * prm.n + row);
+            ex_next = __ldcg(prm.xexp + (((size_t)w.grp * prm.blocks + block) * CP + dcol) / 2 +
+                             lane % (NC / 2));
+            w.skip(prm);
+        };
+        if (S == 7) exponents();
         for (long long it = it0; it < it1; ++it, ++k) {
             const int ab = k % kSets;
+            const uint32_t er = er_next | er_next << 16, ex = ex_next;
+            if constexpr (S == 7) {
+                exponents();
+                sums.raise([&](int j) { return er + __shfl_sync(0xffffffffu, ex, j); });
+            }
             // warp-uniform decision: the TMEM loads below are warp-collective
             if (!__all_sync(0xffffffffu, tc::mbar_wait(acc_full(ab), (uint32_t)((k / kSets) & 1),
                                                        err, 16, false))) {
@@ -696,25 +811,66 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t addr =
                 tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ab * V * CP + dcol);
+            auto drained = [&]() {
+                // the last columns are in registers: the MMAs of a later item
+                // may overwrite the set
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(acc_empty(ab));
+            };
+            if constexpr (S == 7) {
+                // four columns and half their levels at a time (more do not fit
+                // in the registers): the first four, which then change places
+                // with the rest.  (Unrolled, the drain's instructions crowd the
+                // converters' out of the instruction cache: 170 us instead of
+                // 157 at n = 8192, 32 columns.)
+#pragma unroll 1
+                for (int j0 = 0; j0 < NC; j0 += 4) {
+                    uint32_t v[4][4];
+                    long long hi[4];
+                    __syncwarp();  // the loads and their wait are warp-collective
 #pragma unroll
-            for (int j0 = 0; j0 < NC; j0 += 4) {
-                uint32_t v[V][4];
+                    for (int l = 0; l < 4; ++l) tmem_ld_cols(addr + (uint32_t)(l * CP + j0), v[l]);
+                    uint32_t down[2];
 #pragma unroll
-                for (int l = 0; l < V; ++l) tmem_ld_4cols(addr + (uint32_t)(l * CP + j0), v[l]);
-                tmem_ld_wait<V>(v);
-                if (j0 + 4 >= NC) {
-                    // the last columns are in registers: the MMAs of a later
-                    // item may overwrite the set
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) tc::mbar_arrive(acc_empty(ab));
+                    for (int j = 0; j < 2; ++j) {
+                        const uint32_t e = er + __shfl_sync(0xffffffffu, ex, j0 / 2 + j);
+                        down[j] = __vminu2(sums.E[j] - e, 95u | 95u << 16);
+                    }
+                    tmem_ld_wait(v);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        hi[j] = sums.combine(v[0][j], v[1][j], v[2][j], v[3][j]);
+                    }
+#pragma unroll
+                    for (int l = 0; l < 4; ++l) {
+                        tmem_ld_cols(addr + (uint32_t)((4 + l) * CP + j0), v[l]);
+                    }
+                    tmem_ld_wait(v);
+                    if (j0 + 4 >= NC) drained();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const long long lo = sums.combine(v[0][j], v[1][j], v[2][j], v[3][j]);
+                        sums.add(j, hi[j], lo,
+                                 (j & 1) != 0 ? down[j >> 1] >> 16 : down[j >> 1] & 0xFFFFu);
+                    }
+                    sums.rotate();
                 }
+            } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t lv[V];
+                for (int j0 = 0; j0 < NC; j0 += 4) {
+                    uint32_t v[V][4];
 #pragma unroll
-                    for (int l = 0; l < V; ++l) lv[l] = v[l][j];
-                    sums.add(j0 + j, lv);
+                    for (int l = 0; l < V; ++l) tmem_ld_cols(addr + (uint32_t)(l * CP + j0), v[l]);
+                    tmem_ld_wait(v);
+                    if (j0 + 4 >= NC) drained();
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        uint32_t lv[V];
+#pragma unroll
+                        for (int l = 0; l < V; ++l) lv[l] = v[l][j];
+                        sums.add(j0 + j, lv);
+                    }
                 }
             }
             const long long gt = it / prm.periods;
@@ -790,7 +946,8 @@ __global__ void oz_colmax_kernel(const double *__restrict__ X, long long ldx, in
 // along K in row (group * S + t) * cp + j of B, zero beyond n and for
 // c >= C.  Grid (padded column, K chunk); colexp[c] records the column's
 // exponent; colmax_next (may be null) is cleared for the pass that writes
-// the next block.
+// the next block.  S = 7: a warp takes a block of 128 entries, whose exponent
+// it leaves in xexp ([group][block][cp]).
 //
 // With norms.count > 0 an extra block (x = the number of padded columns)
 // finishes the norms of the update before, whose blocks only left their parts:
@@ -826,7 +983,8 @@ __global__ void __launch_bounds__(256)
 oz_slice_x_kernel(const double *__restrict__ X, long long ldx, int n, int C, int cp, int ldp,
                   const unsigned long long *__restrict__ colmax,
                   unsigned long long *__restrict__ colmax_next, __half *__restrict__ B,
-                  int *__restrict__ colexp, PendingNorms norms)
+                  int *__restrict__ colexp, uint16_t *__restrict__ xexp, int blocks,
+                  PendingNorms norms)
 {
     pdl_wait();
     const int c = blockIdx.x;
@@ -842,13 +1000,31 @@ oz_slice_x_kernel(const double *__restrict__ X, long long ldx, int n, int C, int
     const double *xc = X + (size_t)c * ldx;
     uint2 *row = reinterpret_cast<uint2 *>(B + ((size_t)(c / cp) * S * cp + c % cp) * ldp);
     const size_t stride = (size_t)cp * (size_t)ldp / 4;
-    for (int j = 4 * (blockIdx.y * blockDim.x + threadIdx.x); j < ldp;
-         j += 4 * gridDim.y * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    static_assert(kOzBlock == 4 * 32, "one block per warp");
+    for (int j0 = 4 * (blockIdx.y * blockDim.x + threadIdx.x - lane); j0 < ldp;
+         j0 += 4 * gridDim.y * blockDim.x) {
+        const int j = j0 + 4 * lane;
         double v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] = (c < C && j + u < n) ? xc[j + u] : 0.0;
-        const uint4 p0 = oz_pack_pair<S>(oz_biased_any<S>(v[0], e), oz_biased_any<S>(v[1], e));
-        const uint4 p1 = oz_pack_pair<S>(oz_biased_any<S>(v[2], e), oz_biased_any<S>(v[3], e));
+        int ev = e;
+        if (S == 7) {
+            unsigned long long m = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned long long a = abs_bits(v[u]);
+                m = a > m ? a : m;
+            }
+            ev = oz_block_exponent(warp_max(m));
+            if (lane == 0) {
+                xexp[((size_t)(c / cp) * blocks + j0 / kOzBlock) * cp + c % cp] =
+                    oz_pack_exponent(ev);
+            }
+        }
+        if (j >= ldp) continue;
+        const uint4 p0 = oz_pack_pair<S>(oz_biased_any<S>(v[0], ev), oz_biased_any<S>(v[1], ev));
+        const uint4 p1 = oz_pack_pair<S>(oz_biased_any<S>(v[2], ev), oz_biased_any<S>(v[3], ev));
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             row[(size_t)s * stride + j / 4] =
@@ -864,6 +1040,7 @@ struct Partials {
     const int *rowexp;
     const int *colexp;
     int n, cp, tiles, periods, maxslots, out;  // out: OzSplit::kOut
+    int scaled;  // S = 7: the partials are values of Delta X
     long long items, G;
     // FP64 FMAs: the partials are `maxslots` n x C blocks of H X
     int fma, C;
@@ -881,15 +1058,8 @@ __device__ __forceinline__ int slots_of(const Partials &p, int c, int tile)
            1;
 }
 
-// v 2^e; one multiplication where 2^e is a normal number.
-__device__ __forceinline__ double scale2(double v, int e)
-{
-    if (e > -1022 && e < 1023) return v * __hiloint2double((e + 1023) << 20, 0);
-    return ldexp(v, e);
-}
-
 // (Delta X)_ic from its `slots` partials, in their fixed order (finite row
-// and column scales).
+// and column).
 __device__ __forceinline__ double delta_entry(const Partials &p, int i, int c, int slots, int ei,
                                               int fc)
 {
@@ -902,7 +1072,7 @@ __device__ __forceinline__ double delta_entry(const Partials &p, int i, int c, i
     double s = 0.0;
 #pragma unroll 4
     for (int u = 0; u < slots; ++u) s += q[u * stride];
-    return scale2(s, ei + fc + p.out);
+    return p.scaled ? s : scale2(s, ei + fc + p.out);
 }
 
 // (H X)_ic from the K slices of an FP64 FMA product, in order.
@@ -1078,11 +1248,11 @@ __global__ void gap_reciprocals_kernel(const double *__restrict__ d, int n, int 
     g[(size_t)i + (size_t)j * n] = (isfinite(gap) && gap != 0.0) ? 1.0 / gap : NAN;
 }
 
-// Row maxima of |H_il| (l != i) of a column-major H, as bit patterns, and its
-// diagonal: 256 rows x `cols` columns per block, two neighbouring rows per
+// Maxima of |H_il| (l != i) over the blocks of kOzBlock columns of each row of
+// a column-major H, as bit patterns ([block][row]), and its diagonal: 256 rows x `cols` columns per block, two neighbouring rows per
 // thread (16-byte loads when n is even and H aligned), eight columns in flight.
 constexpr int kScanThreads = 128;
-constexpr int kScanCols = 64;     // columns of a block, fewer (a multiple of 8)
+constexpr int kScanCols = 64;     // columns of a block, fewer (a power of two)
 constexpr int kScanMinCols = 8;  // while the grid is small: n = 1024 16.7 -> 7.4 us
 
 template <bool VEC>
@@ -1127,53 +1297,96 @@ oz_rowmax_kernel(const double *__restrict__ H, int n, int cols,
             }
         }
     }
-    if (m0 != 0) atomicMax(rowmax + i, m0);
-    if (m1 != 0 && i + 1 < n) atomicMax(rowmax + i + 1, m1);
+    unsigned long long *out = rowmax + (size_t)(l0 / kOzBlock) * n + i;
+    if (m0 != 0) atomicMax(out, m0);
+    if (m1 != 0 && i + 1 < n) atomicMax(out + 1, m1);
 }
 
-__global__ void oz_rowexp_kernel(const unsigned long long *__restrict__ rowmax, int n,
-                                 int *__restrict__ rowexp)
+// Exponents of the rows and of their blocks: 32 rows per block, eight threads
+// each.
+__global__ void __launch_bounds__(256)
+oz_rowexp_kernel(const unsigned long long *__restrict__ rowmax, int n, int blocks,
+                 int *__restrict__ rowexp, uint16_t *__restrict__ blockexp)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) rowexp[i] = oz_exponent(rowmax[i]);
+    __shared__ unsigned long long part[8][32];
+    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * 32 + lane;
+    unsigned long long m = 0;
+    if (i < n) {
+#pragma unroll 4
+        for (int b = g; b < blocks; b += 8) {
+            const unsigned long long a = rowmax[(size_t)b * n + i];
+            m = a > m ? a : m;
+            blockexp[(size_t)b * n + i] = oz_pack_exponent(oz_block_exponent(a));
+        }
+    }
+    part[g][lane] = m;
+    __syncthreads();
+    if (g != 0 || i >= n) return;
+    for (int q = 1; q < 8; ++q) m = part[q][lane] > m ? part[q][lane] : m;
+    rowexp[i] = oz_exponent(m);
 }
 
-// Digit words of Delta from H: one block per (K stage, row tile).  Lanes run
-// along rows (coalesced reads of H); the 32 KB block is put together in
-// shared memory in its final order and written as it lies.
+// Digit words of Delta from H (words may be null): a block of threads takes
+// `stages` K stages (1 or those of a kOzBlock, while that leaves enough blocks)
+// of a row tile.  Lanes run along rows (coalesced reads of H); the 32 KB of a
+// stage are put together in shared memory in their final order and written as
+// they lie.  S = 7 counts the entries far below their block's largest,
+// below[block][row], and sets *wide where a count passes oz_range_limit.
 constexpr int kWordThreads = 512;
+constexpr int kBlockStages = kOzBlock / kStageK;
 
 template <int S>
 __global__ void __launch_bounds__(kWordThreads)
-oz_words_kernel(const double *__restrict__ H, int n, int nst, const int *__restrict__ rowexp,
-                uint4 *__restrict__ words)
+oz_words_kernel(const double *__restrict__ H, int n, int nst, int stages,
+                const int *__restrict__ rowexp, const uint16_t *__restrict__ blockexp,
+                int *__restrict__ below, int *__restrict__ wide, uint4 *__restrict__ words)
 {
     __shared__ uint4 img[kRawBytes / 16];
+    __shared__ int count[kBM];
     const int t = (int)threadIdx.x;
     const int r = t & 127;
     const int g = t >> 7;
     const int row = blockIdx.y * kBM + r;
-    const int l0 = blockIdx.x * kStageK + 8 * g;
-    double v[8];
+    const int block = blockIdx.x * stages / kBlockStages;
+    int e = S == 7 ? kOzZeroExp : kOzNonFinite;
+    if (row < n) e = S == 7 ? oz_unpack_exponent(blockexp[(size_t)block * n + row]) : rowexp[row];
+    int far = 0;
+    const int last = min((int)(blockIdx.x + 1) * stages, nst);
+    for (int st = blockIdx.x * stages; st < last; ++st) {
+        const int l0 = st * kStageK + 8 * g;
+        double v[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        const int l = l0 + u;
-        v[u] = (row < n && l < n) ? __ldcs(H + (size_t)l * n + row) : 0.0;
-    }
-    const int e = row < n ? rowexp[row] : kOzNonFinite;
+        for (int u = 0; u < 8; ++u) {
+            const int l = l0 + u;
+            v[u] = (row < n && l < n) ? __ldcs(H + (size_t)l * n + row) : 0.0;
+        }
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-        if (l0 + u == row) v[u] = 0.0;
-    }
+        for (int u = 0; u < 8; ++u) {
+            if (l0 + u == row) v[u] = 0.0;
+            else if (S == 7 && l0 + u < n && oz_far_below(v[u], e)) ++far;
+        }
+        if (words == nullptr) continue;
+        __syncthreads();  // the stage before has been written
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        img[r * 16 + ((4 * g + p) ^ (r & 7))] =
-            oz_pack_pair<S>(oz_biased_any<S>(v[2 * p], e), oz_biased_any<S>(v[2 * p + 1], e));
+        for (int p = 0; p < 4; ++p) {
+            img[r * 16 + ((4 * g + p) ^ (r & 7))] =
+                oz_pack_pair<S>(oz_biased_any<S>(v[2 * p], e), oz_biased_any<S>(v[2 * p + 1], e));
+        }
+        __syncthreads();
+        uint4 *dst = words + ((size_t)blockIdx.y * nst + st) * (kRawBytes / 16);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[q * kWordThreads + t] = img[q * kWordThreads + t];
     }
+    if (S != 7) return;
+    if (g == 0) count[r] = 0;
     __syncthreads();
-    uint4 *dst = words + ((size_t)blockIdx.y * nst + blockIdx.x) * (kRawBytes / 16);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) dst[q * kWordThreads + t] = img[q * kWordThreads + t];
+    if (far != 0) atomicAdd(count + r, far);
+    __syncthreads();
+    if (g != 0 || count[r] == 0) return;
+    int total = count[r];
+    if (stages < kBlockStages) total += atomicAdd(below + (size_t)block * n + row, total);
+    if (total > oz_range_limit(min(kOzBlock, n - block * kOzBlock), n)) *wide = 1;
 }
 
 }  // namespace oz
@@ -1191,6 +1404,7 @@ int OzMatrix::init_storage(int n_, cudaStream_t s)
 {
     n = n_;
     nst = (n + oz::kStageK - 1) / oz::kStageK;
+    blocks = (n + kOzBlock - 1) / kOzBlock;
     words_slices = 0;
     return rowexp.alloc((size_t)n, s);
 }
@@ -1206,16 +1420,34 @@ int OzMatrix::alloc_words(int slices, cudaStream_t s)
 int OzMatrix::build_words(int slices, cudaStream_t s)
 {
     const size_t tiles = (size_t)(n + oz::kBM - 1) / oz::kBM;
-    if (tiles * nst * oz::kRawBytes > kMaxWordBytes) return IPT_CUDA_SUCCESS;
-    if (alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
+    if (tiles * nst * oz::kRawBytes <= kMaxWordBytes && alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
         cudaGetLastError();  // not enough memory: the product reads H itself
         words_slices = 0;
+    }
+    DeviceBuffer<int> below;  // counts, and the flag behind them
+    // a block of threads per kOzBlock counts without atomics in memory
+    const int stages = (long long)tiles * blocks >= 4 * device_sm_count() ? oz::kBlockStages : 1;
+    const size_t counts = stages == 1 ? (size_t)blocks * n : 0;
+    if (slices == 7) {
+        IPTGB_CHECK(below.alloc(counts + 1, s));
+        IPTGB_CUDA(cudaMemsetAsync(below.ptr, 0, (counts + 1) * sizeof(int), s));
+    } else if (words_slices == 0) {
         return IPT_CUDA_SUCCESS;
     }
     auto kernel = slices == 7 ? oz::oz_words_kernel<7> : oz::oz_words_kernel<6>;
-    kernel<<<dim3((unsigned)nst, (unsigned)tiles), oz::kWordThreads, 0, s>>>(H, n, nst, rowexp.ptr,
-                                                                            words.ptr);
+    kernel<<<dim3((unsigned)((nst + stages - 1) / stages), (unsigned)tiles), oz::kWordThreads, 0,
+             s>>>(H, n, nst, stages, rowexp.ptr, blockexp.ptr, below.ptr, below.ptr + counts,
+                  words.ptr);
     IPTGB_LAUNCH();
+    if (slices != 7) return IPT_CUDA_SUCCESS;
+    int flag = 0;
+    IPTGB_CUDA(cudaMemcpyAsync(&flag, below.ptr + counts, sizeof(int), cudaMemcpyDeviceToHost, s));
+    IPTGB_CUDA(cudaStreamSynchronize(s));
+    wide = flag != 0;
+    if (wide) {
+        words.release();
+        words_slices = 0;
+    }
     return IPT_CUDA_SUCCESS;
 }
 
@@ -1224,8 +1456,10 @@ int OzMatrix::scan_rows(const double *H_, int n_, double *diag, cudaStream_t s)
     IPTGB_CHECK(init_storage(n_, s));
     H = H_;
     DeviceBuffer<unsigned long long> rm;
-    IPTGB_CHECK(rm.alloc((size_t)n, s));
-    IPTGB_CUDA(cudaMemsetAsync(rm.ptr, 0, (size_t)n * sizeof(unsigned long long), s));
+    const size_t maxima = (size_t)blocks * n;
+    IPTGB_CHECK(blockexp.alloc(maxima, s));
+    IPTGB_CHECK(rm.alloc(maxima, s));
+    IPTGB_CUDA(cudaMemsetAsync(rm.ptr, 0, maxima * sizeof(unsigned long long), s));
     const int rows = 2 * oz::kScanThreads;
     const int row_blocks = (n + rows - 1) / rows;
     int cols = oz::kScanCols;
@@ -1238,7 +1472,8 @@ int OzMatrix::scan_rows(const double *H_, int n_, double *diag, cudaStream_t s)
     auto scan = vec ? oz::oz_rowmax_kernel<true> : oz::oz_rowmax_kernel<false>;
     scan<<<grid, oz::kScanThreads, 0, s>>>(H, n, cols, rm.ptr, diag);
     IPTGB_LAUNCH();
-    oz::oz_rowexp_kernel<<<blocks_for((size_t)n), kThreads, 0, s>>>(rm.ptr, n, rowexp.ptr);
+    oz::oz_rowexp_kernel<<<(n + 31) / 32, 256, 0, s>>>(rm.ptr, n, blocks, rowexp.ptr,
+                                                       blockexp.ptr);
     IPTGB_LAUNCH();
     return IPT_CUDA_SUCCESS;
 }
@@ -1335,14 +1570,16 @@ int OzProduct::shape_for(int C)
     q.ldp = (n + 63) / 64 * 64;
     // Items of kOzPeriod K elements, or (56-bit split, whose sums do not depend
     // on it) half or a quarter of that while it shortens the longest CTA: a
-    // matrix of a few tiles then spreads over more SMs
+    // matrix of a few tiles then spreads over more SMs.  An item's drain takes
+    // about as long as three stages (6400 cycles) beside the MMAs of the next.
     const int nst = (n + oz::kStageK - 1) / oz::kStageK;
     long long best = LLONG_MAX;
     for (int spp = oz::kMaxStagesPerItem; spp >= (slices == 7 ? 1 : oz::kMaxStagesPerItem);
          spp /= 2) {
         const int periods = (nst + spp - 1) / spp;
         const long long items = (long long)q.groups * q.tiles * periods;
-        const long long longest = (items + sms - 1) / sms * spp;
+        const long long longest =
+            (items + sms - 1) / sms * (slices == 7 ? std::max(spp, 3) : spp);
         if (longest >= best) continue;
         best = longest;
         q.spp = spp;
@@ -1362,6 +1599,9 @@ int OzProduct::shape_for(int C)
     const size_t cneed = (size_t)q.groups * q.cp;
     if (B.count < bneed) IPTGB_CHECK(B.alloc(bneed, s));
     if (colexp.count < cneed) IPTGB_CHECK(colexp.alloc(cneed, s));
+    if (slices == 7 && xexp.count < cneed * m->blocks) {
+        IPTGB_CHECK(xexp.alloc(cneed * m->blocks, s));
+    }
     if (colmax.count < 2 * cneed) IPTGB_CHECK(colmax.alloc(2 * cneed, s));
     if (P.count < pneed) IPTGB_CHECK(P.alloc(pneed, s));
     cur = 0;
@@ -1388,12 +1628,15 @@ int OzProduct::slice_and_multiply(const double *X, long long ldx, int clear_othe
                            X, ldx, q.n, q.C, q.cp, q.ldp,
                            (const unsigned long long *)(colmax.ptr + cur * set),
                            clear_other ? colmax.ptr + (1 - cur) * set : nullptr, B.ptr,
-                           colexp.ptr, norms));
+                           colexp.ptr, xexp.ptr, m->blocks, norms));
     pending_count = 0;
     oz::Params prm = {};
     prm.H = m->H;
     prm.words = m->words.ptr;
     prm.rowexp = m->rowexp.ptr;
+    prm.blockexp = m->blockexp.ptr;
+    prm.xexp = reinterpret_cast<const uint32_t *>(xexp.ptr);
+    prm.blocks = m->blocks;
     prm.n = q.n;
     prm.groups = q.groups;
     prm.tiles = q.tiles;
@@ -1423,7 +1666,8 @@ oz::Partials OzProduct::partials() const
     p.tiles = sh.tiles;
     p.periods = sh.periods;
     p.maxslots = sh.maxslots;
-    p.out = slices == 7 ? OzSplit<7>::kOut : OzSplit<6>::kOut;
+    p.out = OzSplit<6>::kOut;
+    p.scaled = slices == 7;
     p.items = sh.items;
     p.G = sh.grid;
     p.err = err.ptr;

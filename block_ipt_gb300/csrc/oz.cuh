@@ -12,7 +12,8 @@
 //  * every row i of Delta is scaled by 2^-e_i, e_i the smallest exponent
 //    with max_j |Delta_ij| < 2^e_i, and rounded to the fixed-point integer
 //    Q_ij = round(Delta_ij 2^(F - e_i)); every column c of X likewise with
-//    its own exponent f_c;
+//    its own exponent f_c (S = 7: every block of 128 entries of a row or
+//    column has its own);
 //  * Q is written in S balanced base-256 digits, Q = sum_s A_s 256^(S-1-s),
 //    A_s in [-128, 127] for s > 0: small integers that FP16 holds exactly;
 //  * the level sums L_l = sum_{s+t=l} A_s B_t are kept for l < V, the
@@ -27,12 +28,17 @@
 //    2^-47 of the fixed-point scale; drains are combined in double-float
 //    arithmetic.
 //  * S = 7, F = 56, V = 8, rounded toward zero (the plain FP64 path): 56 bits
-//    hold every bit of a double within three binades of the row's largest
-//    entry; the errors are the truncation of the operands below 2^-56 of
-//    their row's (column's) scale and the dropped products, each below 2^-64
-//    of the product of the scales.  Levels 0 to 5 stay within 2^24 and add
-//    exactly; a level sum 6 or 7 beyond it may round by one unit, 2^-64 of
-//    the scale.  Drains are added in 64-bit integers, exactly.
+//    hold every bit of a double within three binades of the largest entry of
+//    its block (kOzBlock); the errors are the truncation of the operands
+//    below 2^-56 of their block's scale and the dropped products, each below
+//    2^-64 of the product of the scales.  Levels 0 to 5 stay within 2^24 and
+//    add exactly; a level sum 6 or 7 beyond it may round by one unit, 2^-64
+//    of the scale.  Drains are added as 96-bit integers at the largest scale
+//    so far, cut off below 2^-72 of it.  Over one block an entry of Delta X
+//    is off by up to 128 2^-54 max|Delta_il| max|X_lc|, where FP64 FMAs are
+//    off by a few 2^-53 sum |Delta_il X_lc|: the same where the entries of a
+//    row of Delta do not span many binades within a block.  oz_range_limit
+//    is the line beyond which a matrix is multiplied in FP64 FMAs.
 //
 // The rounding to Q and the digit extraction use integer operations only
 // (GB300 runs FP64 arithmetic at 1/64 of the FP32 rate).
@@ -44,6 +50,8 @@ namespace iptgb {
 
 constexpr int kOzSlices = 6;      // digits per operand of the 48-bit split
 constexpr int kOzPeriod = 128;    // K elements between accumulator drains
+constexpr int kOzBlock = 128;     // S = 7: K elements of a row or column that share an exponent
+static_assert(kOzBlock % kOzPeriod == 0, "a drain's K elements share their exponents");
 
 // S slices: F fixed-point bits, V digit-product levels kept, the bias that
 // makes the low S - 1 digits unsigned bytes and puts the top digit, as the
@@ -64,6 +72,8 @@ struct OzSplit<7> {
 // Row / column exponent of a row that holds Inf or NaN: the product of that
 // row (column) is NaN.
 constexpr int kOzNonFinite = 0x7fffffff;
+// Exponent of a block of zeros (S = 7): below every other.
+constexpr int kOzZeroExp = -8192;
 
 #if defined(__CUDACC__)
 #define OZ_HD __host__ __device__ __forceinline__
@@ -85,6 +95,52 @@ OZ_HD int oz_exponent(uint64_t absbits)
         return p + 1 - 1074;
     }
     return E - 1022;  // 1.f * 2^(E - 1023) < 2^(E - 1022)
+}
+
+// The same for a block of kOzBlock entries.
+OZ_HD int oz_block_exponent(uint64_t absbits)
+{
+    return absbits == 0 ? kOzZeroExp : oz_exponent(absbits);
+}
+
+// A block's exponent as the product kernel keeps it: 16 bits, biased so that a
+// sum of two is positive and below 2^15.  A block that is not finite has zero
+// digits, as one of zeros (its row or column is not taken from the product).
+OZ_HD uint16_t oz_pack_exponent(int e)
+{
+    return (uint16_t)(e == kOzNonFinite ? 0 : e - kOzZeroExp);
+}
+
+OZ_HD int oz_unpack_exponent(uint16_t p)
+{
+    return (int)p + kOzZeroExp;
+}
+
+// Does an entry lie more than six binades below its block's largest, of
+// exponent e?
+OZ_HD bool oz_far_below(double v, int e)
+{
+    uint64_t b;
+#if defined(__CUDA_ARCH__)
+    b = (uint64_t)__double_as_longlong(v);
+#else
+    __builtin_memcpy(&b, &v, sizeof(b));
+#endif
+    return (int)((b >> 52) & 0x7FFu) + 6 < e + 1022;
+}
+
+// The number of off-diagonal entries of a block that may lie that far below
+// (of its `count` columns, in a matrix of n): 3/8 of them, 8 more in the short
+// block at the end of a longer row.  Median relative errors of the vectors'
+// entries after 8 steps, k = 8, FP64 FMAs | this split: couplings N(0,1) with
+// a decay of exp(-|i-j|/64), n = 1500 (28 % below in the worst block) 9e-16 |
+// 6e-16; graded (d from 1 to 1e20, couplings ~ sqrt(d_i d_j)), n = 1024 (30 %)
+// 8e-16 | 1e-15; beyond the line, graded 1 to 1e12, n = 300 (63 %) 4e-16 |
+// 2e-14; decay exp(-|i-j|/16) (76 %) 8e-16 | 9e-14; tridiagonal: the small
+// entries are lost.
+OZ_HD int oz_range_limit(int count, int n)
+{
+    return 3 * count / 8 + (count < kOzBlock && n > kOzBlock ? 8 : 0);
 }
 
 // The F-bit fixed-point value round(v 2^(F - e)) (round half away from

@@ -21,8 +21,13 @@ struct OzMatrix {
     const double *H = nullptr;
     int n = 0;
     int nst = 0;           // 32-element K stages of a row
+    int blocks = 0;        // kOzBlock-element blocks of a row
     int words_slices = 0;  // digits per entry in `words` (0: none)
+    // build_words(7): entries of a row span more binades within a block than
+    // the 56-bit split multiplies as accurately as FP64 FMAs (oz_range_limit)
+    bool wide = false;
     DeviceBuffer<int> rowexp;
+    DeviceBuffer<uint16_t> blockexp;  // [block][row], oz_pack_exponent
     DeviceBuffer<uint4> words;  // oz_word_index
     // H alone, for products in FP64 FMAs
     void reference(const double *H, int n);
@@ -34,7 +39,8 @@ struct OzMatrix {
     int scan_rows(const double *H, int n, double *diag, cudaStream_t s);
     // digit words from a second pass (for matrices multiplied more than once
     // or twice); without an error none where they exceed kMaxWordBytes or the
-    // device's memory
+    // device's memory.  slices = 7: finds out whether the matrix is `wide`
+    // (and waits for that); a wide one gets no words.
     int build_words(int slices, cudaStream_t s);
 };
 
@@ -53,7 +59,7 @@ struct OzShape {
 
 // Y = (diag(d) + Delta) X for an n x C block X (column-major, ld ldx); d may
 // be null (Y = Delta X).  slices = 6: the 48-bit split; 7: the 56-bit split
-// of the plain FP64 path (oz.cuh); 0: no split, FP64 FMAs (k_dense64.cu; step()
+// of the plain FP64 path (oz.cuh), for matrices that are not `wide`; 0: no split, FP64 FMAs (k_dense64.cu; step()
 // only).
 namespace oz {
 struct Partials;
@@ -67,6 +73,7 @@ struct OzProduct {
     OzShape sh;
     DeviceBuffer<__half> B;
     DeviceBuffer<int> colexp;
+    DeviceBuffer<uint16_t> xexp;  // slices = 7: [group][block][cp], oz_pack_exponent
     DeviceBuffer<unsigned long long> colmax;  // two sets of C column maxima
     int cur = 0;                              // the set the next product reads
     // deferred norms of the last step: parts, their number (0: none), target

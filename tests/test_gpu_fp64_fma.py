@@ -31,12 +31,12 @@ def graded(n, decades, seed):
     return H
 
 
-def fixed_point(H, k, steps):
+def fixed_point(H, k, steps, X=None):
     L = H.astype(np.longdouble)
     n = H.shape[0]
     d = np.diag(L).copy()
     D = L - np.diag(d)
-    X = np.eye(n, k, dtype=np.longdouble)
+    X = np.eye(n, k, dtype=np.longdouble) if X is None else X
     gap = d[None, :k] - d[:, None]
     gap[np.arange(k), np.arange(k)] = 1
     for _ in range(steps):
