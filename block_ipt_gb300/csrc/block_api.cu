@@ -169,6 +169,7 @@ struct Fp64Stage final : IptStage {
         }
         scratch.release(s);
         if (status != IPT_CUDA_SUCCESS) return status;
+        IPTGB_CHECK(op->check());
         if (x != X) {
             IPTGB_CUDA(cudaMemcpyAsync(X, x, elems * sizeof(double), cudaMemcpyDeviceToDevice, s));
         }
@@ -669,7 +670,9 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         // (lowp.h set_mixing; tuning knob IPT_GB300_ANDERSON=0 turns it off)
         rin.mixing = lowp != nullptr && env_int("IPT_GB300_ANDERSON", 1) != 0;
         if (lowp) lowp->set_mixing(rin.mixing);
-        IPTGB_CHECK(refine_solve(rin, xout, d_values, report, s, &conv, Xfb.ptr));
+        st = refine_solve(rin, xout, d_values, report, s, &conv, Xfb.ptr);
+        if (st != IPT_CUDA_SUCCESS && apply.oz != nullptr) IPTGB_CHECK(ozp.check());
+        IPTGB_CHECK(st);
         if (lowp) lowp->set_mixing(false);
         done = conv;
     }
@@ -691,7 +694,12 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
             in.initial = Xfb.ptr;
             in.initial_cols = k;
         }
-        IPTGB_CHECK(block_solve(in, xout, d_values, report, s));
+        st = block_solve(in, xout, d_values, report, s);
+        // a product that failed leaves NaN, which no solve certifies
+        if ((st != IPT_CUDA_SUCCESS || !report->converged) && apply.oz != nullptr) {
+            IPTGB_CHECK(ozp.check());
+        }
+        IPTGB_CHECK(st);
         if (Xfb.ptr != nullptr) {
             report->ipt_iterations += first.ipt_iterations;
             report->lowp_matvecs += first.lowp_matvecs;

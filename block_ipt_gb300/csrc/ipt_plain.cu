@@ -219,6 +219,7 @@ int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, 
         for (int iter = 0; iter < maxiter; ++iter) {
             IPTGB_CHECK(op.step(X[iter & 1], X[(iter + 1) & 1], d, 0, &scratch->ns));
         }
+        IPTGB_CHECK(op.check());
         *X_final = X[maxiter & 1];
         *iterations_done = maxiter;
         *fixed_point_residual = NAN;
@@ -280,6 +281,8 @@ int run_plain_ipt(Fp64Operator &op, int n, int k, const double *d, int maxiter, 
         }
     }
     scratch->ns.norms = device_norms;
+    // (a step that failed leaves no finite norms)
+    if (status == IPT_CUDA_INVALID_ARGUMENT) IPTGB_CHECK(op.check());
     IPTGB_CHECK(status);
     *X_final = X[done & 1];
     *iterations_done = done;

@@ -25,6 +25,8 @@ struct Fp64Operator {
         return step(X, Xn, d, 1, ns);
     }
     virtual int flush_norms() { return IPT_CUDA_SUCCESS; }
+    // waits for the steps and reports one that failed (its block is NaN)
+    virtual int check() { return IPT_CUDA_SUCCESS; }
     // values[j] = (H X)_jj.
     virtual int diag_values(const double *X, double *values) = 0;
 };
@@ -65,6 +67,7 @@ struct DenseFp64Operator final : Fp64Operator {
              NormScratch *ns) override;
     int step_ahead(const double *X, double *Xn, const double *d, NormScratch *ns) override;
     int flush_norms() override { return product.flush_norms(); }
+    int check() override { return product.check(); }
     int diag_values(const double *X, double *values) override;
 };
 

@@ -459,7 +459,8 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
             result->max_residual = mx;
             const double dn = host[(size_t)k], xn = host[(size_t)k + 1];
             if (!(xn > 0.0) || !isfinite(xn)) {
-                status = ACX_CUDA_INVALID_ARGUMENT;
+                // (a product that failed leaves no finite norms either)
+                if (lib_ok(F.product.check())) status = ACX_CUDA_INVALID_ARGUMENT;
                 break;
             }
             result->fixed_point_residual = dn / xn;
@@ -491,7 +492,9 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                                         cudaMemcpyDeviceToDevice, s));
             }
             lib_ok(launch_dense64_diag_values(H, n, n, f1, k, values, s));
-            cuda_ok(cudaStreamSynchronize(s));
+            // waits for the stream
+            if (result->converged || F.product.slices == 0) cuda_ok(cudaStreamSynchronize(s));
+            else lib_ok(F.product.check());
         }
         result->finalization_time_sec = seconds_since(t_fin);
     }

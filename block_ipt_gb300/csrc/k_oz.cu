@@ -109,6 +109,7 @@ struct Params {
     int stream_h;    // H is read past L2 (evict first)
     int b_loads;     // TMA boxes per B stage
     uint32_t b_bytes;
+    long long spin;  // polls of a pipeline wait before it gives up
 };
 
 template <int S, int CP>
@@ -483,7 +484,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             Walk w;
             w.start(it0, prm);
             while (w.it < it1 && !abort_flag) {
-                if (issued >= kBStages && !tc::mbar_wait(b_empty(q), par ^ 1u, err, 12, false)) {
+                if (issued >= kBStages && !tc::mbar_wait(b_empty(q), par ^ 1u, err, 12, false, prm.spin)) {
                     abort_flag = 1;
                     break;
                 }
@@ -517,7 +518,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             w.start(it0, prm);
             while (w.it < it1 && !abort_flag) {
                 if (issued >= kRawStages &&
-                    !tc::mbar_wait(raw_empty(q), par ^ 1u, err, 10, false)) {
+                    !tc::mbar_wait(raw_empty(q), par ^ 1u, err, 10, false, prm.spin)) {
                     abort_flag = 1;
                     break;
                 }
@@ -549,7 +550,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             const int use = k / kSets;
             if (use > 0) {
                 ok = __all_sync(0xffffffffu, tc::mbar_wait(acc_empty(ab), (uint32_t)((use - 1) & 1),
-                                                           err, 13, false));
+                                                           err, 13, false, prm.spin));
                 if (!ok) break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -557,8 +558,8 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             const long long item = w.it;
             bool first = true;
             while (w.it == item) {
-                ok = tc::mbar_wait(b_full(bq), bpar, err, 14, false) &&
-                     tc::mbar_wait(a_full(q), par, err, 15, false);
+                ok = tc::mbar_wait(b_full(bq), bpar, err, 14, false, prm.spin) &&
+                     tc::mbar_wait(a_full(q), par, err, 15, false, prm.spin);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -647,7 +648,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
         // which then moves on
         auto load = [&](uint4 (&x)[8]) {
             if (MODE == kWords) {
-                if (!__all_sync(0xffffffffu, tc::mbar_wait(raw_full(rq), rpar, err, 9, false))) {
+                if (!__all_sync(0xffffffffu, tc::mbar_wait(raw_full(rq), rpar, err, 9, false, prm.spin))) {
                     good = false;
                     return;
                 }
@@ -727,7 +728,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
         // of K per slice and K group
         auto emit = [&](const uint4 (&x)[8]) {
             if (done >= kStages &&
-                !__all_sync(0xffffffffu, tc::mbar_wait(a_empty(q), par ^ 1u, err, 11, false))) {
+                !__all_sync(0xffffffffu, tc::mbar_wait(a_empty(q), par ^ 1u, err, 11, false, prm.spin))) {
                 good = false;
                 return;
             }
@@ -804,7 +805,7 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
             }
             // warp-uniform decision: the TMEM loads below are warp-collective
             if (!__all_sync(0xffffffffu, tc::mbar_wait(acc_full(ab), (uint32_t)((k / kSets) & 1),
-                                                       err, 16, false))) {
+                                                       err, 16, false, prm.spin))) {
                 abort_flag = 1;
                 break;
             }
@@ -1172,7 +1173,10 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
         for (int l = 0; l < n; ++l) y = fma(H[(size_t)r + (size_t)l * n], xc[l], y);
         return y - d[r] * xc[r];
     };
+    // a product that failed gives NaN, not a sum over its NaN block per entry
+    const bool failed = *p.err != 0;
     auto delta = [&](int r, int count) {
+        if (failed) return (double)NAN;
         if (p.fma) return fma(-d[r], xc[r], fma_entry(p, r, c));
         const int er = p.rowexp[r];
         return (er == kOzNonFinite || fc == kOzNonFinite) ? direct(r)
@@ -1195,7 +1199,6 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
     }
     __syncthreads();
     const double cj = cj_sh;
-    const bool failed = *p.err != 0;
     double dsq = 0.0, xsq = 0.0, rsq = 0.0;
     unsigned long long m = 0;
     const double hcc = RESID ? fma(d[c], xc[c], cj) : 0.0;  // (H X)_cc
@@ -1543,6 +1546,8 @@ int OzProduct::bind(const OzMatrix *matrix, const double *diag, int digit_slices
     s = stream;
     slices = digit_slices;
     sms = device_sm_count();
+    const int limit = env_int("IPT_GB300_SPIN_LIMIT", 0);
+    spin = limit > 0 ? limit : tc::kSpinLimit;
     if (err.ptr == nullptr) {
         IPTGB_CHECK(err.alloc(1, s));
         IPTGB_CUDA(cudaMemsetAsync(err.ptr, 0, sizeof(int), s));
@@ -1648,6 +1653,7 @@ int OzProduct::slice_and_multiply(const double *X, long long ldx, int clear_othe
     prm.stream_h = (size_t)q.n * q.n * sizeof(double) > oz::kL2ResidentBytes;
     prm.b_loads = slices * q.cp <= 256 ? 1 : 2;
     prm.b_bytes = (uint32_t)(slices * q.cp * 64);
+    prm.spin = spin;
     auto launch = m->words_slices == slices ? launch_product_for<oz::kWords>
                                             : launch_product_for<oz::kRows>;
     return launch(slices, q.cp, mapB, prm, q.grid, P.ptr, err.ptr, s);
@@ -1750,6 +1756,16 @@ int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms
     }
     cur = 1 - cur;
     return IPT_CUDA_SUCCESS;
+}
+
+int OzProduct::check()
+{
+    if (err.ptr == nullptr || slices == 0) return IPT_CUDA_SUCCESS;
+    int code = 0;
+    IPTGB_CHECK(read_error(&code));
+    if (code == 0) return IPT_CUDA_SUCCESS;
+    fprintf(stderr, "ipt_gb300: FP64-accurate product: pipeline wait %d gave up\n", code);
+    return IPT_CUDA_CUDA_ERROR;
 }
 
 int OzProduct::read_error(int *host_err)

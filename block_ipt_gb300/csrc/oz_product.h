@@ -107,8 +107,15 @@ struct OzProduct {
         return slices == 0 ? nullptr : colmax.ptr + (size_t)cur * sh.groups * sh.cp;
     }
 
-    // the kernel's error flag (non-zero: a bounded wait gave up)
+    // polls of a pipeline wait before the kernel gives up (tuning and test knob
+    // IPT_GB300_SPIN_LIMIT; the drain before TMEM is released always uses the
+    // full bound)
+    long long spin = 0;
+    // the kernel's error flag (non-zero: a bounded wait gave up); waits for the
+    // stream
     int read_error(int *host_err);
+    // IPT_CUDA_CUDA_ERROR where it is set, as the results are then NaN
+    int check();
 
   private:
     int shape_for(int C);
