@@ -1423,7 +1423,8 @@ int OzMatrix::alloc_words(int slices, cudaStream_t s)
 int OzMatrix::build_words(int slices, cudaStream_t s)
 {
     const size_t tiles = (size_t)(n + oz::kBM - 1) / oz::kBM;
-    if (tiles * nst * oz::kRawBytes <= kMaxWordBytes && alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
+    const size_t most = (size_t)env_int("IPT_GB300_WORDS_MAX_MB", kMaxWordMb) << 20;
+    if (tiles * nst * oz::kRawBytes <= most && alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
         cudaGetLastError();  // not enough memory: the product reads H itself
         words_slices = 0;
     }

@@ -38,14 +38,16 @@ struct OzMatrix {
     // its diagonal
     int scan_rows(const double *H, int n, double *diag, cudaStream_t s);
     // digit words from a second pass (for matrices multiplied more than once
-    // or twice); without an error none where they exceed kMaxWordBytes or the
+    // or twice); without an error none where they exceed kMaxWordMb or the
     // device's memory.  slices = 7: finds out whether the matrix is `wide`
     // (and waits for that); a wide one gets no words.
     int build_words(int slices, cudaStream_t s);
 };
 
-// n up to 46340; the words go back to the stream-ordered pool after a solve.
-constexpr size_t kMaxWordBytes = (size_t)16 << 30;
+// The most memory the words may take, MB (n up to 46340); they go back to the
+// stream-ordered pool after a solve.  Tuning and test knob IPT_GB300_WORDS_MAX_MB
+// (0: the product always extracts the digits itself).
+constexpr int kMaxWordMb = 16384;
 
 // Launch shape of a product with C columns: `groups` column groups of cp
 // columns; the work items (group, 128-row tile, period of K elements) are
