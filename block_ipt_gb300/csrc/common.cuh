@@ -139,6 +139,21 @@ struct KernelTimerScope {
 // so repeated solves reuse their scratch; once per device and process.
 void retain_pool_memory();
 
+// Memory that the calling thread's solves hold only to be faster (the digit
+// words of OzMatrix) goes back, in stream order; false where there is none.
+bool reclaim_memory(cudaStream_t s);
+
+// cudaMallocAsync, once more after reclaim_memory() where it fails.
+inline cudaError_t device_malloc(void **p, size_t bytes, cudaStream_t s)
+{
+    cudaError_t e = cudaMallocAsync(p, bytes, s);
+    if (e == cudaErrorMemoryAllocation && reclaim_memory(s)) {
+        cudaGetLastError();
+        e = cudaMallocAsync(p, bytes, s);
+    }
+    return e;
+}
+
 template <typename T>
 struct DeviceBuffer {
     T *ptr = nullptr;
@@ -157,7 +172,7 @@ struct DeviceBuffer {
         if (n == 0) {
             return IPT_CUDA_SUCCESS;
         }
-        cudaError_t e = cudaMallocAsync((void **)&ptr, n * sizeof(T), s);
+        cudaError_t e = device_malloc((void **)&ptr, n * sizeof(T), s);
         if (e != cudaSuccess) {
             ptr = nullptr;
             count = 0;

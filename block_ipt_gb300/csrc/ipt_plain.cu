@@ -90,9 +90,9 @@ int CsrFp64Operator::diag_values(const double *X, double *values)
 int SolveScratch::init(size_t max_elems, cudaStream_t stream)
 {
     const int slots = blocks_for(max_elems);
-    IPTGB_CUDA(cudaMallocAsync((void **)&ns.partials, (size_t)slots * sizeof(double2), stream));
+    IPTGB_CUDA(device_malloc((void **)&ns.partials, (size_t)slots * sizeof(double2), stream));
     // [counter u32 | pad][norms double x2]
-    IPTGB_CUDA(cudaMallocAsync((void **)&ns.counter, 32, stream));
+    IPTGB_CUDA(device_malloc((void **)&ns.counter, 32, stream));
     ns.norms = (double *)((char *)ns.counter + 16);
     ns.capacity = slots;
     IPTGB_CUDA(cudaMemsetAsync(ns.counter, 0, 16, stream));
@@ -110,7 +110,7 @@ int SolveScratch::arm_history(int steps, double tol, cudaStream_t stream)
         if (ns.hist != nullptr) cudaFreeAsync(ns.hist, stream);
         ns.hist = nullptr;
         ns.hist_cap = 0;
-        IPTGB_CUDA(cudaMallocAsync((void **)&ns.hist, 2 * (size_t)steps * sizeof(double), stream));
+        IPTGB_CUDA(device_malloc((void **)&ns.hist, 2 * (size_t)steps * sizeof(double), stream));
         ns.hist_cap = steps;
     }
     IPTGB_CUDA(cudaMemsetAsync(ns.hist, 0, 2 * (size_t)steps * sizeof(double), stream));

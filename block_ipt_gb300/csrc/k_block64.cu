@@ -985,7 +985,7 @@ int BlockOps::ensure_partials(size_t count)
         partials = nullptr;
     }
     size_t want = count < (size_t)1 << 16 ? (size_t)1 << 16 : count;
-    IPTGB_CUDA(cudaMallocAsync((void **)&partials, want * sizeof(double), stream));
+    IPTGB_CUDA(device_malloc((void **)&partials, want * sizeof(double), stream));
     partials_capacity = want;
     return IPT_CUDA_SUCCESS;
 }

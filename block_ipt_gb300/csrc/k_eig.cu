@@ -973,7 +973,7 @@ int BlockOps::symmetric_eig(const double *T, int m, double *w, double *Z, int *i
             cudaFreeAsync(eig_scratch, stream);
             eig_scratch = nullptr;
         }
-        IPTGB_CUDA(cudaMallocAsync((void **)&eig_scratch, need * sizeof(double), stream));
+        IPTGB_CUDA(device_malloc((void **)&eig_scratch, need * sizeof(double), stream));
         eig_capacity = need;
     }
     double *Tp = eig_scratch;

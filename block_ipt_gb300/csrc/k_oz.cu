@@ -1420,6 +1420,39 @@ int OzMatrix::alloc_words(int slices, cudaStream_t s)
     return IPT_CUDA_SUCCESS;
 }
 
+namespace {
+// the matrices of this thread whose words may be taken back
+thread_local OzMatrix *t_held = nullptr;
+}  // namespace
+
+bool reclaim_memory(cudaStream_t s)
+{
+    bool any = false;
+    for (OzMatrix *m = t_held; m != nullptr; m = m->held_before) any = m->drop_words(s) || any;
+    return any;
+}
+
+bool OzMatrix::drop_words(cudaStream_t s)
+{
+    if (words.ptr == nullptr) return false;
+    const cudaStream_t owner = words.stream;
+    words.release();
+    words_slices = 0;
+    // memory freed on one stream serves another one once that has got there
+    if (owner != s) cudaStreamSynchronize(owner);
+    return true;
+}
+
+OzMatrix::~OzMatrix()
+{
+    if (!listed) return;
+    for (OzMatrix **p = &t_held; *p != nullptr; p = &(*p)->held_before) {
+        if (*p != this) continue;
+        *p = held_before;
+        break;
+    }
+}
+
 int OzMatrix::build_words(int slices, cudaStream_t s)
 {
     const size_t tiles = (size_t)(n + oz::kBM - 1) / oz::kBM;
@@ -1427,6 +1460,11 @@ int OzMatrix::build_words(int slices, cudaStream_t s)
     if (tiles * nst * oz::kRawBytes <= most && alloc_words(slices, s) != IPT_CUDA_SUCCESS) {
         cudaGetLastError();  // not enough memory: the product reads H itself
         words_slices = 0;
+    }
+    if (!listed) {
+        held_before = t_held;
+        t_held = this;
+        listed = true;
     }
     DeviceBuffer<int> below;  // counts, and the flag behind them
     // a block of threads per kOzBlock counts without atomics in memory

@@ -29,6 +29,8 @@ struct OzMatrix {
     DeviceBuffer<int> rowexp;
     DeviceBuffer<uint16_t> blockexp;  // [block][row], oz_pack_exponent
     DeviceBuffer<uint4> words;  // oz_word_index
+    OzMatrix() = default;
+    ~OzMatrix();
     // H alone, for products in FP64 FMAs
     void reference(const double *H, int n);
     int init_storage(int n, cudaStream_t s);
@@ -41,7 +43,12 @@ struct OzMatrix {
     // or twice); without an error none where they exceed kMaxWordMb or the
     // device's memory.  slices = 7: finds out whether the matrix is `wide`
     // (and waits for that); a wide one gets no words.
+    // Until the object goes, an allocation of this thread that fails takes the
+    // words' memory (reclaim_memory): the products then read H.
     int build_words(int slices, cudaStream_t s);
+    bool drop_words(cudaStream_t s);
+    OzMatrix *held_before = nullptr;  // the thread's list of matrices with words
+    bool listed = false;
 };
 
 // The most memory the words may take, MB (n up to 46340); they go back to the
