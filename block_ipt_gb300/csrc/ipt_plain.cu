@@ -4,6 +4,7 @@
 
 #include "common.cuh"
 #include "ipt_plain.h"
+#include "thread_slots.h"
 
 namespace iptgb {
 
@@ -158,23 +159,21 @@ void SolveScratch::release(cudaStream_t stream)
 namespace {
 
 // Per host thread: two page-locked slots of two norms each that the update
-// kernels of alternate steps write directly (allocated on the thread's first
-// tolerance-stopped solve and kept for the life of the process).
+// kernels of alternate steps write directly (taken on the thread's first
+// tolerance-stopped solve and handed on to another thread when it ends).
 constexpr int kNormSlots = 2;
 
-double *pinned_norm_slots()
+double *make_norm_slots()
 {
-    static thread_local double *buf = nullptr;
-    if (buf == nullptr) {
-        void *p = nullptr;
-        if (cudaMallocHost(&p, 2 * kNormSlots * sizeof(double)) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        buf = static_cast<double *>(p);
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, 2 * kNormSlots * sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    return buf;
+    return static_cast<double *>(p);
 }
+
+double *pinned_norm_slots() { return ThreadSlots<double>::mine(make_norm_slots); }
 
 // A NaN no kernel produces marks a slot as not yet written.
 constexpr uint64_t kNormPending = 0x7FF45EED00000001ULL;
