@@ -15,7 +15,7 @@
 // and the two Frobenius norms in the same pass); an extrapolation step is two
 // launches over (row blocks, columns), the inner products and the update.  The
 // host reads k + 3 values per step.  The map's denominator test only depends
-// on the diagonal: it is made once, with the gap reciprocals.
+// on the diagonal: it is made once.
 #include <cublas_v2.h>
 #include <float.h>
 #include <math.h>
@@ -37,18 +37,12 @@ namespace iptgb {
 constexpr int kAcxThreads = 256;
 constexpr int kAcxNormBlocks = 256;
 
-// g_ic = 1 / (d_c - d_i) of the ACX map, 0 and the flag where |d_c - d_i| <=
-// DBL_EPSILON (acx_cuda.cu:109-172).
-__global__ void acx_gaps_kernel(const double *__restrict__ d, int n, double *__restrict__ g,
-                                int *__restrict__ flag)
+// The flag where |d_c - d_i| <= DBL_EPSILON for an i != c (acx_cuda.cu:109-172).
+__global__ void acx_gaps_kernel(const double *__restrict__ d, int n, int *__restrict__ flag)
 {
     const int c = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double den = d[c] - d[i];
-    const bool zero = fabs(den) <= DBL_EPSILON;
-    g[(size_t)i + (size_t)c * n] = zero ? 0.0 : 1.0 / den;
-    if (zero && i != c) atomicOr(flag, 1);
+    if (i < n && i != c && fabs(d[c] - d[i]) <= DBL_EPSILON) atomicOr(flag, 1);
 }
 
 // resid[c] = ||(H X)_c - X_c (H X)_cc|| from the update's parts, in order.
@@ -305,7 +299,6 @@ namespace {
 struct AcxDense {
     OzMatrix matrix;
     OzProduct product;
-    DeviceBuffer<double> g;      // gap reciprocals, n x k
     DeviceBuffer<double> rpart;  // residual parts of the last norms step
     NormScratch ns;
     int n = 0, k = 0, row_blocks = 0;
@@ -315,7 +308,7 @@ struct AcxDense {
     // of X.  The column maxima of X are those of the last Y (or begin()).
     int apply(const double *X, double *Y, bool norms)
     {
-        IPTGB_CHECK(product.step(X, g.ptr, Y, norms, &ns, norms ? rpart.ptr : nullptr));
+        IPTGB_CHECK(product.step(X, nullptr, Y, norms, &ns, norms ? rpart.ptr : nullptr));
         if (!norms) return IPT_CUDA_SUCCESS;
         return launch_pdl(acx_resid_kernel, dim3(blocks_for((size_t)k)), dim3(kThreads), 0, s,
                           (const double *)rpart.ptr, row_blocks, k, resid);
@@ -392,7 +385,6 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                   part.alloc((size_t)F.row_blocks * k, s) == IPT_CUDA_SUCCESS &&
                   ext.alloc((size_t)ext_blocks * k, s) == IPT_CUDA_SUCCESS &&
                   F.rpart.alloc((size_t)F.row_blocks * k, s) == IPT_CUDA_SUCCESS &&
-                  F.g.alloc(elems, s) == IPT_CUDA_SUCCESS &&
                   flags.alloc(2, s) == IPT_CUDA_SUCCESS;
         if (!ok) status = ACX_CUDA_ALLOCATION_FAILED;
         double *d = small.ptr, *resid = small.ptr + n, *norms = small.ptr + n + k;
@@ -428,8 +420,7 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                                         cudaMemcpyDeviceToDevice, s));
             }
             if (status == ACX_CUDA_SUCCESS) {
-                acx_gaps_kernel<<<dim3(blocks_for((size_t)n), k), kThreads, 0, s>>>(d, n, F.g.ptr,
-                                                                                    flag);
+                acx_gaps_kernel<<<dim3(blocks_for((size_t)n), k), kThreads, 0, s>>>(d, n, flag);
                 cuda_ok(cudaGetLastError());
                 count_launch();
                 lib_ok(F.product.begin(X.ptr, k));

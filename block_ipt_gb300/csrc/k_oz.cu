@@ -50,6 +50,7 @@
 // drains its own copies and MMAs (bounded), frees TMEM and returns.
 #include <cuda.h>
 #include <cuda_fp16.h>
+#include <float.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1129,6 +1130,8 @@ oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
 
 // The IPT map from the partials of Delta X:
 //   c_j = (Delta X)_jj,  X'_ij = ((Delta X)_ij - X_ij c_j) g_ij,  X'_jj = 1
+// (DIVIDE, the ACX map: divided by d_j - d_i, 0 where that is zero, as
+// acx_cuda.cu:109-172 rounds it; 1.5 % of a call at n = 4096, k = 16),
 // (IPT_C_GPU/src/ipt_cuda.cu:1369-1443), the column maxima of X' and with
 // want_norms ||X' - X||_F, ||X||_F (ipt_cuda.cu:1457-1467,1663-1688); with
 // resid_part also the block's part of ||(H X)_c - X_c (H X)_cc||^2 (ACX).  A
@@ -1144,7 +1147,7 @@ oz_finish_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
 // n = 8192, k = 32: 13 us per step together with the digit pass of X.
 constexpr int kUpdateThreads = 256;
 
-template <int R, bool RESID>
+template <int R, bool RESID, bool DIVIDE>
 __global__ void __launch_bounds__(kUpdateThreads + 32)
 oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ H,
                  const double *__restrict__ d, const double *__restrict__ g,
@@ -1190,7 +1193,7 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
             y[q] = x[q] = gi[q] = 0.0;
             if (i < n) {
                 x[q] = xc[i];
-                gi[q] = g[(size_t)i + (size_t)c * n];
+                gi[q] = DIVIDE ? d[c] - d[i] : g[(size_t)i + (size_t)c * n];
                 y[q] = delta(i, slots[(q * kUpdateThreads + t) / kBM]);
             }
         }
@@ -1211,7 +1214,12 @@ oz_update_kernel(const __grid_constant__ Partials p, const double *__restrict__ 
                     const double r = fma(x[q], d[i] - hcc, y[q]);
                     rsq = fma(r, r, rsq);
                 }
-                double out = i == c ? 1.0 : fma(-x[q], cj, y[q]) * gi[q];
+                double out = 1.0;
+                if (i != c) {
+                    out = fma(-x[q], cj, y[q]);
+                    if (!DIVIDE) out *= gi[q];
+                    else out = fabs(gi[q]) <= DBL_EPSILON ? 0.0 : out / gi[q];
+                }
                 if (failed) out = NAN;
                 Xn[(size_t)i + (size_t)c * n] = out;
                 const unsigned long long a = abs_bits(out);
@@ -1780,9 +1788,14 @@ int OzProduct::step(const double *X, const double *g, double *Xn, int want_norms
         }
     }
     KernelTimerScope timer(kProfFp64Update, s);
-    auto update = resid_part == nullptr
-                      ? (wide ? oz::oz_update_kernel<4, false> : oz::oz_update_kernel<1, false>)
-                      : (wide ? oz::oz_update_kernel<4, true> : oz::oz_update_kernel<1, true>);
+    auto update =
+        g != nullptr ? (wide ? oz::oz_update_kernel<4, false, false>
+                             : oz::oz_update_kernel<1, false, false>)
+        : resid_part == nullptr ? (wide ? oz::oz_update_kernel<4, false, true>
+                                        : oz::oz_update_kernel<1, false, true>)
+                                : (wide ? oz::oz_update_kernel<4, true, true>
+                                        : oz::oz_update_kernel<1, true, true>);
+    if (g != nullptr && resid_part != nullptr) return IPT_CUDA_INVALID_ARGUMENT;
     IPTGB_CHECK(launch_pdl(update,
                            dim3((unsigned)grid), dim3(oz::kUpdateThreads + 32), 0, s, partials(),
                            m->H, d, g, X, Xn, colmax.ptr + (1 - cur) * set, row_blocks,

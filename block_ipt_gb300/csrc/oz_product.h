@@ -98,7 +98,7 @@ struct OzProduct {
     // The plain IPT loop keeps the column maxima of its iterate up to date
     // itself: begin() scans the first block, step() forms Delta X from the
     // maxima of set `cur` and then Xn = F(X) (IPT map with g = 1 / (d_j - d_i),
-    // n x C), the maxima of Xn in the other set, and with ns (want_norms)
+    // n x C; null: the ACX map, which divides), the maxima of Xn in the other set, and with ns (want_norms)
     // ||Xn - X||_F and ||X||_F in ns->norms.
     int begin(const double *X, int C);
     // resid_part (optional): update_row_blocks parts per column of
