@@ -588,6 +588,7 @@ int dense_block_device(const double *dH_in, int n, int k, const IPTBlockOptions 
         if (!fused) {
             IPTGB_CHECK(ozm.scan_rows(dH, n, nullptr, s));
             IPTGB_CHECK(ozm.build_words(lowp_mode ? kOzSlices : 7, s));
+            IPTGB_CHECK(ozm.settle(s));
             use_oz = !ozm.wide;
         }
     }

@@ -31,9 +31,7 @@ int DenseFp64Operator::bind(const double *H_, int n_, double *d, cudaStream_t s)
         return d != nullptr ? launch_extract_diagonal(H, n, n, d, s) : IPT_CUDA_SUCCESS;
     }
     IPTGB_CHECK(own.scan_rows(H, n, d, s));
-    IPTGB_CHECK(own.build_words(7, s));
-    if (own.wide) slices = 0;
-    return IPT_CUDA_SUCCESS;
+    return own.build_words(7, s);
 }
 
 void DenseFp64Operator::share(const OzMatrix *scanned, cudaStream_t s)
@@ -51,6 +49,11 @@ int DenseFp64Operator::start(const double *X, int k_, const double *d)
     IPTGB_CHECK(product.bind(matrix, d, slices, stream));
     if (g.count < (size_t)n * k) IPTGB_CHECK(g.alloc((size_t)n * k, stream));
     IPTGB_CHECK(launch_gap_reciprocals(d, n, k, g.ptr, stream));
+    IPTGB_CHECK(product.begin(X, k));
+    IPTGB_CHECK(own.settle(stream));
+    if (slices == 0 || !matrix->wide) return IPT_CUDA_SUCCESS;
+    slices = 0;
+    IPTGB_CHECK(product.bind(matrix, d, slices, stream));
     return product.begin(X, k);
 }
 

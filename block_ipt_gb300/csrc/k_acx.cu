@@ -411,7 +411,7 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                 }
             } else if (lib_ok(F.matrix.scan_rows(H, n, d, s)) &&
                        lib_ok(F.matrix.build_words(7, s))) {
-                lib_ok(F.product.bind(&F.matrix, d, F.matrix.wide ? 0 : 7, s));
+                lib_ok(F.product.bind(&F.matrix, d, 7, s));
             }
             if (initial == nullptr) {
                 lib_ok(launch_set_identity(X.ptr, n, k, s));
@@ -423,7 +423,10 @@ int acx_fp64_run(const double *H, int n, int k, double tol, int maxiter, const d
                 acx_gaps_kernel<<<dim3(blocks_for((size_t)n), k), kThreads, 0, s>>>(d, n, flag);
                 cuda_ok(cudaGetLastError());
                 count_launch();
-                lib_ok(F.product.begin(X.ptr, k));
+                if (lib_ok(F.product.begin(X.ptr, k)) && lib_ok(F.matrix.settle(s)) &&
+                    F.matrix.wide && lib_ok(F.product.bind(&F.matrix, d, 0, s))) {
+                    lib_ok(F.product.begin(X.ptr, k));
+                }
             }
         }
         std::vector<double> host((size_t)k + 2);

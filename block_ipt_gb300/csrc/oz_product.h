@@ -23,8 +23,9 @@ struct OzMatrix {
     int nst = 0;           // 32-element K stages of a row
     int blocks = 0;        // kOzBlock-element blocks of a row
     int words_slices = 0;  // digits per entry in `words` (0: none)
-    // build_words(7): entries of a row span more binades within a block than
-    // the 56-bit split multiplies as accurately as FP64 FMAs (oz_range_limit)
+    // settle() after build_words(7): entries of a row span more binades within
+    // a block than the 56-bit split multiplies as accurately as FP64 FMAs
+    // (oz_range_limit)
     bool wide = false;
     DeviceBuffer<int> rowexp;
     DeviceBuffer<uint16_t> blockexp;  // [block][row], oz_pack_exponent
@@ -41,12 +42,14 @@ struct OzMatrix {
     int scan_rows(const double *H, int n, double *diag, cudaStream_t s);
     // digit words from a second pass (for matrices multiplied more than once
     // or twice); without an error none where they exceed kMaxWordMb or the
-    // device's memory.  slices = 7: finds out whether the matrix is `wide`
-    // (and waits for that); a wide one gets no words.
+    // device's memory.  slices = 7: also finds out whether the matrix is
+    // `wide`, which settle() waits for; a wide one then has no words.
     // Until the object goes, an allocation of this thread that fails takes the
     // words' memory (reclaim_memory): the products then read H.
     int build_words(int slices, cudaStream_t s);
+    int settle(cudaStream_t s);
     bool drop_words(cudaStream_t s);
+    int *answer = nullptr;        // page-locked, while settle() is due
     OzMatrix *held_before = nullptr;  // the thread's list of matrices with words
     bool listed = false;
 };
