@@ -109,7 +109,7 @@ int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cud
 enum ProfiledKernel {
     kProfLowpProduct = 0,   // tensor-core / FP32 SIMT block product (low precision)
     kProfLowpUpdate = 1,    // low-precision IPT update
-    kProfFp64Product = 2,   // FP64 dense split-K block product
+    kProfFp64Product = 2,   // FP64-accurate dense block product
     kProfFp64Update = 3,    // FP64 IPT update / partial sum
     kProfCsrProduct = 4,    // FP64 CSR block product
     kProfSmallEig = 5,      // one-CTA Jacobi eigensolver

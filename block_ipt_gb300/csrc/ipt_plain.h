@@ -34,9 +34,9 @@ struct Fp64Operator {
 // Dense H: Delta X by the 56-bit digit-slice product on the tensor cores
 // (k_oz.cu), whose consumer applies the map.  It replaces a split-K FP64 SIMT
 // product (GB300 runs FP64 FMAs at 1/64 of the FP32 rate; on a matrix of few
-// row blocks most SMs stood idle as well): a step takes 172 us instead of 3.7
-// ms at n = 8192, k = 32, 29 us instead of 105 us at n = 1024, k = 8, so no
-// size keeps the old one for its time; 0.35 instead of 6.1 ms with all n = 1501
+// row blocks most SMs stood idle as well): a step takes 165 us instead of 3.7
+// ms at n = 8192, k = 32, 27 us instead of 105 us at n = 1024, k = 8, so no
+// size keeps the old one for its time; 0.33 instead of 6.1 ms with all n = 1501
 // columns.
 //
 // Its error: in the 2-norm it is the smaller one (after 12 steps at n = k =

@@ -38,7 +38,7 @@
 // bytes per cycle, against 1090 cycles of MMA and 32 KB of HBM traffic (79 us
 // per product of n = 8192 at the measured 6.8 TB/s).  Measured at n = 8192, 32
 // columns: 132 us per product with one scale per row and column (2240 cycles
-// per stage; tensor pipe 50 %, HBM 54 %), 157 us with those of S = 7 (35 more
+// per stage; tensor pipe 50 %, HBM 54 %), 147 us with those of S = 7 (35 more
 // instructions per sum in the drain); the split-K FP64 SIMT product it replaces
 // in the plain path 3.6 ms (95 % of the FP64 pipe).  With one scale: digit
 // slices stored as FP16 (14 bytes per entry with 7 slices) would need 139 us of
@@ -825,8 +825,8 @@ oz_product_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant
                 // four columns and half their levels at a time (more do not fit
                 // in the registers): the first four, which then change places
                 // with the rest.  (Unrolled, the drain's instructions crowd the
-                // converters' out of the instruction cache: 170 us instead of
-                // 157 at n = 8192, 32 columns.)
+                // converters' out of the instruction cache: 13 us more at n =
+                // 8192, 32 columns.)
 #pragma unroll 1
                 for (int j0 = 0; j0 < NC; j0 += 4) {
                     uint32_t v[4][4];

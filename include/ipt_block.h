@@ -33,8 +33,11 @@ extern "C" {
 
 /* Precision of the IPT stage's block product Delta X. */
 enum {
-    IPT_BLOCK_FP64 = 0, /* FP64-accurate product on the FP16 tensor cores (dense),
-                           FP64 or double-float gather (CSR) */
+    IPT_BLOCK_FP64 = 0, /* dense: 56 bits below the largest entry of every 128
+                           columns of a row (and rows of a column of X), on the
+                           FP16 tensor cores; FP64 FMAs where rows span more
+                           binades within them than that holds.  CSR: FP64 or
+                           double-float gather */
     IPT_BLOCK_FP16 = 1, /* FP16 tensor cores (tcgen05), FP32 accumulation */
     IPT_BLOCK_BF16 = 2, /* BF16 tensor cores (tcgen05), FP32 accumulation */
     IPT_BLOCK_TF32 = 3, /* TF32 tensor cores (tcgen05), FP32 accumulation */
